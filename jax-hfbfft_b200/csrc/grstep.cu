@@ -289,47 +289,85 @@ int precond_launch(hfb_ctx_s* c, int prec, int ns, int nneut, const void* src, c
 }
 
 // ------------------------------------------------------ gradient-step glue --
-// Per-state weights (static.py:152-170, 125-136): hpsi weights and the
-// preconditioner weights.
-__global__ void grstep_weights_kernel(int ns, int tbcs, const double* wocc, const double* wguv, const double* pairwg,
-                                      const double* wstates, double* wt, double* wu, double* lw, double* lu) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
-  if (tbcs) {
-    wt[s] = 1.0; wu[s] = 0.0; lw[s] = 1.0; lu[s] = 0.0;
-  } else {
-    wt[s] = wstates[s] * wocc[s];
-    wu[s] = wstates[s] * wguv[s] * pairwg[s];
-    lw[s] = wocc[s];
-    lu[s] = wguv[s] * pairwg[s];
-  }
-}
+// Per-state weights (static.py:152-170, 125-136) -- hpsi weights and the
+// preconditioner weights -- and max(v_pair[iq]) over the grid, in one launch.
+// The maximum reads 2 n^3 doubles: kVmaxBlocks blocks per isospin leave each
+// block a few kB (one block per isospin took 116 us at 40^3, bound by one
+// SM's loads in flight; 3 us here).  The last block to finish combines the
+// blocks' maxima and returns the counter to zero for the next launch.
+constexpr int kVmaxBlocks = 64;
 
-// max(v_pair[iq]) over the grid, one block per isospin (order-independent).
-__global__ void vpair_max_kernel(const double* v_pair, size_t n3, int zero, double* vmax) {
-  __shared__ double red[32];
-  const int iq = blockIdx.x;
+__global__ void __launch_bounds__(256)
+grstep_weights_kernel(int ns, int tbcs, const double* wocc, const double* wguv, const double* pairwg,
+                      const double* wstates, double* wt, double* wu, double* lw, double* lu, const double* v_pair,
+                      size_t n3, double* vpart, int* counter, double* vmax) {
+  const int blk = blockIdx.x + gridDim.x * blockIdx.y;
+  for (int s = blk * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * gridDim.y * blockDim.x) {
+    if (tbcs) {
+      wt[s] = 1.0; wu[s] = 0.0; lw[s] = 1.0; lu[s] = 0.0;
+    } else {
+      wt[s] = wstates[s] * wocc[s];
+      wu[s] = wstates[s] * wguv[s] * pairwg[s];
+      lw[s] = wocc[s];
+      lu[s] = wguv[s] * pairwg[s];
+    }
+  }
+  if (!v_pair) {
+    if (blk == 0 && threadIdx.x < 2) vmax[threadIdx.x] = 0.0;
+    return;
+  }
+  __shared__ double red[8];
+  __shared__ int last;
+  const double* v = v_pair + blockIdx.y * n3;
   double m = -1.0e300;
-  if (!zero)
-    for (size_t i = threadIdx.x; i < n3; i += blockDim.x) m = fmax(m, v_pair[iq * n3 + i]);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x)
+    m = fmax(m, v[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double r = red[0];
-    for (int i = 1; i < (int)(blockDim.x / 32); ++i) r = fmax(r, red[i]);
-    vmax[iq] = zero ? 0.0 : r;
+    for (int i = 1; i < 8; ++i) m = fmax(m, red[i]);
+    vpart[blk] = m;
+    __threadfence();
+    last = atomicAdd(counter, 1) == (int)(gridDim.x * gridDim.y) - 1;
   }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x < 64) {
+    const int iq = threadIdx.x / 32;
+    double r = -1.0e300;
+    for (int i = threadIdx.x % 32; i < (int)gridDim.x; i += 32) r = fmax(r, __ldcg(vpart + iq * gridDim.x + i));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+    if (threadIdx.x % 32 == 0) vmax[iq] = r;
+  }
+  if (threadIdx.x == 0) *counter = 0;
 }
 
-// Per-state sums of plane partials: out[s] = scale * sum_j part[s][j][k].
-__global__ void state_reduce_kernel(int ns, int nplanes, const double* part, int k, double scale, double* out) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
+// Per-state sums of the overlap partials, spe[s] and hexp[s] = scale *
+// sum_j part[s][j][0 / 1]: one warp per state, both sums from one read of
+// the pairs (fixed order).
+__global__ void __launch_bounds__(128)
+state_reduce_kernel(int ns, int nparts, const double2* __restrict__ part, double scale, double* spe, double* hexp) {
+  const int s = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32;
   if (s >= ns) return;
-  double a = 0;
-  for (int j = 0; j < nplanes; ++j) a += part[((size_t)s * nplanes + j) * 2 + k];
-  out[s] = scale * a;
+  double a = 0.0, b = 0.0;
+  for (int j = lane; j < nparts; j += 32) {
+    const double2 v = part[(size_t)s * nparts + j];
+    a += v.x;
+    b += v.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) {
+    spe[s] = scale * a;
+    hexp[s] = scale * b;
+  }
 }
 
 // Simple damped step when e0dmp <= 0 (static.py:181-185).
@@ -346,34 +384,51 @@ __global__ void simple_step_kernel(int ns, size_t n3, const double* spe_new, con
 }
 
 // Finalise efluct, denerg and the running sums (static.py:110-111, 211, 251-257).
-// One block; deterministic sequential sums.
-__global__ void grstep_finish_kernel(int ns, int do_fluct, int nplanes, const double* fl, double wxyz,
-                                     const double* spe_new, const double* wocc, const double* wstates,
-                                     double* sp_energy, double* ef1, double* ef2, double* sums) {
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) {
-    if (do_fluct) {
-      double a = 0, b = 0;
-      for (int j = 0; j < nplanes; ++j) {
-        a += fl[((size_t)s * nplanes + j) * 2 + 0];
-        b += fl[((size_t)s * nplanes + j) * 2 + 1];
+// One block: a warp per state for the plane partials, then one warp's
+// fixed-order sums over the states (a thread per state and one thread's
+// sums took 61 us for 236 states of 48 planes, a serial chain of L2
+// latencies; 6 us here).
+__global__ void __launch_bounds__(1024)
+grstep_finish_kernel(int ns, int do_fluct, int nplanes, const double2* __restrict__ fl, double wxyz,
+                     const double* spe_new, const double* wocc, const double* wstates, double* sp_energy, double* ef1,
+                     double* ef2, double* sums) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (do_fluct)
+    for (int s = warp; s < ns; s += 32) {
+      double a = 0.0, b = 0.0;
+      for (int j = lane; j < nplanes; j += 32) {
+        const double2 v = fl[(size_t)s * nplanes + j];
+        a += v.x;
+        b += v.y;
       }
-      ef1[s] = sqrt(wxyz * a);
-      ef2[s] = sqrt(wxyz * b);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if (lane == 0) {
+        ef1[s] = sqrt(wxyz * a);
+        ef2[s] = sqrt(wxyz * b);
+      }
     }
-  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double sf = 0, sd = 0;
-    for (int s = 0; s < ns; ++s) {
-      double den = (sp_energy[s] - spe_new[s]) / fabs(spe_new[s]);
-      sf += ef1[s];
-      sd += wocc[s] * wstates[s] * den;
-    }
+  if (warp != 0) return;
+  double sf = 0.0, sd = 0.0;
+  for (int s = lane; s < ns; s += 32) {
+    const double e = spe_new[s];
+    sf += ef1[s];
+    sd += wocc[s] * wstates[s] * ((sp_energy[s] - e) / fabs(e));
+    sp_energy[s] = e;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sf += __shfl_xor_sync(0xffffffffu, sf, o);
+    sd += __shfl_xor_sync(0xffffffffu, sd, o);
+  }
+  if (lane == 0) {
     sums[0] = sf;
     sums[1] = sd;
   }
-  __syncthreads();
-  for (int s = threadIdx.x; s < ns; s += blockDim.x) sp_energy[s] = spe_new[s];
 }
 
 }  // namespace hfb
@@ -395,24 +450,22 @@ extern "C" int hfb_grstep(hfb_ctx_t ctx, int prec, const hfb_grstep_args* a, voi
   const size_t n3 = (size_t)n * n * n;
   const int nov = hpsi_ovl_parts(ctx, prec);
   double* part = (double*)scratch(ctx, hfb_ctx_s::S_PART, sizeof(double) * (size_t)ns * (nov + n) * 2);
-  double* vec = (double*)scratch(ctx, hfb_ctx_s::S_SMALL, sizeof(double) * ((size_t)ns * 6 + 8));
+  double* vec = (double*)scratch(ctx, hfb_ctx_s::S_SMALL, sizeof(double) * ((size_t)ns * 6 + 8 + 2 * kVmaxBlocks));
   if (!part || !vec) return HFB_ERR_ALLOC;
   double* ovl = part;
   double* fl = part + (size_t)ns * nov * 2;
   double *wt = vec, *wu = vec + ns, *lw = vec + 2 * ns, *lu = vec + 3 * ns, *spe_new = vec + 4 * ns,
          *hexp = vec + 5 * ns, *vmax = vec + 6 * ns;
-  grstep_weights_kernel<<<(ns + 127) / 128, 128, 0, st>>>(ns, a->tbcs, a->wocc, a->wguv, a->pairwg, a->wstates, wt,
-                                                           wu, lw, lu);
-  HFB_CHECK_LAUNCH();
-  vpair_max_kernel<<<2, 256, 0, st>>>(a->v_pair, n3, a->tbcs || !a->v_pair, vmax);
+  double* vpart = vmax + 8;
+  const double* vp = a->tbcs ? nullptr : a->v_pair;
+  grstep_weights_kernel<<<vp ? dim3(kVmaxBlocks, 2) : dim3((ns + 255) / 256, 1), 256, 0, st>>>(
+      ns, a->tbcs, a->wocc, a->wguv, a->pairwg, a->wstates, wt, wu, lw, lu, vp, n3, vpart, ctx->counters, vmax);
   HFB_CHECK_LAUNCH();
   // 1) h psi_old: ps1 (weighted) into hmfpsi (scratch), h psi into hampsi
   int r = hpsi_launch(ctx, prec, a->pot, 0, ns, a->nneut, a->psi, wt, wu, a->hampsi, a->hmfpsi, a->hampsi, nullptr,
                       ovl, st);
   if (r) return r;
-  state_reduce_kernel<<<(ns + 127) / 128, 128, 0, st>>>(ns, nov, ovl, 0, a->wxyz, spe_new);
-  HFB_CHECK_LAUNCH();
-  state_reduce_kernel<<<(ns + 127) / 128, 128, 0, st>>>(ns, nov, ovl, 1, a->wxyz, hexp);
+  state_reduce_kernel<<<(ns + 3) / 4, 128, 0, st>>>(ns, nov, (const double2*)ovl, a->wxyz, spe_new, hexp);
   HFB_CHECK_LAUNCH();
   // 2) damped step
   if (a->e0dmp > 0.0) {
@@ -430,7 +483,7 @@ extern "C" int hfb_grstep(hfb_ctx_t ctx, int prec, const hfb_grstep_args* a, voi
           ns, n3, spe_new, a->sp_energy, a->x0dmp, a->x0dmp_dev, (const float2*)a->hmfpsi, (float2*)a->psi);
     HFB_CHECK_LAUNCH();
   }
-  grstep_finish_kernel<<<1, 256, 0, st>>>(ns, a->do_fluct && a->e0dmp > 0.0, n, fl, a->wxyz, spe_new, a->wocc,
+  grstep_finish_kernel<<<1, 1024, 0, st>>>(ns, a->do_fluct && a->e0dmp > 0.0, n, (const double2*)fl, a->wxyz, spe_new, a->wocc,
                                           a->wstates, a->sp_energy, a->sp_efluct1, a->sp_efluct2, a->sums);
   HFB_CHECK_LAUNCH();
   // 3) h psi_new into hmfpsi (and v_pair psi_new into delpsi when requested)
