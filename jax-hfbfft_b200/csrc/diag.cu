@@ -8,10 +8,11 @@
 //    lower triangle held in shared memory (round-robin ordering, n/2 disjoint
 //    rotations per round); the rotations are recorded and replayed onto the
 //    eigenvector matrix by a row-parallel kernel.  Eigenvalues ascending.
-//  * small FP64 complex GEMMs for U = S^-1/2 V_lambda, U^H H U, U lambda.
+//  * the small-matrix chains (S^-1/2, eigen refinement, U^H H U, U lambda) as
+//    one cluster launch each (diag_cluster.cu).
 //  * rotation [psi_new | lagrange] = psi [U | U lambda_sym] as one GEMM pass.
 #include <math.h>
-#include "hfb_ctx.cuh"
+#include "diag.cuh"
 
 namespace hfb {
 
@@ -131,12 +132,6 @@ __device__ __forceinline__ void gd_cp16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
                "l"(gmem)
                : "memory");
-}
-
-__device__ __forceinline__ void gd_mma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
 }
 
 __global__ void __launch_bounds__(GD_THREADS) gram_dmma_kernel(GramJob job, size_t K, size_t n3,
@@ -359,10 +354,6 @@ __device__ __forceinline__ void rr_pair(int m, int r, int q, int& a, int& b) {
   if (a > b) { int t = a; a = b; b = t; }
 }
 
-struct Pair2 {
-  int v[2];
-};
-
 struct JacRot {
   double cs, sn;
   double2 om;   // exp(-i phi)
@@ -385,7 +376,7 @@ struct EighBatch {
   int* sweeps;                 // optional device output [nb]: sweeps used
   double tol_rel;              // off-diagonal threshold relative to ||A||_F (0: double eps)
   int stage_half;              // rotations per round in the replay's staging buffer (set by eigh_batch)
-  const int* gate;             // optional device flag: the solve runs only when *gate != 0
+  const int* gate;             // optional device flags [nb]: matrix b is solved only when gate[b] != 0
 };
 
 // One CTA per matrix: cyclic two-sided Jacobi on the packed lower triangle.
@@ -396,8 +387,8 @@ struct EighBatch {
 __global__ void __launch_bounds__(kJacThreads)
 jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t rot_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (eb.gate && *eb.gate == 0) return;
   const int b = blockIdx.x;
+  if (eb.gate && eb.gate[b] == 0) return;
   const int n = eb.n[b], lda = eb.lda[b];
   const int m = n + (n & 1);   // pad odd sizes with a decoupled index
   const int half = m / 2;
@@ -621,9 +612,9 @@ __global__ void __launch_bounds__(256)
 jacobi_vectors_kernel(EighBatch eb, const JacRot* __restrict__ rot, const int* __restrict__ nrounds,
                       size_t rot_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  if (eb.gate && *eb.gate == 0) return;
   int b = 0;
   while (b + 1 < eb.nb && (int)blockIdx.x >= eb.vblk0[b + 1]) ++b;
+  if (eb.gate && eb.gate[b] == 0) return;
   const int rb = blockIdx.x - eb.vblk0[b];
   const int n = eb.n[b], lda = eb.lda[b];
   const int m = n + (n & 1), half = m / 2;
@@ -693,8 +684,8 @@ jacobi_vectors_kernel(EighBatch eb, const JacRot* __restrict__ rot, const int* _
 }
 
 __global__ void sort_values_kernel(EighBatch eb) {
-  if (eb.gate && *eb.gate == 0) return;
   const int b = blockIdx.x;
+  if (eb.gate && eb.gate[b] == 0) return;
   const int n = eb.n[b];
   extern __shared__ double tmpw[];
   double* wb = eb.w[b];
@@ -764,32 +755,21 @@ int eigh_launch(hfb_ctx_s* c, int nb, int n, int lda, const double2* a, double* 
 }
 
 // ========================================================= small GEMMs ====
-// C[b] = alpha A'[b] B'[b] + dadd I with A' = A or A^H, B' = B or B^H;
-// n x n, leading dim ld, batched over blockIdx.z with per-batch strides.
-// When ``gate`` is given the kernel does nothing if gate_k > *gate (used to
-// retire converged Newton-Schulz steps without a host round trip).
-__global__ void zgemm_small_kernel(int n, int ld, int ta, int tb, const double2* A, size_t sa, const double2* B,
-                                   size_t sb, double2* C, size_t sc, Pair2 nper, double alpha, double dadd,
-                                   const int* gate, int gate_k) {
+// C = A' B' with A' = A or A^H, B' = B or B^H; n x n, leading dim ld.
+__global__ void zgemm_small_kernel(int n, int ld, int ta, int tb, const double2* A, const double2* B, double2* C) {
   __shared__ double2 As[16][17], Bs[16][17];
-  if (gate && gate_k > *gate) return;
-  const int b = blockIdx.z;
-  const int nb = nper.v[b] > 0 ? nper.v[b] : n;
   const int i = blockIdx.y * 16 + threadIdx.y, j = blockIdx.x * 16 + threadIdx.x;
-  if (blockIdx.y * 16 >= nb || blockIdx.x * 16 >= nb) return;
-  const double2* Ab = A + b * sa;
-  const double2* Bb = B + b * sb;
   double re = 0, im = 0;
-  for (int k0 = 0; k0 < nb; k0 += 16) {
+  for (int k0 = 0; k0 < n; k0 += 16) {
     const int ka = k0 + threadIdx.x, kb = k0 + threadIdx.y;
     double2 av = make_double2(0, 0), bv = make_double2(0, 0);
-    if (i < nb && ka < nb) {
-      if (ta) { av = Ab[(size_t)ka * ld + i]; av.y = -av.y; }
-      else av = Ab[(size_t)i * ld + ka];
+    if (i < n && ka < n) {
+      if (ta) { av = A[(size_t)ka * ld + i]; av.y = -av.y; }
+      else av = A[(size_t)i * ld + ka];
     }
-    if (j < nb && kb < nb) {
-      if (tb) { bv = Bb[(size_t)j * ld + kb]; bv.y = -bv.y; }
-      else bv = Bb[(size_t)kb * ld + j];
+    if (j < n && kb < n) {
+      if (tb) { bv = B[(size_t)j * ld + kb]; bv.y = -bv.y; }
+      else bv = B[(size_t)kb * ld + j];
     }
     As[threadIdx.y][threadIdx.x] = av;
     Bs[threadIdx.y][threadIdx.x] = bv;
@@ -802,469 +782,34 @@ __global__ void zgemm_small_kernel(int n, int ld, int ta, int tb, const double2*
     }
     __syncthreads();
   }
-  if (i < nb && j < nb)
-    C[b * sc + (size_t)i * ld + j] = make_double2(alpha * re + (i == j ? dadd : 0.0), alpha * im);
-}
-
-static int zgemm_small(int nmax, int ld, int ta, int tb, const double2* A, size_t sa, const double2* B, size_t sb,
-                       double2* C, size_t sc, Pair2 nper, int batch, cudaStream_t st, double alpha = 1.0,
-                       double dadd = 0.0, const int* gate = nullptr, int gate_k = 0) {
-  dim3 grid((nmax + 15) / 16, (nmax + 15) / 16, batch);
-  zgemm_small_kernel<<<grid, dim3(16, 16), 0, st>>>(nmax, ld, ta, tb, A, sa, B, sb, C, sc, nper, alpha, dadd, gate,
-                                                    gate_k);
-  HFB_CHECK_LAUNCH();
-  return HFB_OK;
+  if (i < n && j < n) C[(size_t)i * ld + j] = make_double2(re, im);
 }
 
 // One n x n product C = A' B' (A' = A or A^H, B' = B or B^H), leading
 // dimension ld, for other translation units.
 int zgemm_small_one(int n, int ld, int ta, int tb, const double2* A, const double2* B, double2* C, cudaStream_t st) {
-  Pair2 nper;
-  nper.v[0] = n;
-  nper.v[1] = 0;
-  return zgemm_small(n, ld, ta, tb, A, 0, B, 0, C, 0, nper, 1, st);
-}
-
-// ------------------------------------------ Hermitian eigen refinement ----
-// Eigenpairs of a Hermitian matrix that is already nearly diagonal in the
-// current basis (lambda after a gradient step: the states are the previous
-// eigenvectors), by the iterative refinement of Ogita and Aishima (Japan J.
-// Indust. Appl. Math. 35, 2018; clustered eigenvalues: 36, 2019).  From X
-// (start I):
-//   R = I - X^H X,  S = X^H A X,  l_i = Re S_ii / (1 - Re R_ii),
-//   d = 2 (||S - diag(l)||_F + ||A||_F ||R||_F),
-//   E_ij = (S_ij + l_j R_ij) / (l_j - l_i)  if |l_i - l_j| > d,  R_ij / 2 else,
-//   X <- X (I + E),
-// quadratically convergent for the pairs separated by more than d.  The
-// pairs the last step left coupled (Kramers pairs, accidental
-// near-degeneracies) form clusters that are diagonalised exactly as small
-// blocks of the final X^H A X; the eigenpairs are sorted ascending and
-// accepted only if V^H A V is diagonal and V^H V = I to the requested
-// accuracy.  Only GEMMs on many SMs and a few small kernels: no single-CTA
-// sweep.  When the refinement has not converged after kRefMaxIt steps, a
-// cluster has more than kClusterMax members or the acceptance test fails,
-// the Jacobi solver runs instead (its kernels are gated on a device flag, so
-// the choice needs no host round trip).
-constexpr int kRefMaxIt = 6;
-constexpr int kClusterMax = 16;   // a j = 15/2 shell of a near-spherical nucleus
-constexpr int kRefMaxN = 256;
-
-struct RefWork {
-  double2 *Ah, *X0, *X1, *AX, *S, *R, *E, *Xf, *Q;   // [nb][ld][ld] each; Q [nb][ld][kClusterMax]
-  double *lam, *ev, *anorm, *dlt;                    // [nb][ld], [nb][ld], [nb], [nb]
-  int *conv, *rdone, *fallback, *cinfo;              // conv [nb], cinfo [nb][ld][4]
-};
-
-__device__ __forceinline__ double block_sum(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < (int)(blockDim.x / 32); ++w) t += red[w];
-  return t;
-}
-
-// Ah = the Hermitian matrix of the lower triangle of A (the diagonal's
-// imaginary part dropped, as eigh with UPLO='L'), X0 = I, ||Ah||_F; flags reset.
-__global__ void ref_init_kernel(int ld, Pair2 nper, const double2* A, size_t sA, RefWork w) {
-  __shared__ double red[32];
-  const int b = blockIdx.x, n = nper.v[b];
-  const size_t sm = (size_t)ld * ld;
-  const double2* Ab = A + b * sA;
-  double f2 = 0.0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    double2 v = i >= j ? Ab[(size_t)i * ld + j] : Ab[(size_t)j * ld + i];
-    if (i < j) v.y = -v.y;
-    if (i == j) v.y = 0.0;
-    w.Ah[b * sm + (size_t)i * ld + j] = v;
-    w.X0[b * sm + (size_t)i * ld + j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-    f2 += v.x * v.x + v.y * v.y;
-  }
-  const double t = block_sum(f2, red);
-  if (threadIdx.x == 0) {
-    w.anorm[b] = sqrt(t);
-    w.conv[b] = 0;
-    if (b == 0) {
-      *w.rdone = 1 << 30;
-      *w.fallback = 0;
-    }
-  }
-}
-
-// One refinement step for matrix b: l, d, E' = I + E; conv[b] when the
-// coupling of the separated pairs and the loss of orthonormality are small.
-__global__ void ref_update_kernel(int ld, Pair2 nper, RefWork w, int k, double tol) {
-  __shared__ double red[32];
-  __shared__ double lam[kRefMaxN];
-  if (k > *w.rdone) return;
-  const int b = blockIdx.x, n = nper.v[b];
-  const size_t sm = (size_t)ld * ld;
-  const double2* S = w.S + b * sm;
-  const double2* R = w.R + b * sm;
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    lam[i] = S[(size_t)i * ld + i].x / (1.0 - R[(size_t)i * ld + i].x);
-  __syncthreads();
-  double o2 = 0.0, r2 = 0.0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double2 sv = S[(size_t)i * ld + j], rv = R[(size_t)i * ld + j];
-    const double dx = i == j ? sv.x - lam[i] : sv.x;
-    o2 += dx * dx + sv.y * sv.y;
-    r2 += rv.x * rv.x + rv.y * rv.y;
-  }
-  const double off = sqrt(block_sum(o2, red)), rn = sqrt(block_sum(r2, red));
-  const double an = w.anorm[b];
-  const double d = 2.0 * (off + an * rn);
-  double nc2 = 0.0;
-  double2* E = w.E + b * sm;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double2 sv = S[(size_t)i * ld + j], rv = R[(size_t)i * ld + j];
-    double2 ev;
-    if (i == j) {
-      ev = make_double2(1.0 + 0.5 * rv.x, 0.5 * rv.y);
-    } else if (fabs(lam[i] - lam[j]) > d) {
-      const double den = lam[j] - lam[i];
-      ev = make_double2((sv.x + lam[j] * rv.x) / den, (sv.y + lam[j] * rv.y) / den);
-      nc2 += sv.x * sv.x + sv.y * sv.y;
-    } else {
-      ev = make_double2(0.5 * rv.x, 0.5 * rv.y);
-    }
-    E[(size_t)i * ld + j] = ev;
-  }
-  const double nc = sqrt(block_sum(nc2, red));
-  if (threadIdx.x == 0) {
-    w.dlt[b] = d;
-    // ||I - X^H X||_F cannot go below the rounding of the n-term sums
-    w.conv[b] = (nc <= tol * an && rn <= fmax(tol, 1e-11)) ? 1 : 0;
-  }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) w.lam[b * ld + i] = lam[i];
-}
-
-__global__ void ref_check_kernel(int nb, RefWork w, int k) {
-  if (k > *w.rdone) return;
-  int all = 1;
-  for (int b = 0; b < nb; ++b) all &= w.conv[b];
-  if (all) *w.rdone = k;
-}
-
-// Xf = the X after the last applied step (step g writes buffer (g + 1) % 2);
-// no convergence within kRefMaxIt steps selects the Jacobi solver.
-__global__ void ref_final_x_kernel(int ld, Pair2 nper, RefWork w) {
-  const int b = blockIdx.y, n = nper.v[b];
-  const int g = *w.rdone;
-  const bool ok = g < kRefMaxIt;
-  if (!ok && blockIdx.x == 0 && b == 0 && threadIdx.x == 0) *w.fallback = 1;
-  const size_t sm = (size_t)ld * ld;
-  const double2* X = (((ok ? g : kRefMaxIt - 1) + 1) % 2 == 0) ? w.X0 : w.X1;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int i = e / n, j = e % n;
-    w.Xf[b * sm + (size_t)i * ld + j] = X[b * sm + (size_t)i * ld + j];
-  }
-}
-
-// Clusters: the l_i of the last applied step sorted, consecutive values
-// closer than its d grouped (so every pair that step left coupled lies in
-// one cluster); each cluster's block of the final S = Xf^H A Xf is
-// diagonalised by serial cyclic Jacobi (one thread per cluster).  Output per
-// eigenpair P (sorted position of its cluster start s plus local index):
-// ev[P] and cinfo[P] = (s, size, local, original index of sorted position P).
-__global__ void ref_cluster_kernel(int ld, Pair2 nper, RefWork w) {
-  __shared__ double dg[kRefMaxN];
-  __shared__ int idx[kRefMaxN];
-  __shared__ int cstart[kRefMaxN];
-  const int b = blockIdx.x, n = nper.v[b];
-  const size_t sm = (size_t)ld * ld;
-  const double2* S = w.S + b * sm;
-  if (*w.fallback) return;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dg[i] = w.lam[(size_t)b * ld + i];
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    int r = 0;
-    for (int j = 0; j < n; ++j) r += (dg[j] < dg[i]) || (dg[j] == dg[i] && j < i);
-    idx[r] = i;
-  }
-  __syncthreads();
-  const double tau = w.dlt[b];
-  if (threadIdx.x == 0) {
-    int s0 = 0;
-    for (int p = 0; p < n; ++p) {
-      if (p > 0 && dg[idx[p]] - dg[idx[p - 1]] > tau) s0 = p;
-      cstart[p] = s0;
-    }
-  }
-  __syncthreads();
-  int* ci = w.cinfo + (size_t)b * ld * 4;
-  double* ev = w.ev + (size_t)b * ld;
-  double2* Qb = w.Q + (size_t)b * ld * kClusterMax;
-  for (int p = threadIdx.x; p < n; p += blockDim.x) {
-    if (cstart[p] != p) continue;            // one thread per cluster start
-    int c = 1;
-    while (p + c < n && cstart[p + c] == p) ++c;
-    if (c > kClusterMax) {
-      *w.fallback = 1;
-      continue;
-    }
-    double2 a[kClusterMax][kClusterMax], q[kClusterMax][kClusterMax];
-    for (int r = 0; r < c; ++r)
-      for (int t = 0; t < c; ++t) {
-        a[r][t] = S[(size_t)idx[p + r] * ld + idx[p + t]];
-        q[r][t] = make_double2(r == t ? 1.0 : 0.0, 0.0);
-      }
-    double nrm = 0.0;
-    for (int r = 0; r < c; ++r)
-      for (int t = 0; t < c; ++t) nrm += a[r][t].x * a[r][t].x + a[r][t].y * a[r][t].y;
-    nrm = sqrt(nrm);
-    for (int sweep = 0; sweep < 40 && c > 1; ++sweep) {
-      bool any = false;
-      for (int r = 0; r < c; ++r)
-        for (int t = r + 1; t < c; ++t) {
-          const double2 apq = a[r][t];
-          const double mag = hypot(apq.x, apq.y);
-          if (mag <= 1e-300 || mag <= 2.220446049250313e-16 * 1e-2 * nrm) continue;
-          any = true;
-          const double app = a[r][r].x, aqq = a[t][t].x;
-          const double theta = (aqq - app) / (2.0 * mag);
-          double tt = 1.0 / (fabs(theta) + sqrt(theta * theta + 1.0));
-          if (theta < 0.0) tt = -tt;
-          const double cs = 1.0 / sqrt(tt * tt + 1.0), sn = tt * cs;
-          // apq = mag e^{i phi}; G = [[cs, sn], [-sn e^{-i phi}, cs e^{-i phi}]] on (r, t)
-          const double2 om = make_double2(apq.x / mag, -apq.y / mag);
-          auto cm = [](double2 x, double2 y) { return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x); };
-          for (int u = 0; u < c; ++u) {          // A <- A G, Q <- Q G (columns r, t)
-            const double2 x0 = a[u][r], x1 = cm(a[u][t], om);
-            a[u][r] = make_double2(cs * x0.x - sn * x1.x, cs * x0.y - sn * x1.y);
-            a[u][t] = make_double2(sn * x0.x + cs * x1.x, sn * x0.y + cs * x1.y);
-            const double2 y0 = q[u][r], y1 = cm(q[u][t], om);
-            q[u][r] = make_double2(cs * y0.x - sn * y1.x, cs * y0.y - sn * y1.y);
-            q[u][t] = make_double2(sn * y0.x + cs * y1.x, sn * y0.y + cs * y1.y);
-          }
-          const double2 oc = make_double2(om.x, -om.y);
-          for (int u = 0; u < c; ++u) {          // A <- G^H A (rows r, t)
-            const double2 x0 = a[r][u], x1 = cm(oc, a[t][u]);
-            a[r][u] = make_double2(cs * x0.x - sn * x1.x, cs * x0.y - sn * x1.y);
-            a[t][u] = make_double2(sn * x0.x + cs * x1.x, sn * x0.y + cs * x1.y);
-          }
-          a[r][t] = make_double2(0.0, 0.0);
-          a[t][r] = make_double2(0.0, 0.0);
-        }
-      if (!any) break;
-    }
-    for (int l = 0; l < c; ++l) {
-      ev[p + l] = a[l][l].x;
-      int* cp = ci + (size_t)(p + l) * 4;
-      cp[0] = p;
-      cp[1] = c;
-      cp[2] = l;
-      for (int m = 0; m < c; ++m) Qb[(size_t)(p + m) * kClusterMax + l] = q[m][l];
-    }
-  }
-  for (int pp = threadIdx.x; pp < n; pp += blockDim.x) ci[(size_t)pp * 4 + 3] = idx[pp];
-}
-
-// Acceptance test of the assembled pairs: with S = V^H A V and R = I - V^H V
-// formed, any off-diagonal |S_ij| or diagonal |S_ii - w_i| above
-// tol_s ||A||_F, or |R_ij| above tol_r, selects the Jacobi solver.
-__global__ void ref_accept_kernel(int ld, Pair2 nper, RefWork w, const double* W, size_t sW, double tol_s,
-                                  double tol_r) {
-  __shared__ int bad;
-  const int b = blockIdx.x, n = nper.v[b];
-  if (*w.fallback) return;
-  if (threadIdx.x == 0) bad = 0;
-  __syncthreads();
-  const size_t sm = (size_t)ld * ld;
-  const double lim = tol_s * w.anorm[b];
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    double2 sv = w.S[b * sm + (size_t)i * ld + j];
-    if (i == j) sv.x -= W[b * sW + i];
-    const double2 rv = w.R[b * sm + (size_t)i * ld + j];
-    if (!(hypot(sv.x, sv.y) <= lim) || !(hypot(rv.x, rv.y) <= tol_r)) bad = 1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && bad) *w.fallback = 1;
-}
-
-// V[:, o(P)] = sum_m Xf[:, idx[s + m]] Q[s + m][l], w[o(P)] = ev[P], with o
-// the ascending order of ev (ties by P).
-__global__ void ref_assemble_kernel(int ld, Pair2 nper, RefWork w, double* W, size_t sW, double2* V, size_t sV) {
-  __shared__ int opos[kRefMaxN];
-  const int b = blockIdx.y, n = nper.v[b];
-  if (*w.fallback) return;
-  const size_t sm = (size_t)ld * ld;
-  const double* ev = w.ev + (size_t)b * ld;
-  const int* ci = w.cinfo + (size_t)b * ld * 4;
-  for (int P = threadIdx.x; P < n; P += blockDim.x) {
-    int r = 0;
-    const double e = ev[P];
-    for (int q = 0; q < n; ++q) r += (ev[q] < e) || (ev[q] == e && q < P);
-    opos[P] = r;
-    if (blockIdx.x == 0) W[b * sW + r] = e;
-  }
-  __syncthreads();
-  const double2* X = w.Xf + b * sm;
-  const double2* Qb = w.Q + (size_t)b * ld * kClusterMax;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int row = e / n, P = e % n;
-    const int s0 = ci[(size_t)P * 4], c = ci[(size_t)P * 4 + 1], l = ci[(size_t)P * 4 + 2];
-    double re = 0.0, im = 0.0;
-    for (int m = 0; m < c; ++m) {
-      const int col = ci[(size_t)(s0 + m) * 4 + 3];
-      const double2 x = X[(size_t)row * ld + col], q = Qb[(size_t)(s0 + m) * kClusterMax + l];
-      re += x.x * q.x - x.y * q.y;
-      im += x.x * q.y + x.y * q.x;
-    }
-    V[b * sV + (size_t)row * ld + opos[P]] = make_double2(re, im);
-  }
-}
-
-// ------------------------------------------------- Loewdin by Newton-Schulz --
-// S^-1/2 from the coupled Newton-Schulz iteration on A = S / c, with c the
-// largest absolute row sum (so the spectrum of A lies in (0, 1]):
-//   T = (3 I - Z Y) / 2,  Y <- Y T,  Z <- T Z,   Y -> A^1/2, Z -> A^-1/2.
-// This is the matrix the reference forms as V diag(w^-1/2) V^H
-// (static.py:470-480) whenever no eigenvalue of S falls below its floor
-// max(1e-12, eps max(w) n); S is then positive definite with condition far
-// from that floor.  Steps after convergence are retired on the device.
-constexpr int kNSMaxIt = 16;   // S is close to I after a gradient step: 4-6 steps in practice
-
-// c_b and the start Y = S / c, Z = I; gate = large.
-__global__ void ns_init_kernel(int ld, Pair2 nper, const double2* S, size_t sS, double2* Y, double2* Z, size_t sm,
-                               double* cinv, int* gate) {
-  const int b = blockIdx.x;
-  const int n = nper.v[b];
-  const double2* Sb = S + b * sS;
-  __shared__ double red[32];
-  double mx = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double rs = 0.0;
-    for (int j = 0; j < n; ++j) {
-      const double2 v = Sb[(size_t)i * ld + j];
-      rs += hypot(v.x, v.y);
-    }
-    mx = fmax(mx, rs);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int w = 0; w < (int)(blockDim.x / 32); ++w) m = fmax(m, red[w]);
-    red[0] = m;
-    cinv[b] = 1.0 / m;
-    if (b == 0) *gate = 1 << 30;
-  }
-  __syncthreads();
-  const double ci = 1.0 / red[0];
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double2 v = Sb[(size_t)i * ld + j];
-    Y[b * sm + (size_t)i * ld + j] = make_double2(v.x * ci, v.y * ci);
-    Z[b * sm + (size_t)i * ld + j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-  }
-}
-
-// After T of step k: if max|T - I| over both blocks is below 1e-9, step k
-// is the last one applied (*gate = k); it squares that error to rounding.
-__global__ void ns_check_kernel(int ld, Pair2 nper, const double2* T, size_t sm, int* gate, int k) {
-  if (k > *gate) return;
-  __shared__ double red[32];
-  double mx = 0.0;
-  for (int b = 0; b < 2; ++b) {
-    const int n = nper.v[b];
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e / n, j = e % n;
-      const double2 v = T[b * sm + (size_t)i * ld + j];
-      mx = fmax(mx, hypot(v.x - (i == j ? 1.0 : 0.0), v.y));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = 0.0;
-    for (int w = 0; w < (int)(blockDim.x / 32); ++w) m = fmax(m, red[w]);
-    if (m < 1e-9) *gate = k;
-  }
-}
-
-// U = Z_final / sqrt(c); the result of step k sits in buffer (k + 1) % 2.
-__global__ void ns_final_kernel(int ld, Pair2 nper, const double2* Z0, const double2* Z1, size_t sm,
-                                const double* cinv, const int* gate, double2* U, int* status) {
-  const int b = blockIdx.y;
-  const int n = nper.v[b];
-  const int g = *gate;
-  const bool ok = g < kNSMaxIt;
-  const double2* Z = ((ok ? g : kNSMaxIt - 1) + 1) % 2 == 0 ? Z0 : Z1;
-  const double sc = sqrt(cinv[b]);
-  if (!ok && blockIdx.x == 0 && b == 0 && threadIdx.x == 0) latch_error(status, HFB_ERR_NO_CONVERGENCE);
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double2 v = Z[b * sm + (size_t)i * ld + j];
-    U[b * sm + (size_t)i * ld + j] = make_double2(v.x * sc, v.y * sc);
-  }
+  const unsigned g = (unsigned)((n + 15) / 16);
+  zgemm_small_kernel<<<dim3(g, g), dim3(16, 16), 0, st>>>(n, ld, ta, tb, A, B, C);
+  HFB_CHECK_LAUNCH();
+  return HFB_OK;
 }
 
 // Eigenpairs of up to two nearly diagonal Hermitian matrices (lower
 // triangles at A + b sA, leading dimension ld): w ascending at W + b sW,
-// eigenvectors in the columns of V + b sV; Jacobi when the refinement does
-// not apply (see above).
+// eigenvectors in the columns of V + b sV, by refinement (diag_cluster.cu);
+// Jacobi for the matrices it does not apply to.
 static int eigh_refine(hfb_ctx_s* c, int nb, Pair2 nper, int ld, const double2* A, size_t sA, double* W, size_t sW,
                        double2* V, size_t sV, double tol_rel, cudaStream_t st) {
-  if (ld > kRefMaxN) return HFB_ERR_UNSUPPORTED_GRID;
-  const size_t sm = (size_t)ld * ld;
-  const size_t bytes = sizeof(double2) * (8 * (size_t)nb * sm + (size_t)nb * ld * kClusterMax) +
-                       sizeof(double) * (2 * (size_t)nb * ld + 2 * nb) + sizeof(int) * (nb + 2 + (size_t)nb * ld * 4) +
-                       256;
-  char* buf = (char*)scratch(c, hfb_ctx_s::S_EIG, bytes);
+  const size_t wb = (refine_bytes(nb, ld) + 15) / 16 * 16;
+  char* buf = (char*)scratch(c, hfb_ctx_s::S_EIG, wb + sizeof(int) * nb);
   if (!buf) return HFB_ERR_ALLOC;
-  RefWork w;
-  double2* mp = (double2*)buf;
-  w.Ah = mp; w.X0 = mp + nb * sm; w.X1 = mp + 2 * nb * sm; w.AX = mp + 3 * nb * sm; w.S = mp + 4 * nb * sm;
-  w.R = mp + 5 * nb * sm; w.E = mp + 6 * nb * sm; w.Xf = mp + 7 * nb * sm; w.Q = mp + 8 * nb * sm;
-  double* dp = (double*)(w.Q + (size_t)nb * ld * kClusterMax);
-  w.lam = dp; w.ev = dp + nb * ld; w.anorm = dp + 2 * nb * ld; w.dlt = w.anorm + nb;
-  int* ip = (int*)(w.dlt + nb);
-  w.conv = ip; w.rdone = ip + nb; w.fallback = ip + nb + 1; w.cinfo = ip + nb + 2;
-  const double tol = tol_rel > 0.0 ? tol_rel : 1e-13;
-  ref_init_kernel<<<nb, 1024, 0, st>>>(ld, nper, A, sA, w);
-  HFB_CHECK_LAUNCH();
-  int r;
-  for (int k = 0; k < kRefMaxIt; ++k) {
-    double2* Xc = (k % 2 == 0) ? w.X0 : w.X1;
-    double2* Xn = (k % 2 == 0) ? w.X1 : w.X0;
-    if ((r = zgemm_small(ld, ld, 0, 0, w.Ah, sm, Xc, sm, w.AX, sm, nper, nb, st, 1.0, 0.0, w.rdone, k))) return r;
-    if ((r = zgemm_small(ld, ld, 1, 0, Xc, sm, w.AX, sm, w.S, sm, nper, nb, st, 1.0, 0.0, w.rdone, k))) return r;
-    if ((r = zgemm_small(ld, ld, 1, 0, Xc, sm, Xc, sm, w.R, sm, nper, nb, st, -1.0, 1.0, w.rdone, k))) return r;
-    ref_update_kernel<<<nb, 1024, 0, st>>>(ld, nper, w, k, tol);
-    HFB_CHECK_LAUNCH();
-    ref_check_kernel<<<1, 1, 0, st>>>(nb, w, k);
-    HFB_CHECK_LAUNCH();
-    if ((r = zgemm_small(ld, ld, 0, 0, Xc, sm, w.E, sm, Xn, sm, nper, nb, st, 1.0, 0.0, w.rdone, k))) return r;
-  }
-  ref_final_x_kernel<<<dim3(32, nb), 256, 0, st>>>(ld, nper, w);
-  HFB_CHECK_LAUNCH();
-  if ((r = zgemm_small(ld, ld, 0, 0, w.Ah, sm, w.Xf, sm, w.AX, sm, nper, nb, st))) return r;
-  if ((r = zgemm_small(ld, ld, 1, 0, w.Xf, sm, w.AX, sm, w.S, sm, nper, nb, st))) return r;
-  ref_cluster_kernel<<<nb, 256, 0, st>>>(ld, nper, w);
-  HFB_CHECK_LAUNCH();
-  ref_assemble_kernel<<<dim3(32, nb), 256, 0, st>>>(ld, nper, w, W, sW, V, sV);
-  HFB_CHECK_LAUNCH();
-  // accept only pairs that diagonalise A to the requested accuracy
-  if ((r = zgemm_small(ld, ld, 0, 0, w.Ah, sm, V, sV, w.AX, sm, nper, nb, st))) return r;
-  if ((r = zgemm_small(ld, ld, 1, 0, V, sV, w.AX, sm, w.S, sm, nper, nb, st))) return r;
-  if ((r = zgemm_small(ld, ld, 1, 0, V, sV, V, sV, w.R, sm, nper, nb, st, -1.0, 1.0))) return r;
-  ref_accept_kernel<<<nb, 1024, 0, st>>>(ld, nper, w, W, sW, fmax(1e3 * tol, 1e-11), fmax(1e3 * tol, 1e-11));
-  HFB_CHECK_LAUNCH();
-  // Jacobi for the cases the refinement leaves (runs only when *fallback)
+  int* fallback = (int*)(buf + wb);
+  const RefineArgs a{nper, ld, A, sA, W, sW, V, sV, tol_rel > 0.0 ? tol_rel : 1e-13, fallback};
+  const int r = refine_launch(nb, a, buf, st);
+  if (r) return r;
   EighBatch eb{};
   eb.tol_rel = tol_rel;
-  eb.gate = w.fallback;
+  eb.gate = fallback;
   for (int b = 0; b < nb; ++b) {
     eb.n[eb.nb] = nper.v[b];
     eb.lda[eb.nb] = ld;
@@ -1274,123 +819,6 @@ static int eigh_refine(hfb_ctx_s* c, int nb, Pair2 nper, int ld, const double2* 
     ++eb.nb;
   }
   return eigh_batch(c, eb, st);
-}
-
-// Y0, Z0, Y1, Z1, T: work matrices [2][ld][ld] each; S: [2] with stride sS.
-static int loewdin_ns(hfb_ctx_s* c, int ld, Pair2 nper, const double2* S, size_t sS, double2* Y0, double2* Z0,
-                      double2* Y1, double2* Z1, double2* T, double* cinv, int* gate, double2* U, cudaStream_t st) {
-  const size_t sm = (size_t)ld * ld;
-  ns_init_kernel<<<2, 256, 0, st>>>(ld, nper, S, sS, Y0, Z0, sm, cinv, gate);
-  HFB_CHECK_LAUNCH();
-  int r;
-  for (int k = 0; k < kNSMaxIt; ++k) {
-    double2* Yc = (k % 2 == 0) ? Y0 : Y1;
-    double2* Zc = (k % 2 == 0) ? Z0 : Z1;
-    double2* Yn = (k % 2 == 0) ? Y1 : Y0;
-    double2* Zn = (k % 2 == 0) ? Z1 : Z0;
-    if ((r = zgemm_small(ld, ld, 0, 0, Zc, sm, Yc, sm, T, sm, nper, 2, st, -0.5, 1.5, gate, k))) return r;
-    ns_check_kernel<<<1, 1024, 0, st>>>(ld, nper, T, sm, gate, k);
-    HFB_CHECK_LAUNCH();
-    if ((r = zgemm_small(ld, ld, 0, 0, Yc, sm, T, sm, Yn, sm, nper, 2, st, 1.0, 0.0, gate, k))) return r;
-    if ((r = zgemm_small(ld, ld, 0, 0, T, sm, Zc, sm, Zn, sm, nper, 2, st, 1.0, 0.0, gate, k))) return r;
-  }
-  ns_final_kernel<<<dim3(32, 2), 256, 0, st>>>(ld, nper, Z0, Z1, sm, cinv, gate, U, c->dev_status);
-  HFB_CHECK_LAUNCH();
-  return HFB_OK;
-}
-
-// T = V diag(1/sqrt(max(w, thr))) with thr = max(1e-12, eps max(w) n) (static.py:473-479)
-__global__ void loewdin_scale_kernel(int ld, Pair2 nper, const double* w, size_t sw, const double2* V,
-                                     double2* T, size_t sm) {
-  const int b = blockIdx.y;
-  const int n = nper.v[b];
-  const double* wb = w + b * sw;
-  __shared__ double thr;
-  if (threadIdx.x == 0) {
-    double mx = wb[0];
-    for (int k = 1; k < n; ++k) mx = fmax(mx, wb[k]);
-    thr = fmax(1e-12, 2.220446049250313e-16 * mx * n);
-  }
-  __syncthreads();
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double s = 1.0 / sqrt(fmax(wb[j], thr));
-    const double2 v = V[b * sm + (size_t)i * ld + j];
-    T[b * sm + (size_t)i * ld + j] = make_double2(v.x * s, v.y * s);
-  }
-}
-
-// Copy the diagonal's real part (sp_norm), and the lower-Hermitian lambda.
-__global__ void diag_real_kernel(int ld, Pair2 nper, Pair2 off, const double2* S, size_t sm, double* out) {
-  const int b = blockIdx.x;
-  for (int k = threadIdx.x; k < nper.v[b]; k += blockDim.x) out[off.v[b] + k] = S[b * sm + (size_t)k * ld + k].x;
-}
-
-// construct_hfb_matrices after h, gap are in the new basis (static.py:511-575).
-// One CTA per isospin.  H, G: [b][ld][ld]; writes hmatrix, gapmatrix,
-// symcond, lambda_save [b][nmax][nmax], sp_energy, deltaf, efluct.
-__global__ void __launch_bounds__(1024)
-lambda_kernel(int ld, int nmax, Pair2 nper, Pair2 off, int ipair, int tbcs, const double2* H,
-              const double2* G, size_t sm, const double* wocc, const double* wguv, const double* pairwg,
-              const double* wstates, double2* hmat, double2* gmat, double2* symc, double2* lsave, double* sp_energy,
-              double* deltaf, double* efluct) {
-  const int b = blockIdx.x;
-  const int n = nper.v[b], o = off.v[b];
-  __shared__ double red_max[32], red_sum[32];
-  const double2* Hb = H + b * sm;
-  const double2* Gb = G + b * sm;
-  double mx = 0.0, sm2 = 0.0;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e / n, j = e % n;
-    const double2 h = Hb[(size_t)i * ld + j];
-    const double2 ht = Hb[(size_t)j * ld + i];
-    double2 g = ipair ? Gb[(size_t)i * ld + j] : make_double2(0, 0);
-    double2 gt = ipair ? Gb[(size_t)j * ld + i] : make_double2(0, 0);
-    hmat[((size_t)b * nmax + i) * nmax + j] = h;
-    if (tbcs && i != j) { g = make_double2(0, 0); }
-    if (tbcs && i != j) { gt = make_double2(0, 0); }
-    gmat[((size_t)b * nmax + i) * nmax + j] = g;
-    // lambda_ij = w_j h_ij - wuv_j g_ij ; lambda^H_ij = conj(lambda_ji)
-    const double wj = wocc[o + j] * wstates[o + j], wi = wocc[o + i] * wstates[o + i];
-    const double uj = wguv[o + j] * pairwg[o + j] * wstates[o + j];
-    const double ui = wguv[o + i] * pairwg[o + i] * wstates[o + i];
-    const double2 l = make_double2(wj * h.x - uj * g.x, wj * h.y - uj * g.y);
-    const double2 lt = make_double2(wi * ht.x - ui * gt.x, -(wi * ht.y - ui * gt.y));   // conj(lambda_ji)
-    const double2 as = make_double2(0.5 * (l.x - lt.x), 0.5 * (l.y - lt.y));
-    const double2 sy = make_double2(0.5 * (l.x + lt.x), 0.5 * (l.y + lt.y));
-    symc[((size_t)b * nmax + i) * nmax + j] = as;
-    lsave[((size_t)b * nmax + i) * nmax + j] = sy;
-    const double ab = hypot(as.x, as.y);
-    mx = fmax(mx, ab);
-    sm2 += ab * ab;
-  }
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    sp_energy[o + k] = Hb[(size_t)k * ld + k].x;
-    if (ipair) deltaf[o + k] = Gb[(size_t)k * ld + k].x * pairwg[o + k];
-  }
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-    sm2 += __shfl_xor_sync(0xffffffffu, sm2, s);
-  }
-  if (threadIdx.x % 32 == 0) { red_max[threadIdx.x / 32] = mx; red_sum[threadIdx.x / 32] = sm2; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, s = 0;
-    for (int k = 0; k < (int)(blockDim.x / 32); ++k) { a = fmax(a, red_max[k]); s += red_sum[k]; }
-    efluct[b] = a;
-    efluct[2 + b] = sqrt(s / ((double)n * n));
-  }
-}
-
-// lsave [b][nmax][nmax] -> L [b][ld][ld] (lambda used for the Lagrange update)
-__global__ void copy_lambda_kernel(int ld, int nmax, Pair2 nper, const double2* lsave, double2* L, size_t sm) {
-  const int b = blockIdx.y;
-  const int n = nper.v[b];
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
-    const int i = e / n, j = e % n;
-    L[b * sm + (size_t)i * ld + j] = lsave[((size_t)b * nmax + i) * nmax + j];
-  }
 }
 
 // ============================================================== rotate ====
@@ -1720,7 +1148,7 @@ extern "C" int hfb_eigh(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, 
 extern "C" int hfb_eigh_near_diagonal(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w,
                                       double* v, void* stream) {
   if (!ctx || !a || !w || !v || n <= 0 || lda < n || nb <= 0) return HFB_ERR_ARG;
-  if (lda > kRefMaxN) return HFB_ERR_UNSUPPORTED_GRID;
+  if (lda > 256) return HFB_ERR_UNSUPPORTED_GRID;
   cudaStream_t st = as_stream(stream);
   const size_t mstride = (size_t)n * lda;
   for (int b0 = 0; b0 < nb; b0 += 2) {
@@ -1746,41 +1174,38 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
   const int ld = n0 > n1 ? n0 : n1;
   const size_t sm = (size_t)ld * ld;
   const size_t n3 = (size_t)ctx->n * ctx->n * ctx->n;
-  // workspace: 4 Gram matrices + 10 work matrices per isospin, eigenvalues,
-  // Newton-Schulz scalars
-  const size_t nmat = 2 * (4 + 10);
+  // workspace per isospin: 4 Gram matrices, S^-1/2, the eigenvectors of
+  // lambda, U and U lambda; then the eigenvalues and the chains' own work
+  const size_t wl = loewdin_bytes(ld), wc = construct_bytes(ld);
   char* ws = (char*)scratch(ctx, hfb_ctx_s::S_SMALL,
-                            sizeof(double2) * nmat * sm + sizeof(double) * 4 * ld + 8 * sizeof(double));
+                            sizeof(double2) * 16 * sm + sizeof(double) * 2 * ld + (wl > wc ? wl : wc));
   if (!ws) return HFB_ERR_ALLOC;
   double2* gm = (double2*)ws;                 // [iq][4][ld][ld]: S, Lambda, H_old, G_old
-  double2* Y0 = gm + 2 * 4 * sm;              // Newton-Schulz work
-  double2* Z0 = Y0 + 2 * sm;
-  double2* Y1 = Z0 + 2 * sm;
-  double2* Z1 = Y1 + 2 * sm;
-  double2* T = Z1 + 2 * sm;                   // scratch
-  double2* Ur = T + 2 * sm;                   // S^-1/2
+  double2* Ur = gm + 8 * sm;                  // S^-1/2
   double2* Vl = Ur + 2 * sm;                  // eigenvectors of lambda
   double2* U = Vl + 2 * sm;                   // total transform
-  double2* Hn = U + 2 * sm;                   // U^H H U
-  double2* Gn = Hn + 2 * sm;                  // U^H G U
-  double2* Lw = Gn;                           // U lambda (Gn is dead by then)
-  double* w = (double*)(Gn + 2 * sm);         // [iq][ld] (x2: unused, lambda)
-  double* cinv = w + 4 * ld;
-  int* gate = (int*)(cinv + 4);
+  double2* Lw = U + 2 * sm;                   // U lambda
+  double* w = (double*)(Lw + 2 * sm);         // [iq][ld] eigenvalues of lambda
+  void* work = w + 2 * ld;                    // loewdin, then construct
   Pair2 nper, off;
   nper.v[0] = n0; nper.v[1] = n1;
   off.v[0] = 0; off.v[1] = n0;
   const int nq[2] = {n0, n1}, so[2] = {0, n0};
   int r;
-  // The eigensolve of lambda runs on the side stream on a few SMs.  H and G
-  // are needed only by the construct step after it, so when both are asked
-  // for, the Gram launch computes S and lambda first and H, G follow on the
-  // main stream while the eigensolve runs (HFB_GRAM_SPLIT=0: one launch).
+  // The eigensolve of lambda takes a few SMs and follows the first Gram
+  // launch on the calling stream.  S^-1/2 needs S only and runs beside it on
+  // the second side stream.  H and G are needed only by the construct step,
+  // so when they are asked for, the first Gram launch computes S and lambda
+  // and H, G follow on the side stream (HFB_GRAM_SPLIT=0: one launch).  The
+  // chains go first and the H, G launch, which fills the SMs, one event
+  // later: a chain that finds the SMs full starts when the launch ends
+  // (measured on Pb208 FP64: 2.9 ms late, iteration 34.7 ms against 32.2 ms).
   int mask = 1;
   if (a->diagonalize) mask |= 2;
   if (a->construct) mask |= 4;
   if (a->construct && a->ipair) mask |= 8;
-  const bool split = a->diagonalize && a->construct && ctx->side && ctx->gram_split;
+  const bool beside = a->diagonalize && ctx->side2;
+  const bool split = beside && a->construct && ctx->side && ctx->gram_split;
   const double* vp[2] = {a->v_pair, a->v_pair ? a->v_pair + n3 : nullptr};
   double2* outs[8];
   for (int iq = 0; iq < 2; ++iq)
@@ -1791,28 +1216,20 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
     r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, st);
     if (r) return r;
   }
-  diag_real_kernel<<<2, 256, 0, st>>>(ld, nper, off, gm, 4 * sm, a->sp_norm);
-  HFB_CHECK_LAUNCH();
-  // Newton-Schulz needs S only: with the split Gram it runs on a second side
-  // stream, beside the H, G launch and the eigensolve, on the SMs they leave
-  const bool ns_side = split && ctx->side2;
   cudaStream_t nst = st;
-  if (ns_side) {
-    cudaEventRecord(ctx->ev_fork2, st);
-    cudaStreamWaitEvent(ctx->side2, ctx->ev_fork2, 0);
+  if (beside) {
+    cudaEventRecord(ctx->ev_fork, st);
+    cudaStreamWaitEvent(ctx->side2, ctx->ev_fork, 0);
+    if (split) cudaEventRecord(ctx->ev_fork2, ctx->side2);
     nst = ctx->side2;
   }
-  // eigh of lambda (Jacobi, one CTA per isospin, or the refinement) on the
-  // side stream while the main stream runs the H, G Gram launch (or, without
-  // the split, the Newton-Schulz GEMMs for S^-1/2)
-  const bool fork = a->diagonalize && ctx->side;
+  // Beside the single-precision Gram launch (one CTA per SM with all its
+  // shared memory, on 144 of the 148 SMs) each isospin takes one SM, which
+  // the launch leaves free; otherwise as many as its products can use.
+  const bool few = split && prec != HFB_F64 && ctx->use_tcgen05;
+  r = loewdin_launch(LoewdinArgs{nper, off, ld, gm, 4 * sm, Ur, a->sp_norm, ctx->dev_status}, work, !few, nst);
+  if (r) return r;
   if (a->diagonalize) {
-    cudaStream_t es = st;
-    if (fork) {
-      cudaEventRecord(ctx->ev_fork, st);
-      cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
-      es = ctx->side;
-    }
     // single-precision states carry rounding noise of 2^-24 relative in
     // lambda; converging below that level refines nothing
     const double tol_rel = prec != HFB_F64 ? 5.9604644775390625e-08 : 0.0;
@@ -1822,7 +1239,7 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
     // ms per Pb208 iteration: in the bulk the refinement's acceptance test
     // fails and the Jacobi runs after it)
     if (ctx->lambda_refine && prec == HFB_F64) {
-      r = eigh_refine(ctx, 2, nper, ld, gm + sm, 4 * sm, w + 2 * ld, ld, Vl, sm, tol_rel, es);
+      r = eigh_refine(ctx, 2, nper, ld, gm + sm, 4 * sm, w, ld, Vl, sm, tol_rel, st);
     } else {
       EighBatch eb{};
       eb.tol_rel = tol_rel;
@@ -1830,27 +1247,26 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
         eb.n[eb.nb] = nq[iq];
         eb.lda[eb.nb] = ld;
         eb.a[eb.nb] = gm + (size_t)iq * 4 * sm + sm;
-        eb.w[eb.nb] = w + 2 * ld + (size_t)iq * ld;
+        eb.w[eb.nb] = w + (size_t)iq * ld;
         eb.v[eb.nb] = Vl + (size_t)iq * sm;
         ++eb.nb;
       }
-      r = eigh_batch(ctx, eb, es);
+      r = eigh_batch(ctx, eb, st);
     }
     if (r) return r;
-    if (fork) cudaEventRecord(ctx->ev_join, ctx->side);
   }
   if (split) {
+    cudaStreamWaitEvent(ctx->side, ctx->ev_fork2, 0);
     const int m2 = mask & 12;
     const int masks[2] = {m2, m2};
-    r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, st);
+    r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, ctx->side);
     if (r) return r;
+    cudaEventRecord(ctx->ev_join, ctx->side);
   }
-  r = loewdin_ns(ctx, ld, nper, gm, 4 * sm, Y0, Z0, Y1, Z1, T, cinv, gate, Ur, nst);
-  if (r) return r;
   // the rotation's transposes of the states depend on psi only: they follow
-  // Newton-Schulz on the second side stream
+  // S^-1/2 on the second side stream
   int pre[2] = {-1, -1};
-  if (ns_side && prec != HFB_F64 && ctx->use_tcgen05) {
+  if (split && prec != HFB_F64 && ctx->use_tcgen05) {
     const size_t Kc = (size_t)2 * n3;
     for (int iq = 0; iq < 2; ++iq) {
       r = rotate_tc_transpose(ctx, iq, nq[iq], (const float2*)a->psi + (size_t)so[iq] * Kc, nst);
@@ -1858,42 +1274,20 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
       else if (r != HFB_ERR_UNSUPPORTED_GRID) return r;
     }
   }
-  if (ns_side) {
+  if (beside) {
     cudaEventRecord(ctx->ev_join2, ctx->side2);
     cudaStreamWaitEvent(st, ctx->ev_join2, 0);
   }
-  double2* Uuse = Ur;
-  if (a->diagonalize) {
-    if (fork) cudaStreamWaitEvent(st, ctx->ev_join, 0);
-    r = zgemm_small(ld, ld, 0, 0, Ur, sm, Vl, sm, U, sm, nper, 2, st);
-    if (r) return r;
-    Uuse = U;
-  }
-  const int nmax = a->nmax;
-  if (a->construct) {
-    // H = U^H (H_old U), G likewise
-    r = zgemm_small(ld, ld, 0, 0, gm + 2 * sm, 4 * sm, Uuse, sm, T, sm, nper, 2, st);
-    if (r) return r;
-    r = zgemm_small(ld, ld, 1, 0, Uuse, sm, T, sm, Hn, sm, nper, 2, st);
-    if (r) return r;
-    if (a->ipair) {
-      r = zgemm_small(ld, ld, 0, 0, gm + 3 * sm, 4 * sm, Uuse, sm, T, sm, nper, 2, st);
-      if (r) return r;
-      r = zgemm_small(ld, ld, 1, 0, Uuse, sm, T, sm, Gn, sm, nper, 2, st);
-      if (r) return r;
-    }
-    lambda_kernel<<<2, 1024, 0, st>>>(ld, nmax, nper, off, a->ipair, a->tbcs, Hn, Gn, sm, a->wocc, a->wguv, a->pairwg,
-                                      a->wstates, (double2*)a->hmatrix, (double2*)a->gapmatrix, (double2*)a->symcond,
-                                      (double2*)a->lambda_save, a->sp_energy, a->deltaf, a->efluct);
-    HFB_CHECK_LAUNCH();
-  }
-  // L = U lambda_save (lambda_save just written when construct)
-  copy_lambda_kernel<<<dim3(64, 2), 256, 0, st>>>(ld, nmax, nper, (const double2*)a->lambda_save, T, sm);
-  HFB_CHECK_LAUNCH();
-  r = zgemm_small(ld, ld, 0, 0, Uuse, sm, T, sm, Lw, sm, nper, 2, st);
+  if (split) cudaStreamWaitEvent(st, ctx->ev_join, 0);
+  r = construct_launch(
+      ConstructArgs{nper, off, ld, a->nmax, a->diagonalize, a->construct, a->ipair, a->tbcs, Ur, Vl, U, gm + 2 * sm,
+                    gm + 3 * sm, 4 * sm, Lw, a->wocc, a->wguv, a->pairwg, a->wstates, (double2*)a->hmatrix,
+                    (double2*)a->gapmatrix, (double2*)a->symcond, (double2*)a->lambda_save, a->sp_energy, a->deltaf,
+                    a->efluct},
+      work, st);
   if (r) return r;
   for (int iq = 0; iq < 2; ++iq) {
-    r = rotate_launch(ctx, prec, so[iq], nq[iq], a->psi, Uuse + (size_t)iq * sm, Lw + (size_t)iq * sm, ld, a->psi_out,
+    r = rotate_launch(ctx, prec, so[iq], nq[iq], a->psi, U + (size_t)iq * sm, Lw + (size_t)iq * sm, ld, a->psi_out,
                       a->lagrange, st, pre[iq]);
     if (r) return r;
   }
