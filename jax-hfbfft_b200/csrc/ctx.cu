@@ -119,6 +119,11 @@ extern "C" int hfb_ctx_create(int nx, int ny, int nz, double dx, double dy, doub
     free(c);
     return HFB_ERR_CUDA;
   }
+  if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess) {
+    cudaGetLastError();
+    free(c);
+    return HFB_ERR_CUDA;
+  }
   c->n2 = periodic ? nx : 2 * nx;
   {
     const char* e = getenv("HFB_NO_TCGEN05");
@@ -155,11 +160,11 @@ extern "C" int hfb_ctx_create(int nx, int ny, int nz, double dx, double dy, doub
     cudaMemcpy(c->der1[a], d1.data(), nn * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(c->der2[a], d2.data(), nn * sizeof(double), cudaMemcpyHostToDevice);
   }
-  if (cudaMalloc(&c->dev_status, 2 * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&c->dev_status, 4 * sizeof(int)) != cudaSuccess) {
     hfb_ctx_destroy(c);
     return HFB_ERR_ALLOC;
   }
-  cudaMemset(c->dev_status, 0, 2 * sizeof(int));
+  cudaMemset(c->dev_status, 0, 4 * sizeof(int));
   c->counters = c->dev_status + 1;
   if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||

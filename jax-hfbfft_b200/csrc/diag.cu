@@ -113,124 +113,6 @@ gram_kernel(GramJob job, size_t K, size_t n3, const cplx<R>* __restrict__ psi, c
       o[(ty + 12 * u) * GT + tx + 16 * v] = make_double2((double)acc[u][v][0], (double)acc[u][v][1]);
 }
 
-// FP64 states: the same tiles, split-K chunks and partial layout on the
-// FP64 tensor cores (mma.sync m8n8k4 .f64).  Over the interleaved storage,
-// with k' running over (Re, Im) of each element,
-//   Re C_ij = sum_k' a_ik' b_jk',   a = psi_i, b = x_j,
-//   Im C_ij = sum_k' a_ik' bt_jk',  bt = (Im x, -Re x) per element,
-// so each 8 x 8 output block takes two real MMAs per four k'; bt is b with
-// the partner lane's value (one shuffle).  A CTA (4 warps, 24 x 24 outputs
-// per warp, 3 x 3 MMA blocks) streams K in stages of GD_KB elements through
-// cp.async double buffers (rows padded by one element: the 8 rows a
-// fragment load touches fall on distinct bank groups).
-constexpr int GD_KB = 16;              // complex k per shared-memory stage
-constexpr int GD_LD = GD_KB + 1;       // padded row length (complex)
-constexpr int GD_THREADS = 128;
-constexpr size_t GD_SMEM = sizeof(double2) * 2 * 2 * GT * GD_LD;
-
-__device__ __forceinline__ void gd_cp16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
-               "l"(gmem)
-               : "memory");
-}
-
-__global__ void __launch_bounds__(GD_THREADS) gram_dmma_kernel(GramJob job, size_t K, size_t n3,
-                                                                const double2* __restrict__ psi,
-                                                                const double2* __restrict__ hampsi,
-                                                                const double2* __restrict__ hmfpsi, double2* part,
-                                                                int nchunk, int kchunk) {
-  extern __shared__ double2 gd_smem[];
-  double2* As = gd_smem;                 // [2][GT][GD_LD]
-  double2* Bs = gd_smem + 2 * GT * GD_LD;
-  const GramTile tl = job.t[blockIdx.x];
-  const int b = tl.b, am = tl.a;
-  const int ns = job.ns[b];
-  const int i0 = tl.ti * GT, j0 = tl.tj * GT;
-  const double2* P = psi + (size_t)job.s0[b] * K;
-  const double2* X = am == 1 ? hampsi + (size_t)job.s0[b] * K : am == 2 ? hmfpsi + (size_t)job.s0[b] * K : P;
-  const double* vp = job.vp[b];
-  const size_t k0 = (size_t)blockIdx.y * kchunk;
-  const size_t k1 = min(K, k0 + (size_t)kchunk);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rw = warp >> 1, cw = warp & 1;
-  const int fr = lane >> 2, fk = lane & 3;   // fragment row (A) / column (B), k' within the 4
-  double accR[3][3][2], accI[3][3][2];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) accR[i][j][0] = accR[i][j][1] = accI[i][j][0] = accI[i][j][1] = 0.0;
-  // one stage: GT rows x GD_KB elements of each operand, consecutive
-  // threads on consecutive elements of a row (coalesced)
-  auto load = [&](int buf, size_t kb) {
-#pragma unroll
-    for (int h = 0; h < GT * GD_KB / GD_THREADS; ++h) {
-      const int e = threadIdx.x + GD_THREADS * h;
-      const int r = e / GD_KB, kk = e % GD_KB;
-      const size_t k = kb + kk;
-      double2* da = As + ((size_t)buf * GT + r) * GD_LD + kk;
-      double2* db = Bs + ((size_t)buf * GT + r) * GD_LD + kk;
-      const int gi = i0 + r, gj = j0 + r;
-      if (k < k1 && gi < ns) gd_cp16(da, P + (size_t)gi * K + k);
-      else *da = make_double2(0.0, 0.0);
-      if (k < k1 && gj < ns) {
-        if (am == 3) {
-          const double2 v = X[(size_t)gj * K + k];
-          const double w = vp[k % n3];
-          *db = make_double2(w * v.x, w * v.y);
-        } else {
-          gd_cp16(db, X + (size_t)gj * K + k);
-        }
-      } else {
-        *db = make_double2(0.0, 0.0);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  load(0, k0);
-  int buf = 0;
-  for (size_t kb = k0; kb < k1; kb += GD_KB) {
-    if (kb + GD_KB < k1) {
-      load(buf ^ 1, kb + GD_KB);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-    __syncthreads();
-    const double* A = reinterpret_cast<const double*>(As + (size_t)buf * GT * GD_LD);
-    const double* B = reinterpret_cast<const double*>(Bs + (size_t)buf * GT * GD_LD);
-#pragma unroll 4
-    for (int ks = 0; ks < GD_KB / 2; ++ks) {
-      const int kd = 2 * (2 * ks) + fk;      // double index of k' in the row
-      double a[3], bv[3], bt[3];
-#pragma unroll
-      for (int mi = 0; mi < 3; ++mi) a[mi] = A[(24 * rw + 8 * mi + fr) * (2 * GD_LD) + kd];
-#pragma unroll
-      for (int nj = 0; nj < 3; ++nj) {
-        bv[nj] = B[(24 * cw + 8 * nj + fr) * (2 * GD_LD) + kd];
-        const double o = __shfl_xor_sync(0xffffffffu, bv[nj], 1);
-        bt[nj] = (fk & 1) ? -o : o;
-      }
-#pragma unroll
-      for (int mi = 0; mi < 3; ++mi)
-#pragma unroll
-        for (int nj = 0; nj < 3; ++nj) {
-          gd_mma(accR[mi][nj], a[mi], bv[nj]);
-          gd_mma(accI[mi][nj], a[mi], bt[nj]);
-        }
-    }
-    __syncthreads();
-    buf ^= 1;
-  }
-  double2* o = part + ((size_t)blockIdx.x * nchunk + blockIdx.y) * GT * GT;
-#pragma unroll
-  for (int mi = 0; mi < 3; ++mi)
-#pragma unroll
-    for (int nj = 0; nj < 3; ++nj)
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        o[(24 * rw + 8 * mi + fr) * GT + 24 * cw + 8 * nj + 2 * fk + i] = make_double2(accR[mi][nj][i], accI[mi][nj][i]);
-}
-
 struct GramOut {
   double2* p[8];   // [block * 4 + matrix]
 };
@@ -267,14 +149,16 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
                    double2* const* outs_host, int ldo, cudaStream_t st);   // gram_tc.cu
 
 // One launch for the requested matrices of up to two state blocks.
-// outs[b * 4 + a] receives matrix a of block b (leading dimension ldo).
+// outs[b * 4 + a] receives matrix a of block b (leading dimension ldo); the
+// FP64 tensor-core launch stays off ``leave`` SMs.
 
 int gram_launch(hfb_ctx_s* c, int prec, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
                 const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz, double2* const* outs_host,
-                int ldo, cudaStream_t st) {
+                int ldo, cudaStream_t st, int leave = 0) {
   // single precision: tensor cores (three-term tf32) unless disabled for this context
   if (prec != HFB_F64 && c->use_tcgen05) {
-    const int r = gram_tc_launch(c, nblk, s0, ns, masks, psi, hampsi, hmfpsi, vp, wxyz, outs_host, ldo, st);
+    const int mk[2] = {masks[0] & 15, nblk > 1 ? masks[1] & 15 : 0};
+    const int r = gram_tc_launch(c, nblk, s0, ns, mk, psi, hampsi, hmfpsi, vp, wxyz, outs_host, ldo, st);
     if (r != HFB_ERR_UNSUPPORTED_GRID) return r;
   }
   const size_t n3 = (size_t)c->n * c->n * c->n, K = 2 * n3;
@@ -297,6 +181,8 @@ int gram_launch(hfb_ctx_s* c, int prec, int nblk, const int* s0, const int* ns, 
     }
   }
   if (job.ntile == 0) return HFB_OK;
+  if (prec == HFB_F64 && c->f64_mma)
+    return gram_f64_launch(c, nblk, s0, ns, masks, psi, hampsi, hmfpsi, vp, wxyz, outs_host, ldo, leave, st);
   // split K so that the grid has about two CTAs per SM even for few tiles
   // and short K (small grids): chunks a multiple of 64 elements, at most
   // GCHUNK
@@ -314,14 +200,7 @@ int gram_launch(hfb_ctx_s* c, int prec, int nblk, const int* s0, const int* ns, 
   GramOut ot;
   for (int q = 0; q < 8; ++q) ot.p[q] = outs_host[q];
   dim3 grid(job.ntile, nchunk);
-  if (prec == HFB_F64 && c->f64_mma) {
-    static const bool smem_ok =
-        cudaFuncSetAttribute(gram_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GD_SMEM) ==
-        cudaSuccess;
-    if (!smem_ok) return HFB_ERR_CUDA;
-    gram_dmma_kernel<<<grid, GD_THREADS, GD_SMEM, st>>>(job, K, n3, (const double2*)psi, (const double2*)hampsi,
-                                                     (const double2*)hmfpsi, part, nchunk, kchunk);
-  } else if (prec == HFB_F64)
+  if (prec == HFB_F64)
     gram_kernel<double><<<grid, GTHREADS, 0, st>>>(job, K, n3, (const double2*)psi, (const double2*)hampsi,
                                               (const double2*)hmfpsi, part, nchunk, kchunk);
   else
@@ -894,97 +773,6 @@ rotate_kernel(int ns, size_t K, const cplx<R>* __restrict__ psi, const double2* 
   }
 }
 
-// FP64 states on the FP64 tensor cores (mma.sync m8n8k4 .f64): with the
-// state index interleaved with (Re, Im), i' = 2 i + part,
-//   A'[k][i'] = (Re, Im) psi_i(k),
-//   Re out_j(k) = sum_i' A'[k][i'] Br[i'][j],  Br = (Re W_ij, -Im W_ij),
-//   Im out_j(k) = sum_i' A'[k][i'] Bi[i'][j],  Bi = (Im W_ij,  Re W_ij),
-// W = [U | L].  A CTA (8 warps, 4 along k x 2 along j, 32 x 32 outputs
-// per warp, 4 x 4 MMA blocks) computes 128 grid points x 64 outputs,
-// streaming the states in double-buffered stages of 4.
-constexpr int RD_KT = 128, RD_JT = 64, RD_IT = 4;
-
-__global__ void __launch_bounds__(256) rotate_dmma_kernel(int ns, size_t K, const double2* __restrict__ psi,
-                                                          const double2* __restrict__ U,
-                                                          const double2* __restrict__ L, int ld, double2* out1,
-                                                          double2* out2) {
-  __shared__ double2 Ps[2][RD_IT][RD_KT + 1];
-  __shared__ double2 Ws[2][RD_IT][RD_JT + 1];
-  const int njt = (2 * ns + RD_JT - 1) / RD_JT;
-  const int jt = blockIdx.x % njt;
-  const size_t k0 = (size_t)(blockIdx.x / njt) * RD_KT;
-  const int j0 = jt * RD_JT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wk = warp & 3, wj = warp >> 2;
-  const int fr = lane >> 2, fk = lane & 3;
-  double accR[4][4][2], accI[4][4][2];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) accR[u][v][0] = accR[u][v][1] = accI[u][v][0] = accI[u][v][1] = 0.0;
-  auto load = [&](int buf, int i0) {
-    for (int e = threadIdx.x; e < RD_IT * RD_KT; e += 256) {
-      const int ii = e / RD_KT, kk = e % RD_KT;
-      const size_t k = k0 + kk;
-      Ps[buf][ii][kk] = (i0 + ii < ns && k < K) ? psi[(size_t)(i0 + ii) * K + k] : make_double2(0.0, 0.0);
-    }
-    for (int e = threadIdx.x; e < RD_IT * RD_JT; e += 256) {
-      const int ii = e / RD_JT, jj = e % RD_JT;
-      const int j = j0 + jj;
-      double2 w = make_double2(0.0, 0.0);
-      if (i0 + ii < ns && j < 2 * ns)
-        w = j < ns ? U[(size_t)(i0 + ii) * ld + j] : L[(size_t)(i0 + ii) * ld + (j - ns)];
-      Ws[buf][ii][jj] = w;
-    }
-  };
-  load(0, 0);
-  __syncthreads();
-  int buf = 0;
-  for (int i0 = 0; i0 < ns; i0 += RD_IT) {
-    if (i0 + RD_IT < ns) load(buf ^ 1, i0 + RD_IT);
-#pragma unroll
-    for (int kk = 0; kk < RD_IT / 2; ++kk) {
-      const int ii = 2 * kk + (fk >> 1);     // state of this lane's k' within the step
-      const bool im = fk & 1;
-      double a[4], br[4], bi[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const double2 p = Ps[buf][ii][32 * wk + 8 * u + fr];
-        a[u] = im ? p.y : p.x;
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const double2 w = Ws[buf][ii][32 * wj + 8 * v + fr];
-        br[v] = im ? -w.y : w.x;
-        bi[v] = im ? w.x : w.y;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          gd_mma(accR[u][v], a[u], br[v]);
-          gd_mma(accI[u][v], a[u], bi[v]);
-        }
-    }
-    __syncthreads();
-    buf ^= 1;
-  }
-  // the thread holds rows k = 32 wk + 8 u + fr, columns j = 32 wj + 8 v + 2 fk + c
-#pragma unroll
-  for (int v = 0; v < 4; ++v)
-#pragma unroll
-    for (int c2 = 0; c2 < 2; ++c2) {
-      const int j = j0 + 32 * wj + 8 * v + 2 * fk + c2;
-      if (j >= 2 * ns) continue;
-      double2* o = j < ns ? out1 + (size_t)j * K : out2 + (size_t)(j - ns) * K;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const size_t k = k0 + 32 * wk + 8 * u + fr;
-        if (k < K) o[k] = make_double2(accR[u][v][c2], accI[u][v][c2]);
-      }
-    }
-}
-
 // Single-precision variant with a larger register tile: 128 (k) x 96 (j)
 // per CTA, 256 threads holding 8 x 6 complex accumulators each (48
 // independent chains), 8 states per double-buffered shared-memory stage.
@@ -1095,6 +883,8 @@ int rotate_tc_transpose(hfb_ctx_s* c, int which, int ns, const void* psi, cudaSt
 int rotate_launch(hfb_ctx_s* c, int prec, int s0, int ns, const void* psi, const double2* U, const double2* L, int ld,
                   void* out1, void* out2, cudaStream_t st, int pre) {
   if (ns <= 0) return HFB_OK;
+  if (prec == HFB_F64 && c->f64_mma)
+    return rotate_f64_launch(c, 1, &s0, &ns, psi, &U, &L, ld, out1, out2, st);
   if (prec != HFB_F64 && c->use_tcgen05) {
     const size_t Kc = (size_t)2 * c->n * c->n * c->n, offc = (size_t)s0 * Kc;
     const int r = rotate_tc_launch(c, ns, (const float2*)psi + offc, U, L, ld, (float2*)out1 + offc,
@@ -1105,12 +895,7 @@ int rotate_launch(hfb_ctx_s* c, int prec, int s0, int ns, const void* psi, const
   const int njt = (2 * ns + 63) / 64;
   const size_t nkt = (K + 63) / 64;
   const size_t off = (size_t)s0 * K;
-  if (prec == HFB_F64 && c->f64_mma) {
-    const int njd = (2 * ns + RD_JT - 1) / RD_JT;
-    const size_t nkd = (K + RD_KT - 1) / RD_KT;
-    rotate_dmma_kernel<<<(unsigned)(nkd * njd), 256, 0, st>>>(ns, K, (const double2*)psi + off, U, L, ld,
-                                                             (double2*)out1 + off, (double2*)out2 + off);
-  } else if (prec == HFB_F64)
+  if (prec == HFB_F64)
     rotate_kernel<double><<<(unsigned)(nkt * njt), 256, 0, st>>>(ns, K, (const double2*)psi + off, U, L, ld,
                                                                  (double2*)out1 + off, (double2*)out2 + off);
   else {
@@ -1136,6 +921,7 @@ extern "C" int hfb_gram(hfb_ctx_t ctx, int prec, int s0, int ns, int mask, const
   double2* outs[8] = {o, o + (size_t)ns * ns, o + 2 * (size_t)ns * ns, o + 3 * (size_t)ns * ns,
                       nullptr, nullptr, nullptr, nullptr};
   const double* vp[2] = {v_pair_iq, nullptr};
+  mask &= 15;
   return gram_launch(ctx, prec, 1, &s0, &ns, &mask, psi, hampsi, hmfpsi, vp, wxyz, outs, ns, as_stream(stream));
 }
 
@@ -1192,26 +978,30 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
   off.v[0] = 0; off.v[1] = n0;
   const int nq[2] = {n0, n1}, so[2] = {0, n0};
   int r;
-  // The eigensolve of lambda takes a few SMs and follows the first Gram
-  // launch on the calling stream.  S^-1/2 needs S only and runs beside it on
-  // the second side stream.  H and G are needed only by the construct step,
-  // so when they are asked for, the first Gram launch computes S and lambda
-  // and H, G follow on the side stream (HFB_GRAM_SPLIT=0: one launch).  The
-  // chains go first and the H, G launch, which fills the SMs, one event
-  // later: a chain that finds the SMs full starts when the launch ends
-  // (measured on Pb208 FP64: 2.9 ms late, iteration 34.7 ms against 32.2 ms).
+  // The eigensolve of lambda and S^-1/2 need the first Gram launch only.  H
+  // and G are needed only by the construct step, so when they are asked for,
+  // the first launch computes S and lambda and the H, G launch runs beside
+  // the two chains (HFB_GRAM_SPLIT=0: one launch).  A kernel of a chain that
+  // found every SM in use would wait for the launch to drain (2.9 ms on
+  // Pb208 FP64; stream priority did not help, no CTA of the launch ends
+  // early), so the H, G launch comes last and leaves four SMs alone: two for
+  // the Jacobi solver, one for each isospin's S^-1/2.  The refinement, which
+  // is short, takes its SMs before the launch; the launch's CTAs that do not
+  // fit at once follow it.  Pb208 FP64 iteration: 34.7 ms with the H, G
+  // launch first, 32.2 ms with it last, 26.5 ms with contract_f64.cu and the
+  // free SMs (27.8 ms without them).
   int mask = 1;
-  if (a->diagonalize) mask |= 2;
+  if (a->diagonalize) mask |= 2 | kGramLowerLambda;   // the eigensolver reads the lower triangle
   if (a->construct) mask |= 4;
   if (a->construct && a->ipair) mask |= 8;
-  const bool beside = a->diagonalize && ctx->side2;
-  const bool split = beside && a->construct && ctx->side && ctx->gram_split;
+  const bool beside = a->diagonalize && ctx->side && ctx->side2;
+  const bool split = beside && a->construct && ctx->gram_split;
   const double* vp[2] = {a->v_pair, a->v_pair ? a->v_pair + n3 : nullptr};
   double2* outs[8];
   for (int iq = 0; iq < 2; ++iq)
     for (int m = 0; m < 4; ++m) outs[iq * 4 + m] = gm + ((size_t)iq * 4 + m) * sm;
   {
-    const int m1 = split ? (mask & 3) : mask;
+    const int m1 = split ? (mask & (3 | kGramLowerLambda)) : mask;
     const int masks[2] = {m1, m1};
     r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, st);
     if (r) return r;
@@ -1223,11 +1013,7 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
     if (split) cudaEventRecord(ctx->ev_fork2, ctx->side2);
     nst = ctx->side2;
   }
-  // Beside the single-precision Gram launch (one CTA per SM with all its
-  // shared memory, on 144 of the 148 SMs) each isospin takes one SM, which
-  // the launch leaves free; otherwise as many as its products can use.
-  const bool few = split && prec != HFB_F64 && ctx->use_tcgen05;
-  r = loewdin_launch(LoewdinArgs{nper, off, ld, gm, 4 * sm, Ur, a->sp_norm, ctx->dev_status}, work, !few, nst);
+  r = loewdin_launch(LoewdinArgs{nper, off, ld, gm, 4 * sm, Ur, a->sp_norm, ctx->dev_status}, work, !split, nst);
   if (r) return r;
   if (a->diagonalize) {
     // single-precision states carry rounding noise of 2^-24 relative in
@@ -1259,7 +1045,7 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
     cudaStreamWaitEvent(ctx->side, ctx->ev_fork2, 0);
     const int m2 = mask & 12;
     const int masks[2] = {m2, m2};
-    r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, ctx->side);
+    r = gram_launch(ctx, prec, 2, so, nq, masks, a->psi, a->hampsi, a->hmfpsi, vp, a->wxyz, outs, ld, ctx->side, 4);
     if (r) return r;
     cudaEventRecord(ctx->ev_join, ctx->side);
   }
@@ -1286,6 +1072,10 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
                     a->efluct},
       work, st);
   if (r) return r;
+  if (prec == HFB_F64 && ctx->f64_mma) {
+    const double2 *Us[2] = {U, U + sm}, *Ls[2] = {Lw, Lw + sm};
+    return rotate_f64_launch(ctx, 2, so, nq, a->psi, Us, Ls, ld, a->psi_out, a->lagrange, st);
+  }
   for (int iq = 0; iq < 2; ++iq) {
     r = rotate_launch(ctx, prec, so[iq], nq[iq], a->psi, U + (size_t)iq * sm, Lw + (size_t)iq * sm, ld, a->psi_out,
                       a->lagrange, st, pre[iq]);

@@ -15,6 +15,17 @@ __device__ __forceinline__ void gd_mma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// ---- contract_f64.cu: Gram and rotation on the FP64 tensor cores -----------
+// Mask bits 0-3 ask for S, lambda, H, G; with kGramLowerLambda matrix 1 is
+// written on and below its diagonal only; ``leave`` SMs stay free.
+constexpr int kGramLowerLambda = 16;
+int gram_f64_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
+                    const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz,
+                    double2* const* outs, int ldo, int leave, cudaStream_t st);
+// out1 = psi U, out2 = psi L for up to two blocks of states of one array
+int rotate_f64_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const void* psi, const double2* const* U,
+                      const double2* const* L, int ld, void* out1, void* out2, cudaStream_t st);
+
 // ---- diag_cluster.cu: matrix chains of the two isospins, one cluster each --
 struct RefineArgs {
   Pair2 nper;

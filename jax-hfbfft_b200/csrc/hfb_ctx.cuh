@@ -12,12 +12,14 @@ struct hfb_ctx_s {
   int periodic;
   int nstmax;
   int device;            // CUDA device current when the context was created
+  int sms;               // its multiprocessors
   int n2;                // Coulomb grid size (2n, or n when periodic)
   double* der1[3];       // dense spectral derivative matrices (grids.py:36-61)
   double* der2[3];
   double2* coul_q;       // Green's function in k space, n2^3 (coulomb.py:23-52)
   int* dev_status;       // latched device-side error code
-  int* counters;         // finished-blocks counter of the gradient step's maximum (behind dev_status; zero between launches)
+  int* counters;         // behind dev_status, zero between launches: [0] finished blocks of the gradient step's
+                         // maximum, [1] tickets of the FP64 Gram
   cudaStream_t side;     // secondary stream for independent work inside a call
   int use_tcgen05;       // single-precision contractions on the tensor cores (default 1;
                          // HFB_NO_TCGEN05=1 in the environment at creation selects CUDA cores)
