@@ -140,7 +140,7 @@ int hfb_poisson(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream)
  * (HFB_ERR_ARG otherwise).  The first call on each device looks up the
  * array's device address, so make that first call before any stream
  * capture.  All calls share the one buffer (it keeps the last call's
- * contents; each call rewrites all of it, padding zeros included): calls
+ * contents; each call writes every element it reads): calls
  * that overlap on the GPU -- concurrent streams, host threads -- race and
  * must be serialised by the caller. */
 int hfb_poisson_noalloc(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream);

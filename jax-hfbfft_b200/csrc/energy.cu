@@ -2,13 +2,9 @@
 // (output.py:187-226, 246) and the harmonic-oscillator initial states
 // (harmosc, static.py:580-738).  FP64, deterministic two-stage reductions.
 #include <math.h>
-#include "hfb_ctx.cuh"
+#include "fields.cuh"
 
 namespace hfb {
-
-int density_derivatives(hfb_ctx_s* c, const double* rho, const double* cur, const double* sd, const double* so,
-                        bool need_grad_curls, double** dv_out, cudaStream_t st);
-constexpr int kNDerivE = 11;   // layout of density_derivatives (skyrme.cu)
 
 enum { I_EHF0 = 0, I_CRHO0, I_CRHO1, I_EHF3, I_EHF2, I_CDRHO0, I_CDRHO1, I_CTAU0, I_CTAU1, I_EHF1, I_LSEVEN, I_CDJ0,
        I_CDJ1, I_LSODD, I_EHFC, I_ECORC, I_EHFT, I_NSUM };
@@ -22,7 +18,7 @@ energy_points_kernel(hfb_force f, int tcoul, size_t n3, const double* rho, const
 #pragma unroll
   for (int k = 0; k < I_NSUM; ++k) acc[k] = 0.0;
   const double* d0 = dv;
-  const double* d1 = dv + (size_t)kNDerivE * n3;
+  const double* d1 = dv + (size_t)kNDeriv * n3;
   const double sc = (f.ex != 0) ? -3.0 / 4.0 * f.slate : 0.0;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
     const double rn = rho[i], rp = rho[n3 + i];
@@ -80,18 +76,23 @@ energy_points_kernel(hfb_force f, int tcoul, size_t n3, const double* rho, const
 
 __global__ void energy_final_kernel(hfb_force f, int tcoul, double A, double wxyz, int n, int nblk, const double* part,
                                     const double* cur, const double* epair, double* out, int* status) {
+  // a warp per integral over the blocks' partials (a thread per integral was
+  // a serial chain of ``nblk`` loads: 26 us, 6 us here)
   __shared__ double s[I_NSUM];
-  if (threadIdx.x < I_NSUM) {
+  {
+    const int k = threadIdx.x / 32, lane = threadIdx.x % 32;
     double v = 0.0;
-    for (int b = 0; b < nblk; ++b) v += part[(size_t)b * I_NSUM + threadIdx.x];
-    s[threadIdx.x] = wxyz * v;
+    for (int b = lane; b < nblk; b += 32) v += part[(size_t)b * I_NSUM + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) s[k] = wxyz * v;
   }
-  __syncthreads();
   // energies.py:157-167 (diagnostic; indexes current[iq, comp, x, c, s] with
-  // y = c, z = s): the 2 x 3 x n x 3 terms spread over the warp
+  // y = c, z = s): the 2 x 3 x n x 3 terms spread over the block
+  __shared__ double r0[I_NSUM], r1[I_NSUM];
   const size_t n3 = (size_t)n * n * n;
   double cj0 = 0.0, cj1 = 0.0;
-  for (int e = threadIdx.x; e < 2 * 3 * n * 3; e += blockDim.x) {
+  for (int e = threadIdx.x; e < 2 * 3 * n * 3; e += 32 * I_NSUM) {
     const int c = e % 3, x = (e / 3) % n, comp = (e / (3 * n)) % 3, iq = e / (9 * n);
     const double* base = cur + ((size_t)iq * 3 + comp) * n3 + (size_t)x * n * n + (size_t)c * n;
     const double a0 = base[0], a1 = base[1];
@@ -103,7 +104,17 @@ __global__ void energy_final_kernel(hfb_force f, int tcoul, double A, double wxy
     cj0 += __shfl_xor_sync(0xffffffffu, cj0, o);
     cj1 += __shfl_xor_sync(0xffffffffu, cj1, o);
   }
+  if (threadIdx.x % 32 == 0) {
+    r0[threadIdx.x / 32] = cj0;
+    r1[threadIdx.x / 32] = cj1;
+  }
+  __syncthreads();
   if (threadIdx.x != 0) return;
+  cj0 = cj1 = 0.0;
+  for (int k = 0; k < I_NSUM; ++k) {
+    cj0 += r0[k];
+    cj1 += r1[k];
+  }
   const double ep = epair[0] + epair[1];
   const double ehf3 = s[I_EHF3];
   const double e3corr = -f.power * ehf3 / 2.0;
@@ -315,7 +326,7 @@ energy_grad_points_kernel(hfb_force f, size_t n3, const double* rho, const doubl
 #pragma unroll
   for (int k = 0; k < G_NSUM; ++k) acc[k] = 0.0;
   const double* d0 = dv;
-  const double* d1 = dv + (size_t)kNDerivE * n3;
+  const double* d1 = dv + (size_t)kNDeriv * n3;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3; i += (size_t)gridDim.x * blockDim.x) {
     const double rn = rho[i], rp = rho[n3 + i];
     const double rt = rn + rp, rq2 = rn * rn + rp * rp;
@@ -384,7 +395,7 @@ extern "C" int hfb_energies(hfb_ctx_t ctx, const hfb_force* f, int tcoul, double
   if (!part) return HFB_ERR_ALLOC;
   energy_points_kernel<<<kEnBlocks, 256, 0, st>>>(*f, tcoul, n3, rho, tau, sdens, wcoul, dv, part);
   HFB_CHECK_LAUNCH();
-  energy_final_kernel<<<1, 32, 0, st>>>(*f, tcoul, mass_number, ctx->wxyz, ctx->n, kEnBlocks, part, current, epair,
+  energy_final_kernel<<<1, 32 * I_NSUM, 0, st>>>(*f, tcoul, mass_number, ctx->wxyz, ctx->n, kEnBlocks, part, current, epair,
                                         out, ctx->dev_status);
   HFB_CHECK_LAUNCH();
   return HFB_OK;
