@@ -157,6 +157,14 @@ int hfb_add_density(hfb_ctx_t ctx, int prec, int nst, int nneut, const void* psi
                     const double* wstates, double mix, double* rho, double* chi, double* tau,
                     double* current, double* sdens, double* sodens, const double* h2m,
                     double* sp_kinetic, void* stream);
+/* Pair densities of two sets of states: sum_s w_s F(a_s, b_s) for rho, tau,
+ * current, sdens, sodens and sum_s wu_s chi(a_s, b_s), where F(a, b) is the
+ * symmetric bilinear form with F(psi, psi) the density term of psi (the
+ * potentials' cotangents in the VJP of hpsi; no counterpart in the
+ * reference).  w and wu are device double[nst]. */
+int hfb_pair_density(hfb_ctx_t ctx, int prec, int nst, int nneut, const void* a, const void* b,
+                     const double* w, const double* wu, double* rho, double* chi, double* tau,
+                     double* current, double* sdens, double* sodens, void* stream);
 /* sp_properties kinetic part alone (inout.py:64-150); h2m host array [2]. */
 int hfb_sp_kinetic(hfb_ctx_t ctx, int prec, int nst, int nneut, const void* psi,
                    const double* h2m, double* sp_kinetic, void* stream);

@@ -1,13 +1,29 @@
-// Occupation-weighted densities (add_density, densities.py:177-330) and the
-// single-particle kinetic energy of sp_properties (inout.py:64-150).
+// Occupation-weighted densities (add_density, densities.py:177-330), the
+// single-particle kinetic energy of sp_properties (inout.py:64-150) and the
+// pair densities of two sets of states.
 //
 // Every density term is local or bilinear in psi and ONE first derivative
-// d_d psi (cderv d00), so the work splits into three line kernels, one per
-// axis d.  A CTA owns a tile of lines along d and loops over a chunk of
-// states of one isospin: per state it FFTs each line, forms d_d psi, and
-// accumulates its fields in FP64 registers (lane-owned points, no atomics).
-// Per-chunk partial fields are summed in a fixed order by a combine kernel,
-// which also applies the density mixing of static.py:1820-1823.
+// d_d psi (cderv d00).  A work unit is one state on a tile of lines along one
+// axis d: the lines are transformed, d_d psi formed and the terms added to
+// FP64 accumulators in registers (no atomics).  P lanes own a line of one
+// spinor component and P neighbouring lanes the same line of the other one,
+// so a lane accumulates the terms that start from its own derivative and
+// takes the partner component's value by one shuffle; sums and differences
+// over the two components are taken once, when a tile is written.  The local
+// densities ride on axes x and y, so that no axis has more than five
+// accumulators per point.
+//
+// Units are numbered axis, isospin, tile, state; a CTA (128 threads) takes
+// an equal run of consecutive units whatever the state counts, and writes
+// one partial tile per (axis, isospin, tile) it meets.  A combine kernel adds
+// the partials in order and applies the density mixing of
+// static.py:1820-1823.  (With both components and up to nine accumulators per
+// point in a thread, one CTA per SM, equal chunks of unequal isospins in three
+// launches and bank conflicts in the transforms' exchange: 670 us for 90 + 60
+// single-precision states at 40^3, 2.32 ms for 236 double-precision ones at
+// 48^3; 480 us and 1.72 ms here.  Both components in a thread on this scheme:
+// 550 us, the registers leave half the warps.)  What bounds it is issue: the
+// transforms, and FP64 accumulation with its conversions.
 //
 // Kinetic energy: with the unnormalised FFT and Parseval,
 //   sum_k k_d^2 |psi_k|^2 / Ntot = sum_r |D_d psi|^2
@@ -18,290 +34,423 @@
 
 namespace hfb {
 
+namespace {
+
 template <class R, int N>
 struct DensGeo {
   static constexpr int P = (N >= 32) ? 8 : (N >= 16 ? 4 : 2);
   static constexpr int M = N / P;
   static constexpr int T = (M + P - 1) / P;
-  static constexpr int L = 256 / P;          // lines per CTA
-  static constexpr int THREADS = L * P;
-  static constexpr int NB = N + 4;
-  static constexpr int NTILE = (N * N + L - 1) / L;
+  static constexpr int THREADS = 128;
+  static constexpr int L = THREADS / (2 * P);   // lines per tile
+  static constexpr int NB = Pencil<R, N, P>::XB;
+  static constexpr int NTILE = N * N / L;
   static constexpr int WARPS = THREADS / 32;
+  static_assert(N * N % L == 0, "whole tiles");
 };
 
-// number of accumulated fields per axis kernel
-template <int AXIS> struct DensFields { static constexpr int value = AXIS == 2 ? 9 : 4; };
+// Fields of a partial tile.  Axis x: tau, current, J parts (two), rho, chi,
+// s_z; axis y: tau, current, J parts (two), s_x, s_y; axis z: tau, current,
+// J parts (two).
+constexpr int kDensFields = 7;
 
-template <class R, int N, int AXIS>
-__global__ void __launch_bounds__(DensGeo<R, N>::THREADS)
-density_axis_kernel(const cplx<R>* __restrict__ psi, int nst, int nneut, int nchunk, const double* __restrict__ wocc,
-                    const double* __restrict__ wguv, const double* __restrict__ pairwg,
-                    const double* __restrict__ wstates, double kscale, double nyq_fac, int want_fields, double* part,
-                    double* kin_part) {
+// How the units are cut up, and where a partial tile lies.
+struct DensCut {
+  int nq;                   // isospin blocks that have states
+  int iq[2], s0[2], cnt[2]; // isospin, first state, states of each
+  int ntile, nst;
+  long units, run;          // all units; units per CTA
+  int segs;                 // partial tiles a CTA can write at most
+};
+// first unit of (axis, block, tile), and its number among all tiles
+__host__ __device__ __forceinline__ long dens_first(const DensCut& c, int axis, int q, int tile) {
+  return (long)axis * c.ntile * c.nst + (q ? (long)c.ntile * c.cnt[0] : 0) + (long)tile * c.cnt[q];
+}
+__device__ __forceinline__ void dens_decode(const DensCut& c, long u, int& axis, int& q, int& tile, int& s) {
+  const long per = (long)c.ntile * c.nst;
+  axis = (int)(u / per);
+  long r = u - axis * per;
+  q = c.nq > 1 && r >= (long)c.ntile * c.cnt[0];
+  if (q) r -= (long)c.ntile * c.cnt[0];
+  tile = (int)(r / c.cnt[q]);
+  s = (int)(r - (long)tile * c.cnt[q]);
+}
+
+enum { DENS_KINETIC = 0, DENS_FIELDS = 1, DENS_PAIR = 2 };   // kinetic energies only; densities; pair densities
+
+struct DensArgs {
+  const void *psi, *psi2;   // psi2: the second set of a pair density
+  const double *wocc, *wguv, *pairwg, *wstates;
+  double ks[3], nf[3];
+  double* part;
+  double* kin;              // [state][axis][tile][warp], or null
+  DensCut cut;
+};
+
+// States sa..sb of one block on one tile of one axis.
+template <class R, int N, int AXIS, int KIND>
+__device__ __forceinline__ void dens_segment(const DensArgs& a, int tile, int sa, int sb, double* out,
+                                             cplx<R>* xb, const cplx<R>* tw, const R* sk) {
   using G = DensGeo<R, N>;
   using PC = Pencil<R, N, G::P>;
   using Z = cplx<R>;
   constexpr int P = G::P, M = G::M, T = G::T;
-  constexpr int NF = DensFields<AXIS>::value;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
-  __shared__ __align__(16) cplx<R> xball[G::L * G::NB];
-  __shared__ cplx<R> tw[N];
-  fill_twiddles<R>(tw, N);
-  __syncthreads();
-  const int tile = blockIdx.x;
-  const int iq = blockIdx.y / nchunk, chunk = blockIdx.y % nchunk;
-  const int q0 = iq == 0 ? 0 : nneut, q1 = iq == 0 ? nneut : nst;
-  const int cnt = q1 - q0;
-  const int sa = q0 + (int)(((long)cnt * chunk) / nchunk), sb = q0 + (int)(((long)cnt * (chunk + 1)) / nchunk);
-  const int lg = threadIdx.x / P, p = threadIdx.x % P;
-  const int line_raw = tile * G::L + lg;
-  const bool active = line_raw < N * N;
-  const int line = active ? line_raw : 0;
-  // line -> (u, v) transverse coordinates with the contiguous one fastest
-  const int u = line / N, v = line % N;
+  constexpr bool PAIR = KIND == DENS_PAIR, FIELDS = KIND != DENS_KINETIC;
+  constexpr int NA = !FIELDS ? 1 : AXIS == 0 ? 5 : 4;
+  const int lg = threadIdx.x / (2 * P), c = (threadIdx.x / P) & 1, p = threadIdx.x % P;
+  const int line = tile * G::L + lg, u = line / N, v = line % N;
+  // line -> transverse coordinates with the contiguous one fastest
   size_t base, stride;
   if (AXIS == 2) { base = (size_t)u * N2 + (size_t)v * N; stride = 1; }        // (x, y) fixed
   else if (AXIS == 1) { base = (size_t)u * N2 + v; stride = N; }               // (x, z) fixed
   else { base = (size_t)u * N + v; stride = N2; }                             // (y, z) fixed
-  Z* xb = xball + lg * G::NB;
-  double acc[NF][M];
+  base += c * N3 + p * stride;
+  double acc[NA][M];
 #pragma unroll
-  for (int f = 0; f < NF; ++f)
+  for (int f = 0; f < NA; ++f)
 #pragma unroll
     for (int m = 0; m < M; ++m) acc[f][m] = 0.0;
-
+  const Z* src = (const Z*)a.psi + base + (size_t)sa * 2 * N3;
+  const Z* src2 = (const Z*)a.psi2 + base + (size_t)sa * 2 * N3;
   // the line values of the next state are loaded while this one is
-  // transformed and accumulated
-  Z an[M], bn[M];
-  if (sa < sb) {
-    const Z* ps = psi + (size_t)sa * 2 * N3 + base;
+  // transformed and accumulated (not for pairs: the registers are needed)
+  Z xn[M];
+  if (!PAIR) {
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      an[m] = ps[(size_t)(p + P * m) * stride];
-      bn[m] = ps[N3 + (size_t)(p + P * m) * stride];
-    }
+    for (int m = 0; m < M; ++m) xn[m] = src[m * (P * stride)];
   }
-  for (int s = sa; s < sb; ++s) {
-    const double w = want_fields ? wocc[s] * wstates[s] : 0.0;
-    const double wu = want_fields ? wguv[s] * pairwg[s] * wstates[s] : 0.0;
-    Z a[M], b[M], da[M], db[M];
+  // wave numbers of this lane's frequencies
+  const R* skl = sk + AXIS * N + p;
+  // D_d of a line (cderv d00: k = 0 and Nyquist zeroed)
+  auto diff = [&](const Z (&x)[M], Z (&d)[M], double& nyq) {
+    Z vv[M];
+    Z f[T][P];
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      a[m] = an[m];
-      b[m] = bn[m];
+    for (int m = 0; m < M; ++m) vv[m] = x[m];
+    PC::forward(vv, f, xb, tw, p, 0xffffffffu);
+    nyq = p == 0 ? (double)f[0][P / 2].x * f[0][P / 2].x + (double)f[0][P / 2].y * f[0][P / 2].y : 0.0;
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+      for (int k1 = 0; k1 < P; ++k1) {
+        const R sc = PC::valid(p, t) ? skl[P * t + M * k1] : R(0);
+        const Z z = f[t][k1];
+        f[t][k1] = mk<R>(-sc * z.y, sc * z.x);
+      }
+    PC::inverse(f, d, xb, tw, p, 0xffffffffu);
+  };
+  auto partner = [&](Z x) {
+    Z y;
+    y.x = __shfl_xor_sync(0xffffffffu, x.x, P);
+    y.y = __shfl_xor_sync(0xffffffffu, x.y, P);
+    return y;
+  };
+  for (int s = sa; s < sb; ++s) {
+    double w = 0.0, wu = 0.0;
+    if (FIELDS) {
+      const double ws = PAIR ? 1.0 : a.wstates[s];
+      w = a.wocc[s] * ws;
+      if (AXIS == 0) wu = PAIR ? a.wguv[s] : a.wguv[s] * a.pairwg[s] * ws;
     }
-    if (s + 1 < sb) {
-      const Z* ps = psi + (size_t)(s + 1) * 2 * N3 + base;
+    Z x[M], d[M];
+    double nyq;
+    if (PAIR) {
+      Z y[M], e[M];
 #pragma unroll
       for (int m = 0; m < M; ++m) {
-        an[m] = ps[(size_t)(p + P * m) * stride];
-        bn[m] = ps[N3 + (size_t)(p + P * m) * stride];
+        x[m] = src[m * (P * stride)];
+        y[m] = src2[m * (P * stride)];
       }
-    }
-    double knyq = 0.0;
-    // D_d psi for both components (cderv d00: k = 0 and Nyquist zeroed)
+      src += 2 * N3;
+      src2 += 2 * N3;
+      diff(x, d, nyq);
+      diff(y, e, nyq);
+      const double h = 0.5 * w;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      Z vv[M];
-      Z f[T][P];
+      for (int m = 0; m < M; ++m) {
+        const Z px = partner(x[m]), py = partner(y[m]);
+        const double xr = x[m].x, xi = x[m].y, yr = y[m].x, yi = y[m].y;
+        const double dr = d[m].x, di = d[m].y, er = e[m].x, ei = e[m].y;
+        const double pr = px.x, pi = px.y, qr = py.x, qi = py.y;
+        acc[0][m] += w * (dr * er + di * ei);
+        acc[1][m] += h * (di * yr - dr * yi + ei * xr - er * xi);
+        if (AXIS != 1) acc[2][m] += h * (dr * qr + di * qi + er * pr + ei * pi);
+        if (AXIS != 0) acc[AXIS == 2 ? 3 : 2][m] += h * (di * qr - dr * qi + ei * pr - er * pi);
+        if (AXIS == 0) {
+          const double xy = xr * yr + xi * yi;
+          acc[3][m] += w * xy;
+          acc[4][m] += wu * xy;
+        }
+        if (AXIS == 1)
+          acc[3][m] += h * (c == 0 ? xr * qr + xi * qi + yr * pr + yi * pi : pr * yi - pi * yr + qr * xi - qi * xr);
+      }
+    } else {
 #pragma unroll
-      for (int m = 0; m < M; ++m) vv[m] = c == 0 ? a[m] : b[m];
-      PC::forward(vv, f, xb, tw, p, 0xffffffffu);
-      if (p == 0) knyq += (double)f[0][P / 2].x * f[0][P / 2].x + (double)f[0][P / 2].y * f[0][P / 2].y;
+      for (int m = 0; m < M; ++m) x[m] = xn[m];
+      src += 2 * N3;
+      if (s + 1 < sb) {
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
+        for (int m = 0; m < M; ++m) xn[m] = src[m * (P * stride)];
+      }
+      diff(x, d, nyq);
+      double kin = 0.0;
 #pragma unroll
-        for (int k1 = 0; k1 < P; ++k1) {
-          int k = PC::freq(p, t, k1);
-          R sc = (k == 0 || 2 * k == N) ? R(0) : (R)(signed_k(k, N) * kscale);
-          Z z = f[t][k1];
-          f[t][k1] = mk<R>(-sc * z.y, sc * z.x);
+      for (int m = 0; m < M; ++m) {
+        const double xr = x[m].x, xi = x[m].y, dr = d[m].x, di = d[m].y;
+        const double dd = dr * dr + di * di;
+        kin += dd;
+        if (FIELDS) {
+          const Z px = partner(x[m]);
+          const double pr = px.x, pi = px.y, wr = w * dr, wi = w * di;
+          acc[0][m] += w * dd;
+          acc[1][m] += wi * xr;                                  // Im(d conj(x))
+          acc[1][m] -= wr * xi;
+          if (AXIS != 1) {
+            acc[2][m] += wr * pr;                                // Re(d conj(partner))
+            acc[2][m] += wi * pi;
+          }
+          if (AXIS != 0) {
+            acc[AXIS == 2 ? 3 : 2][m] += wi * pr;                // Im(d conj(partner))
+            acc[AXIS == 2 ? 3 : 2][m] -= wr * pi;
+          }
+          if (AXIS == 0) {
+            const double xx = xr * xr + xi * xi;
+            acc[3][m] += w * xx;
+            acc[4][m] += wu * xx;
+          }
+          // Re(conj(up) down) in the lanes of the up component, Im in the others
+          if (AXIS == 1) acc[3][m] += w * (c == 0 ? xr * pr + xi * pi : pr * xi - pi * xr);
         }
       }
-      if (c == 0) PC::inverse(f, da, xb, tw, p, 0xffffffffu);
-      else PC::inverse(f, db, xb, tw, p, 0xffffffffu);
-    }
-    double kin = 0.0;
+      if (a.kin) {
+        // per-warp partials, summed in a fixed order by kinetic_reduce_kernel
+        kin += a.nf[AXIS] * nyq;
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double ar = a[m].x, ai = a[m].y, br = b[m].x, bi = b[m].y;
-      const double d0r = da[m].x, d0i = da[m].y, d1r = db[m].x, d1i = db[m].y;
-      const double dd = d0r * d0r + d0i * d0i + d1r * d1r + d1i * d1i;
-      kin += dd;
-      if (want_fields) {
-        // Im(d0 conj(a) + d1 conj(b)), Im(d0 conj(a) - d1 conj(b)), ...
-        const double im_d0a = d0i * ar - d0r * ai, im_d1b = d1i * br - d1r * bi;
-        const double im_d1a = d1i * ar - d1r * ai, im_d0b = d0i * br - d0r * bi;
-        const double re_d1a = d1r * ar + d1i * ai, re_d0b = d0r * br + d0i * bi;
-        if (AXIS == 2) {
-          const double aa = ar * ar + ai * ai, bb = br * br + bi * bi;
-          acc[0][m] += w * (aa + bb);
-          acc[1][m] += 0.5 * wu * (aa + bb);
-          acc[2][m] += 2.0 * w * (ar * br + ai * bi);     // Re(conj(a) b)
-          acc[3][m] += 2.0 * w * (ar * bi - ai * br);     // Im(conj(a) b)
-          acc[4][m] += w * (aa - bb);
-          acc[5][m] += w * dd;
-          acc[6][m] += w * (im_d0a + im_d1b);
-          acc[7][m] += w * (re_d1a - re_d0b);             // J_x, z part (densities.py:308-311)
-          acc[8][m] += w * (im_d1a + im_d0b);             // J_y, z part (312-315)
-        } else if (AXIS == 1) {
-          acc[0][m] += w * dd;
-          acc[1][m] += w * (im_d0a + im_d1b);
-          acc[2][m] += w * (im_d0a - im_d1b);             // J_x, y part (289-292)
-          acc[3][m] += -w * (im_d1a + im_d0b);            // J_z, y part (293-296)
-        } else {
-          // Re(a conj(d1) - b conj(d0)) = Re(d1 conj(a)) - Re(d0 conj(b))
-          acc[0][m] += w * dd;
-          acc[1][m] += w * (im_d0a + im_d1b);
-          acc[2][m] += -w * (im_d0a - im_d1b);            // J_y, x part (270-273)
-          acc[3][m] += -w * (re_d1a - re_d0b);            // J_z, x part (274-277)
-        }
+        for (int o = 16; o > 0; o >>= 1) kin += __shfl_xor_sync(0xffffffffu, kin, o);
+        if ((threadIdx.x & 31) == 0)
+          a.kin[(((size_t)s * 3 + AXIS) * G::NTILE + tile) * G::WARPS + threadIdx.x / 32] = kin;
       }
-    }
-    kin += nyq_fac * knyq;
-    if (!active) kin = 0.0;
-    if (kin_part) {
-      // per-warp partials, summed in a fixed order by kinetic_reduce_kernel
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) kin += __shfl_xor_sync(0xffffffffu, kin, o);
-      if ((threadIdx.x & 31) == 0)
-        kin_part[((size_t)s * G::NTILE + tile) * G::WARPS + threadIdx.x / 32] = kin;
     }
   }
-  if (want_fields && active) {
-    double* dst = part + (size_t)blockIdx.y * NF * N3;
+  if (!FIELDS) return;
+  // sums over the components; the two lanes write alternate points
 #pragma unroll
-    for (int f = 0; f < NF; ++f)
+  for (int m = 0; m < M && FIELDS; ++m) {
+    double up[NA], dn[NA];
 #pragma unroll
-      for (int m = 0; m < M; ++m) dst[(size_t)f * N3 + base + (size_t)(p + P * m) * stride] = acc[f][m];
+    for (int f = 0; f < NA; ++f) {
+      const double o = __shfl_xor_sync(0xffffffffu, acc[f][m], P);
+      up[f] = c == 0 ? acc[f][m] : o;
+      dn[f] = c == 0 ? o : acc[f][m];
+    }
+    if ((m & 1) != c) continue;
+    const int j = p + P * m;
+    double* w = out + (AXIS == 2 ? lg * N + j : j * G::L + lg);
+    constexpr int FS = G::L * N;
+    w[0] = up[0] + dn[0];
+    w[FS] = up[1] + dn[1];
+    if (AXIS == 0) {
+      w[2 * FS] = -(up[1] - dn[1]);            // J_y, x part (densities.py:270-273)
+      w[3 * FS] = -(dn[2] - up[2]);            // J_z, x part (274-277)
+      w[4 * FS] = up[3] + dn[3];
+      w[5 * FS] = 0.5 * (up[4] + dn[4]);
+      w[6 * FS] = up[3] - dn[3];
+    } else if (AXIS == 1) {
+      w[2 * FS] = up[1] - dn[1];               // J_x, y part (289-292)
+      w[3 * FS] = -(dn[2] + up[2]);            // J_z, y part (293-296)
+      w[4 * FS] = 2.0 * up[3];
+      w[5 * FS] = 2.0 * dn[3];
+    } else {
+      w[2 * FS] = dn[2] - up[2];               // J_x, z part (308-311)
+      w[3 * FS] = dn[3] + up[3];               // J_y, z part (312-315)
+    }
   }
 }
 
-// Sum the per-chunk partials of the three axis kernels into the reference's
-// density arrays; rho, tau, chi are mixed as mix*new + (1-mix)*old.
-__global__ void density_combine_kernel(size_t n3, int nchunk, const double* pz, const double* py, const double* px,
-                                       double mix, double* rho, double* chi, double* tau, double* cur, double* sd,
-                                       double* so) {
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+template <class R, int N, int KIND>
+__global__ void __launch_bounds__(DensGeo<R, N>::THREADS, sizeof(R) == 8 || KIND == DENS_PAIR ? 2 : N > 40 ? 3 : 4)
+density_kernel(const __grid_constant__ DensArgs a) {
+  using G = DensGeo<R, N>;
+  __shared__ __align__(16) cplx<R> xball[G::THREADS / G::P * G::NB];
+  __shared__ cplx<R> tw[N];
+  __shared__ R sk[3 * N];   // k of each axis, 0 at k = 0 and at the Nyquist mode
+  fill_twiddles<R>(tw, N);
+  for (int e = threadIdx.x; e < 3 * N; e += G::THREADS) {
+    const int k = e % N;
+    sk[e] = (k == 0 || 2 * k == N) ? R(0) : (R)(signed_k(k, N) * a.ks[e / N]);
+  }
+  __syncthreads();
+  cplx<R>* xb = xball + (threadIdx.x / G::P) * G::NB;
+  const DensCut& cut = a.cut;
+  long u = (long)blockIdx.x * cut.run;
+  const long end = min(cut.units, u + cut.run);
+  for (int seg = 0; u < end; ++seg) {
+    int axis, q, tile, s;
+    dens_decode(cut, u, axis, q, tile, s);
+    const int n = (int)min((long)(cut.cnt[q] - s), end - u);
+    const int sa = cut.s0[q] + s;
+    double* out = a.part + ((size_t)blockIdx.x * cut.segs + seg) * kDensFields * G::L * N;
+    if (axis == 0) dens_segment<R, N, 0, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
+    else if (axis == 1) dens_segment<R, N, 1, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
+    else dens_segment<R, N, 2, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
+    u += n;
+  }
+}
+
+// Sum the partial tiles of the three axes into the reference's density
+// arrays; rho, tau, chi are mixed as mix*new + (1-mix)*old.
+template <int N, int L>
+__global__ void __launch_bounds__(128)
+density_combine_kernel(DensCut cut, const double* __restrict__ part, double mix, double* rho, double* chi, double* tau,
+                       double* cur, double* sd, double* so) {
+  constexpr size_t N2 = (size_t)N * N, n3 = N2 * N;
+  constexpr int FS = L * N;
+  const size_t i = blockIdx.x * (size_t)128 + threadIdx.x;
   const int iq = blockIdx.y;
   if (i >= n3) return;
-  double f9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  double fy[4] = {0, 0, 0, 0}, fx[4] = {0, 0, 0, 0};
-  for (int c = 0; c < nchunk; ++c) {
-    const size_t b = (size_t)(iq * nchunk + c);
-    for (int f = 0; f < 9; ++f) f9[f] += pz[(b * 9 + f) * n3 + i];
-    for (int f = 0; f < 4; ++f) {
-      fy[f] += py[(b * 4 + f) * n3 + i];
-      fx[f] += px[(b * 4 + f) * n3 + i];
+  const int x = (int)(i / N2), y = (int)((i / N) % N), z = (int)(i % N);
+  double f[3][kDensFields];
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax)
+#pragma unroll
+    for (int k = 0; k < kDensFields; ++k) f[ax][k] = 0.0;
+  for (int q = 0; q < cut.nq; ++q) {
+    if (cut.iq[q] != iq) continue;
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      const int line = ax == 0 ? y * N + z : ax == 1 ? x * N + z : x * N + y;
+      const int j = ax == 0 ? x : ax == 1 ? y : z;
+      const int tile = line / L, l = line % L;
+      const int off = ax == 2 ? l * N + j : j * L + l;
+      const long u0 = dens_first(cut, ax, q, tile), u1 = u0 + cut.cnt[q];
+      const long id = ((long)ax * cut.nq + q) * cut.ntile + tile;   // number of the tile
+      for (long k = u0 / cut.run; k <= (u1 - 1) / cut.run; ++k) {
+        int a0, q0, t0, s0;
+        dens_decode(cut, k * cut.run, a0, q0, t0, s0);               // where CTA k starts
+        const long seg = id - (((long)a0 * cut.nq + q0) * cut.ntile + t0);
+        const double* p = part + ((size_t)k * cut.segs + seg) * kDensFields * FS + off;
+        constexpr int NF[3] = {7, 6, 4};
+#pragma unroll
+        for (int g = 0; g < NF[ax]; ++g) f[ax][g] += p[g * FS];
+      }
     }
   }
-  const double tnew = f9[5] + fy[0] + fx[0];
+  const double tnew = f[2][0] + f[1][0] + f[0][0];
   const size_t o = (size_t)iq * n3 + i;
   if (mix < 1.0) {
-    rho[o] = mix * f9[0] + (1.0 - mix) * rho[o];
-    chi[o] = mix * f9[1] + (1.0 - mix) * chi[o];
+    rho[o] = mix * f[0][4] + (1.0 - mix) * rho[o];
+    chi[o] = mix * f[0][5] + (1.0 - mix) * chi[o];
     tau[o] = mix * tnew + (1.0 - mix) * tau[o];
   } else {
-    rho[o] = f9[0];
-    chi[o] = f9[1];
+    rho[o] = f[0][4];
+    chi[o] = f[0][5];
     tau[o] = tnew;
   }
   const size_t v = (size_t)iq * 3 * n3 + i;
-  sd[v] = f9[2];
-  sd[v + n3] = f9[3];
-  sd[v + 2 * n3] = f9[4];
-  cur[v] = fx[1];
-  cur[v + n3] = fy[1];
-  cur[v + 2 * n3] = f9[6];
-  so[v] = fy[2] + f9[7];
-  so[v + n3] = fx[2] + f9[8];
-  so[v + 2 * n3] = fx[3] + fy[3];
+  sd[v] = f[1][4];
+  sd[v + n3] = f[1][5];
+  sd[v + 2 * n3] = f[0][6];
+  cur[v] = f[0][1];
+  cur[v + n3] = f[1][1];
+  cur[v + 2 * n3] = f[2][1];
+  so[v] = f[1][2] + f[2][2];
+  so[v + n3] = f[0][2] + f[2][3];
+  so[v + 2 * n3] = f[0][3] + f[1][3];
 }
 
-// sp_kinetic[s] = wxyz h2m_q sum over axes, tiles and warps (``np`` partials
-// per state and axis); one warp per state, lanes over strided partials, then
-// a fixed shuffle tree.
-__global__ void kinetic_reduce_kernel(int nst, int nneut, int np, const double* kz, const double* ky,
-                                      const double* kx, double wxyz, double h2m_n, double h2m_p, double* out) {
-  const int s = blockIdx.x, lane = threadIdx.x;
-  if (s >= nst) return;
+// sp_kinetic[s] = wxyz h2m_q times the ``np`` partials of the state, in a
+// fixed order; one block per state.
+__global__ void __launch_bounds__(128) kinetic_reduce_kernel(int nneut, int np, const double* __restrict__ kin,
+                                                             double wxyz, double h2m_n, double h2m_p, double* out) {
+  __shared__ double red[4];
+  const int s = blockIdx.x;
   double t = 0;
-  for (int j = lane; j < np; j += 32)
-    t += kx[(size_t)s * np + j] + ky[(size_t)s * np + j] + kz[(size_t)s * np + j];
+  for (int j = threadIdx.x; j < np; j += 128) t += kin[(size_t)s * np + j];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0) out[s] = wxyz * (s >= nneut ? h2m_p : h2m_n) * t;
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) out[s] = wxyz * (s >= nneut ? h2m_p : h2m_n) * (red[0] + red[1] + red[2] + red[3]);
 }
 
-template <class R, int N>
-int density_launch_t(hfb_ctx_s* c, int nst, int nneut, const void* psi, const double* wocc, const double* wguv,
-                     const double* pairwg, const double* wstates, double mix, double* rho, double* chi, double* tau,
-                     double* cur, double* sd, double* so, const double* h2m, double* sp_kinetic, cudaStream_t st) {
+struct DensOut {
+  double mix;
+  double *rho, *chi, *tau, *cur, *sd, *so;   // rho null: kinetic energies only
+  const double* h2m;
+  double* sp_kinetic;
+};
+
+template <class R, int N, int KIND>
+int density_launch_t(hfb_ctx_s* c, DensArgs a, int nst, int nneut, const DensOut& o, cudaStream_t st) {
   using G = DensGeo<R, N>;
-  using Z = cplx<R>;
-  constexpr size_t N3 = (size_t)N * N * N;
-  const bool fields = rho != nullptr;
-  const int nq = 2;
-  int nchunk = (2 * 148 + 2 * G::NTILE - 1) / (2 * G::NTILE);
-  if (nchunk < 1) nchunk = 1;
-  if (nchunk > 8) nchunk = 8;
-  const int nb = nq * nchunk;
-  double* part = nullptr;
-  if (fields) {
-    part = (double*)scratch(c, hfb_ctx_s::S_DENS, sizeof(double) * (size_t)nb * 17 * N3);
-    if (!part) return HFB_ERR_ALLOC;
+  // CTAs that are resident together
+  static const int per_sm = [] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, density_kernel<R, N, KIND>, G::THREADS, 0) != cudaSuccess)
+      cudaGetLastError();
+    return n > 0 ? n : 1;
+  }();
+  DensCut cut{};
+  nneut = nneut < 0 ? 0 : nneut > nst ? nst : nneut;
+  const int cnt[2] = {nneut, nst - nneut};
+  for (int iq = 0; iq < 2; ++iq)
+    if (cnt[iq] > 0) {
+      cut.iq[cut.nq] = iq;
+      cut.s0[cut.nq] = iq ? nneut : 0;
+      cut.cnt[cut.nq++] = cnt[iq];
+    }
+  cut.ntile = G::NTILE;
+  cut.nst = nst;
+  cut.units = 3L * G::NTILE * nst;
+  // one run per resident CTA; at least two units, below which a CTA's start
+  // and its partial tiles cost more than the balance gives
+  const long places = (long)per_sm * c->sms;
+  cut.run = (cut.units + places - 1) / places;
+  if (cut.run < 2) cut.run = 2;
+  const int least = cut.nq > 1 && cut.cnt[1] < cut.cnt[0] ? cut.cnt[1] : cut.cnt[0];
+  cut.segs = (int)((cut.run + least - 2) / least + 1);
+  const long ctas = (cut.units + cut.run - 1) / cut.run;
+  a.cut = cut;
+  a.part = nullptr;
+  if (KIND != DENS_KINETIC) {
+    a.part = (double*)scratch(c, hfb_ctx_s::S_DENS, sizeof(double) * (size_t)ctas * cut.segs * kDensFields * G::L * N);
+    if (!a.part) return HFB_ERR_ALLOC;
   }
-  double* kin = nullptr;
-  if (sp_kinetic) {
-    kin = (double*)scratch(c, hfb_ctx_s::S_RED, sizeof(double) * (size_t)3 * nst * G::NTILE * G::WARPS);
-    if (!kin) return HFB_ERR_ALLOC;
+  a.kin = nullptr;
+  if (o.sp_kinetic) {
+    a.kin = (double*)scratch(c, hfb_ctx_s::S_RED, sizeof(double) * (size_t)3 * nst * G::NTILE * G::WARPS);
+    if (!a.kin) return HFB_ERR_ALLOC;
   }
-  double* pz = part;
-  double* py = part ? part + (size_t)nb * 9 * N3 : nullptr;
-  double* px = part ? py + (size_t)nb * 4 * N3 : nullptr;
-  double* kz = kin;
-  double* ky = kin ? kin + (size_t)nst * G::NTILE * G::WARPS : nullptr;
-  double* kx = kin ? kin + (size_t)2 * nst * G::NTILE * G::WARPS : nullptr;
-  dim3 grid(G::NTILE, nb);
-  const double ks[3] = {2.0 * kPi / (c->d[0] * N) / N, 2.0 * kPi / (c->d[1] * N) / N, 2.0 * kPi / (c->d[2] * N) / N};
-  double nf[3];
-  for (int a = 0; a < 3; ++a) nf[a] = (kPi / c->d[a]) * (kPi / c->d[a]) / N;
-  density_axis_kernel<R, N, 2><<<grid, G::THREADS, 0, st>>>((const Z*)psi, nst, nneut, nchunk, wocc, wguv, pairwg,
-                                                            wstates, ks[2], nf[2], fields, pz, kz);
+  for (int ax = 0; ax < 3; ++ax) {
+    a.ks[ax] = 2.0 * kPi / (c->d[ax] * N) / N;
+    a.nf[ax] = (kPi / c->d[ax]) * (kPi / c->d[ax]) / N;
+  }
+  density_kernel<R, N, KIND><<<(unsigned)ctas, G::THREADS, 0, st>>>(a);
   HFB_CHECK_LAUNCH();
-  density_axis_kernel<R, N, 1><<<grid, G::THREADS, 0, st>>>((const Z*)psi, nst, nneut, nchunk, wocc, wguv, pairwg,
-                                                            wstates, ks[1], nf[1], fields, py, ky);
-  HFB_CHECK_LAUNCH();
-  density_axis_kernel<R, N, 0><<<grid, G::THREADS, 0, st>>>((const Z*)psi, nst, nneut, nchunk, wocc, wguv, pairwg,
-                                                            wstates, ks[0], nf[0], fields, px, kx);
-  HFB_CHECK_LAUNCH();
-  if (fields) {
-    dim3 g2((unsigned)((N3 + 255) / 256), 2);
-    density_combine_kernel<<<g2, 256, 0, st>>>(N3, nchunk, pz, py, px, mix, rho, chi, tau, cur, sd, so);
+  if (KIND != DENS_KINETIC) {
+    const dim3 g2((unsigned)(((size_t)N * N * N + 127) / 128), 2);
+    density_combine_kernel<N, G::L><<<g2, 128, 0, st>>>(cut, a.part, o.mix, o.rho, o.chi, o.tau, o.cur, o.sd, o.so);
     HFB_CHECK_LAUNCH();
   }
-  if (sp_kinetic) {
-    kinetic_reduce_kernel<<<nst, 32, 0, st>>>(nst, nneut, G::NTILE * G::WARPS, kz, ky, kx, c->wxyz, h2m[0], h2m[1],
-                                              sp_kinetic);
+  if (o.sp_kinetic) {
+    kinetic_reduce_kernel<<<nst, 128, 0, st>>>(nneut, 3 * G::NTILE * G::WARPS, a.kin, c->wxyz, o.h2m[0], o.h2m[1],
+                                               o.sp_kinetic);
     HFB_CHECK_LAUNCH();
   }
   return HFB_OK;
 }
 
-int density_launch(hfb_ctx_s* c, int prec, int nst, int nneut, const void* psi, const double* wocc,
-                   const double* wguv, const double* pairwg, const double* wstates, double mix, double* rho,
-                   double* chi, double* tau, double* cur, double* sd, double* so, const double* h2m,
-                   double* sp_kinetic, cudaStream_t st) {
+template <int KIND>
+int density_launch(hfb_ctx_s* c, int prec, const DensArgs& a, int nst, int nneut, const DensOut& o, cudaStream_t st) {
   return dispatch_n(c->n, [&](auto nn) -> int {
     constexpr int N = decltype(nn)::value;
-    if (prec == HFB_F64)
-      return density_launch_t<double, N>(c, nst, nneut, psi, wocc, wguv, pairwg, wstates, mix, rho, chi, tau, cur, sd,
-                                         so, h2m, sp_kinetic, st);
-    return density_launch_t<float, N>(c, nst, nneut, psi, wocc, wguv, pairwg, wstates, mix, rho, chi, tau, cur, sd, so,
-                                      h2m, sp_kinetic, st);
+    if (prec == HFB_F64) return density_launch_t<double, N, KIND>(c, a, nst, nneut, o, st);
+    return density_launch_t<float, N, KIND>(c, a, nst, nneut, o, st);
   });
 }
+
+}  // namespace
 
 }  // namespace hfb
 
@@ -315,14 +464,34 @@ extern "C" int hfb_add_density(hfb_ctx_t ctx, int prec, int nst, int nneut, cons
     return HFB_ERR_ARG;
   if (sp_kinetic && !h2m) return HFB_ERR_ARG;
   if (nst <= 0) return HFB_ERR_ARG;
-  return density_launch(ctx, prec, nst, nneut, psi, wocc, wguv, pairwg, wstates, mix, rho, chi, tau, current, sdens,
-                        sodens, h2m, sp_kinetic, as_stream(stream));
+  DensArgs a{};
+  a.psi = psi;
+  a.wocc = wocc; a.wguv = wguv; a.pairwg = pairwg; a.wstates = wstates;
+  return density_launch<DENS_FIELDS>(ctx, prec, a, nst, nneut,
+                               DensOut{mix, rho, chi, tau, current, sdens, sodens, h2m, sp_kinetic}, as_stream(stream));
 }
 
 extern "C" int hfb_sp_kinetic(hfb_ctx_t ctx, int prec, int nst, int nneut, const void* psi, const double* h2m,
                               double* sp_kinetic, void* stream) {
   if (!ctx || !psi || !h2m || !sp_kinetic || nst <= 0) return HFB_ERR_ARG;
   // weights are not read when no fields are accumulated
-  return density_launch(ctx, prec, nst, nneut, psi, nullptr, nullptr, nullptr, nullptr, 1.0, nullptr, nullptr, nullptr,
-                        nullptr, nullptr, nullptr, h2m, sp_kinetic, as_stream(stream));
+  DensArgs a{};
+  a.psi = psi;
+  DensOut o{};
+  o.h2m = h2m;
+  o.sp_kinetic = sp_kinetic;
+  return density_launch<DENS_KINETIC>(ctx, prec, a, nst, nneut, o, as_stream(stream));
+}
+
+extern "C" int hfb_pair_density(hfb_ctx_t ctx, int prec, int nst, int nneut, const void* a, const void* b,
+                                const double* w, const double* wu, double* rho, double* chi, double* tau,
+                                double* current, double* sdens, double* sodens, void* stream) {
+  if (!ctx || !a || !b || !w || !wu || !rho || !chi || !tau || !current || !sdens || !sodens || nst <= 0)
+    return HFB_ERR_ARG;
+  DensArgs d{};
+  d.psi = a;
+  d.psi2 = b;
+  d.wocc = w; d.wguv = wu;
+  return density_launch<DENS_PAIR>(ctx, prec, d, nst, nneut,
+                              DensOut{1.0, rho, chi, tau, current, sdens, sodens, nullptr, nullptr}, as_stream(stream));
 }

@@ -20,7 +20,7 @@ struct PlaneGeo {
   static constexpr int M = N / P;
   static constexpr int T = (M + P - 1) / P;
   static constexpr int LD = N + 4;
-  static constexpr int NB = N + 4;
+  static constexpr int NB = Pencil<R, N, P>::XB;
   static constexpr int THREADS = ((N * P + 31) / 32) * 32;
   static constexpr int LINES = THREADS / P;
   static constexpr size_t SMEM = sizeof(cplx<R>) * (size_t)(2 * N * LD + LINES * NB + N);

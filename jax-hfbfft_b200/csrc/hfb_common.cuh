@@ -196,6 +196,13 @@ template <class R, int N_, int P_> struct Pencil {
   static constexpr int T = (M + P - 1) / P;
   static_assert(N % P == 0 && 32 % P == 0, "pencil split");
   using Z = cplx<R>;
+  // The exchange buffer is [M][P] with rows of P + 1 (a lane reads its own
+  // row: rows of P put the lanes of a line on two to four banks, 4.6-way
+  // conflicts), and XB elements per line, so that the lines of a warp cover
+  // every bank equally in both directions.
+  static constexpr int XS = P + 1;
+  static constexpr int XB_ODD = P == 8 ? 8 : P == 4 ? 4 : 2;   // XB mod 16
+  static constexpr int XB = M * XS + (16 + XB_ODD - M * XS % 16) % 16;
 
   // Index of frequency slot (t, k1) held by lane q.
   __device__ __forceinline__ static int freq(int q, int t, int k1) { return q + P * t + M * k1; }
@@ -212,14 +219,14 @@ template <class R, int N_, int P_> struct Pencil {
   __device__ __forceinline__ static void forward(Z (&v)[M], Z (&f)[T][P], Z* xb, const Z* tw, int p, unsigned mask) {
     DFT<M, -1, Z>::run(v);
 #pragma unroll
-    for (int k2 = 0; k2 < M; ++k2) xb[k2 * P + p] = (k2 == 0 || p == 0) ? v[k2] : tw_mul<-1>(v[k2], tw, p * k2);
+    for (int k2 = 0; k2 < M; ++k2) xb[k2 * XS + p] = (k2 == 0 || p == 0) ? v[k2] : tw_mul<-1>(v[k2], tw, p * k2);
     __syncwarp(mask);
 #pragma unroll
     for (int t = 0; t < T; ++t) {
       int k2 = p + P * t;
       if (T * P == M || k2 < M) {
 #pragma unroll
-        for (int pp = 0; pp < P; ++pp) f[t][pp] = xb[k2 * P + pp];
+        for (int pp = 0; pp < P; ++pp) f[t][pp] = xb[k2 * XS + pp];
         DFT<P, -1, Z>::run(f[t]);
       }
     }
@@ -233,12 +240,12 @@ template <class R, int N_, int P_> struct Pencil {
       if (T * P == M || k2 < M) {
         DFT<P, +1, Z>::run(f[t]);
 #pragma unroll
-        for (int pp = 0; pp < P; ++pp) xb[k2 * P + pp] = (k2 == 0 || pp == 0) ? f[t][pp] : tw_mul<+1>(f[t][pp], tw, pp * k2);
+        for (int pp = 0; pp < P; ++pp) xb[k2 * XS + pp] = (k2 == 0 || pp == 0) ? f[t][pp] : tw_mul<+1>(f[t][pp], tw, pp * k2);
       }
     }
     __syncwarp(mask);
 #pragma unroll
-    for (int k2 = 0; k2 < M; ++k2) v[k2] = xb[k2 * P + p];
+    for (int k2 = 0; k2 < M; ++k2) v[k2] = xb[k2 * XS + p];
     DFT<M, +1, Z>::run(v);
     __syncwarp(mask);
   }

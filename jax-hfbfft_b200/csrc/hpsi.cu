@@ -30,7 +30,7 @@ struct HpsiGeo {
   static constexpr int M = N / P;
   static constexpr int T = (M + P - 1) / P;
   static constexpr int LD = N + 4;                   // shared row stride (elements)
-  static constexpr int NB = N + 4;                   // exchange buffer per line
+  static constexpr int NB = Pencil<R, N, P>::XB;                   // exchange buffer per line
   static constexpr int THREADS = ((N * P + 31) / 32) * 32;
   static constexpr int LINES = THREADS / P;          // >= N (extra lines are idle)
   static constexpr size_t SMEM = sizeof(cplx<R>) * (size_t)(2 * N * LD + LINES * NB + N);

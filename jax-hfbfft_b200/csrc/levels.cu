@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(256)
 cderv_kernel(int nfield, const cplx<R>* __restrict__ in, const double* __restrict__ bf, double kscale, double k2scale,
              double nyq_scale, cplx<R>* d1, cplx<R>* d2) {
   constexpr int P = PencilSplit<R, N>::P;
-  constexpr int M = N / P, T = (M + P - 1) / P, L = 256 / P, NB = N + 4;
+  constexpr int M = N / P, T = (M + P - 1) / P, L = 256 / P, NB = Pencil<R, N, P>::XB;
   using PC = Pencil<R, N, P>;
   using Z = cplx<R>;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;

@@ -197,7 +197,7 @@ int density_derivatives(hfb_ctx_s* c, const double* rho, const double* cur, cons
 template <int N2, int AXIS>
 __global__ void __launch_bounds__(128) coul_fft_kernel(double2* a) {
   constexpr int P = PencilSplit<double, N2>::P;
-  constexpr int M = N2 / P, T = (M + P - 1) / P, L = 128 / P, NB = N2 + 4;
+  constexpr int M = N2 / P, T = (M + P - 1) / P, L = 128 / P, NB = Pencil<double, N2, P>::XB;
   using PC = Pencil<double, N2, P>;
   __shared__ __align__(16) double2 xball[L * NB];
   __shared__ double2 tw[N2];
@@ -299,7 +299,7 @@ int coulomb_init(hfb_ctx_s* c) {
 // complex array: 90 us at n2 = 96, 45 us here.)
 template <int N2> struct CoulGeo {
   static constexpr int P = PencilSplit<double, N2>::P, M = N2 / P, T = (M + P - 1) / P;
-  static constexpr int THREADS = 256, L = THREADS / P, NB = N2 + 4;
+  static constexpr int THREADS = 256, L = THREADS / P, NB = Pencil<double, N2, P>::XB;
   static constexpr int NZ = N2 / 2 + 1;
   static constexpr size_t SMEM = sizeof(double2) * ((size_t)N2 * NZ + L * NB + N2);
 };

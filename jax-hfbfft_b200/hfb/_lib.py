@@ -89,6 +89,7 @@ _PROTOS = {
     "hfb_poisson_noalloc": [vp, vp, vp, vp],
     "hfb_add_density": [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_double] + [vp] * 6 +
                        [C.POINTER(C.c_double), vp, vp],
+    "hfb_pair_density": [vp, C.c_int, C.c_int, C.c_int] + [vp] * 11,
     "hfb_sp_kinetic": [vp, C.c_int, C.c_int, C.c_int, vp, C.POINTER(C.c_double), vp, vp],
     "hfb_harmosc": [vp, C.c_int, C.c_int, vp, C.c_double, C.c_double, C.c_double, vp, vp],
     "hfb_grstep": [vp, C.c_int, C.POINTER(GrstepArgs), vp],
