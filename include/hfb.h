@@ -125,6 +125,12 @@ int hfb_skyrme(hfb_ctx_t ctx, const hfb_force* f, int tcoul, const double* rho, 
                double* wlspot, double* dbmass, double* wcoul, double* ecorrp, int prec, void* pot,
                void* stream);
 
+/* The packed hpsi potentials pot[2][12][n^3] (precision prec) from the six
+ * field arrays; a NULL field is zero (no counterpart in the reference, whose
+ * hpsi01 reads the arrays themselves). */
+int hfb_pack_pot(hfb_ctx_t ctx, int prec, const double* upot, const double* bmass, const double* v_pair,
+                 const double* aq, const double* spot, const double* wlspot, void* pot, void* stream);
+
 /* ---- coulomb.py -------------------------------------------------------- */
 /* poisson (coulomb.py:54-75): wcoul[nx][ny][nz] from the proton density. */
 int hfb_poisson(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream);

@@ -587,9 +587,35 @@ __global__ void ecorrp_kernel(size_t n3, const double* t, double wxyz, double* o
   }
 }
 
+// pot[iq][field][i] from the field arrays (null: zero).
+struct PackIn {
+  const double* f[6];   // upot, bmass, v_pair, aq, spot, wlspot
+};
+template <class R>
+__global__ void pack_pot_kernel(size_t n3, PackIn in, R* pot) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i >= n3) return;
+  const int k = blockIdx.y % 12, iq = blockIdx.y / 12;
+  const int a = k < 3 ? k : 3 + (k - 3) / 3;
+  const size_t row = k < 3 ? iq : iq * 3 + (k - 3) % 3;
+  pot[blockIdx.y * n3 + i] = in.f[a] ? (R)in.f[a][row * n3 + i] : R(0);
+}
+
 }  // namespace hfb
 
 using namespace hfb;
+
+extern "C" int hfb_pack_pot(hfb_ctx_t ctx, int prec, const double* upot, const double* bmass, const double* v_pair,
+                            const double* aq, const double* spot, const double* wlspot, void* pot, void* stream) {
+  if (!ctx || !pot) return HFB_ERR_ARG;
+  const size_t n3 = (size_t)ctx->n * ctx->n * ctx->n;
+  const dim3 grid((unsigned)((n3 + 255) / 256), 24);
+  const PackIn in{{upot, bmass, v_pair, aq, spot, wlspot}};
+  if (prec == HFB_F64) pack_pot_kernel<double><<<grid, 256, 0, as_stream(stream)>>>(n3, in, (double*)pot);
+  else pack_pot_kernel<float><<<grid, 256, 0, as_stream(stream)>>>(n3, in, (float*)pot);
+  HFB_CHECK_LAUNCH();
+  return HFB_OK;
+}
 
 extern "C" int hfb_poisson(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream) {
   if (!ctx || !rho_p || !wcoul) return HFB_ERR_ARG;

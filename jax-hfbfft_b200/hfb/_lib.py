@@ -85,6 +85,7 @@ _PROTOS = {
     "hfb_laplace": [vp, C.c_int, C.c_int, vp, vp, vp, C.c_double, C.c_double, C.c_double, vp, vp],
     "hfb_hpsi": [vp, C.c_int, vp, C.c_int, C.c_int, vp, vp, vp, vp, vp, vp, vp],
     "hfb_skyrme": [vp, C.POINTER(HfbForce), C.c_int] + [vp] * 6 + [vp] * 8 + [vp, vp, C.c_int, vp, vp],
+    "hfb_pack_pot": [vp, C.c_int] + [vp] * 8,
     "hfb_poisson": [vp, vp, vp, vp],
     "hfb_poisson_noalloc": [vp, vp, vp, vp],
     "hfb_add_density": [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_double] + [vp] * 6 +

@@ -27,11 +27,11 @@ Complex gradients follow torch's convention, dL = Re sum conj(x.grad) dx.
 States are [nst][2][nx][ny][nz], neutrons first (``nneut`` of them); fields
 are per isospin, [2][...].
 """
+from types import SimpleNamespace
+
 import torch
 
-from ._lib import call, ptr, stream_ptr, prec_of
-from .densities import init_densities
-from .meanfield import init_meanfield
+from ._lib import call, ptr, stream_ptr, prec_of, HFB_F64, HFB_F32
 
 _FIELDS = ("upot", "bmass", "v_pair", "aq", "spot", "wlspot")
 _DENS = ("rho", "chi", "tau", "current", "sdens", "sodens")
@@ -41,49 +41,50 @@ def _vec(x, nst, dev):
     return torch.as_tensor(x, dtype=torch.float64, device=dev).reshape(-1).expand(nst).contiguous()
 
 
+def _empty_densities(grids, dev):
+    """The six density arrays, to be written by the library."""
+    g = (grids.nx, grids.ny, grids.nz)
+    return {k: torch.empty(((2,) if k in _DENS[:3] else (2, 3)) + g, dtype=torch.float64, device=dev) for k in _DENS}
+
+
 def _densities(grids, psi, nneut, w, wu):
     """Densities of ``psi`` with occupation weights w and pairing weights wu."""
     nst = psi.shape[0]
-    d = init_densities(grids)
+    d = _empty_densities(grids, psi.device)
     one = torch.ones(nst, dtype=torch.float64, device=psi.device)
     call("hfb_add_density", grids.ctx.handle, prec_of(psi), nst, nneut, ptr(psi), ptr(w), ptr(wu), ptr(one), ptr(one),
-         1.0, ptr(d.rho), ptr(d.chi), ptr(d.tau), ptr(d.current), ptr(d.sdens), ptr(d.sodens), None, None,
-         stream_ptr())
+         1.0, *(ptr(d[k]) for k in _DENS), None, None, stream_ptr())
     return d
-
-
-def _axpby_diag(grids, a, x, b, y):
-    call("hfb_state_axpby_diag", grids.ctx.handle, prec_of(x), x.shape[0], ptr(a), ptr(x), float(b), ptr(y),
-         stream_ptr())
 
 
 def pair_densities(grids, a, b, nneut, w, wu):
     """sum_s w_s F(a_s, b_s) for rho, tau, current, sdens, sodens and
-    sum_s wu_s chi(a_s, b_s), the pair densities Re(a^dagger O_F b), by
-    polarisation of the density kernel (each pair balanced in norm)."""
-    nst = a.shape[0]
-    na = torch.linalg.vector_norm(a.reshape(nst, -1), dim=1).double()
-    nb = torch.linalg.vector_norm(b.reshape(nst, -1), dim=1).double()
-    ok = (na > 0) & (nb > 0)
-    s = torch.where(ok, torch.sqrt(nb / torch.where(ok, na, torch.ones_like(na))), torch.ones_like(na)).contiguous()
-    inv = (1.0 / s).contiguous()
-    p = torch.zeros_like(a)
-    m = torch.zeros_like(a)
-    _axpby_diag(grids, s, a, 0.0, p)       # p = s a
-    _axpby_diag(grids, s, a, 0.0, m)
-    _axpby_diag(grids, inv, b, 1.0, p)     # p = s a + b / s
-    _axpby_diag(grids, -inv, b, 1.0, m)    # m = s a - b / s
-    dp = _densities(grids, p, nneut, w, wu)
-    dm = _densities(grids, m, nneut, w, wu)
-    return {k: (getattr(dp, k) - getattr(dm, k)) * 0.25 for k in _DENS}
+    sum_s wu_s chi(a_s, b_s), the pair densities Re(a^dagger O_F b)."""
+    d = _empty_densities(grids, a.device)
+    call("hfb_pair_density", grids.ctx.handle, prec_of(a), a.shape[0], nneut, ptr(a), ptr(b), ptr(w), ptr(wu),
+         *(ptr(d[k]) for k in _DENS), stream_ptr())
+    return d
 
 
 def _pack(grids, fields, dtype):
-    """A Meanfield whose fields are ``fields`` (missing ones zero), packed."""
-    mf = init_meanfield(grids, dtype)
-    for k, v in fields.items():
-        getattr(mf, k).copy_(v)
-    return mf.pack(dtype)
+    """The packed hpsi potentials (``.pot``, [2][12][n^3] in the precision of
+    ``dtype``) of ``fields``; missing ones are zero."""
+    g = (grids.nx, grids.ny, grids.nz)
+    rd = torch.float64 if dtype == torch.complex128 else torch.float32
+    pot = torch.empty((2, 12) + g, dtype=rd, device="cuda")
+    src = []
+    for k in _FIELDS:
+        f = fields.get(k)
+        if f is not None:
+            shape = ((2,) if k in _FIELDS[:3] else (2, 3)) + g
+            if f.dtype != torch.float64 or not f.is_cuda:
+                f = f.detach().to(device="cuda", dtype=torch.float64)
+            if f.shape != shape or not f.is_contiguous():
+                f = torch.broadcast_to(f, shape).contiguous()
+        src.append(f)
+    call("hfb_pack_pot", grids.ctx.handle, HFB_F64 if rd == torch.float64 else HFB_F32, *(ptr(f) for f in src), ptr(pot),
+         stream_ptr())
+    return SimpleNamespace(pot=pot)
 
 
 def _hpsi(grids, pot, x, nneut, w, wu):
@@ -96,12 +97,12 @@ def _hpsi(grids, pot, x, nneut, w, wu):
 def hpsi_vjp(grids, pot, psi, nneut, w, wu, ybar):
     """(psi_bar, {field: cotangent}) for y = w h psi - wu v_pair psi."""
     nst = psi.shape[0]
-    psi_bar = _hpsi(grids, pot, ybar.contiguous(), nneut, w, wu)
-    pd = pair_densities(grids, ybar.contiguous(), psi, nneut, w, wu)
-    bmass = pd["tau"].clone()
-    call("hfb_nyquist_pair", grids.ctx.handle, prec_of(psi), nst, nneut, ptr(ybar.contiguous()), ptr(psi), ptr(w),
-         ptr(bmass), stream_ptr())
-    bars = dict(upot=pd["rho"], bmass=bmass, v_pair=-2.0 * pd["chi"], aq=pd["current"], spot=pd["sdens"],
+    ybar = ybar.contiguous()
+    psi_bar = _hpsi(grids, pot, ybar, nneut, w, wu)
+    pd = pair_densities(grids, ybar, psi, nneut, w, -2.0 * wu)
+    call("hfb_nyquist_pair", grids.ctx.handle, prec_of(psi), nst, nneut, ptr(ybar), ptr(psi), ptr(w), ptr(pd["tau"]),
+         stream_ptr())
+    bars = dict(upot=pd["rho"], bmass=pd["tau"], v_pair=pd["chi"], aq=pd["current"], spot=pd["sdens"],
                 wlspot=pd["sodens"])
     return psi_bar, bars
 
@@ -116,10 +117,8 @@ def densities_vjp(grids, psi, nneut, w, wu, bars):
     out = _hpsi(grids, mf.pot, psi, nneut, w2, (-wu).contiguous())
     tau = bars.get("tau")
     if tau is not None:
-        tmp = out.clone()
         call("hfb_nyquist_apply", grids.ctx.handle, prec_of(psi), psi.shape[0], nneut, ptr(tau.contiguous()), ptr(w2),
-             ptr(psi), ptr(tmp), stream_ptr())
-        out = tmp
+             ptr(psi), ptr(out), stream_ptr())
     return out
 
 
@@ -159,7 +158,7 @@ class Densities(torch.autograd.Function):
         d = _densities(grids, psi, nneut, w, wu)
         ctx.save_for_backward(psi, w, wu)
         ctx.grids, ctx.nneut = grids, nneut
-        return tuple(getattr(d, k) for k in _DENS)
+        return tuple(d[k] for k in _DENS)
 
     @staticmethod
     def backward(ctx, *grads):
