@@ -146,19 +146,18 @@ __global__ void gram_reduce_kernel(GramJob job, int nchunk, const double2* part,
 
 int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
                    const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz,
-                   double2* const* outs_host, int ldo, cudaStream_t st);   // gram_tc.cu
+                   double2* const* outs_host, int ldo, int leave, cudaStream_t st);   // gram_tc.cu
 
 // One launch for the requested matrices of up to two state blocks.
 // outs[b * 4 + a] receives matrix a of block b (leading dimension ldo); the
-// FP64 tensor-core launch stays off ``leave`` SMs.
+// tensor-core launches stay off ``leave`` SMs.
 
 int gram_launch(hfb_ctx_s* c, int prec, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
                 const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz, double2* const* outs_host,
                 int ldo, cudaStream_t st, int leave = 0) {
   // single precision: tensor cores (three-term tf32) unless disabled for this context
   if (prec != HFB_F64 && c->use_tcgen05) {
-    const int mk[2] = {masks[0] & 15, nblk > 1 ? masks[1] & 15 : 0};
-    const int r = gram_tc_launch(c, nblk, s0, ns, mk, psi, hampsi, hmfpsi, vp, wxyz, outs_host, ldo, st);
+    const int r = gram_tc_launch(c, nblk, s0, ns, masks, psi, hampsi, hmfpsi, vp, wxyz, outs_host, ldo, leave, st);
     if (r != HFB_ERR_UNSUPPORTED_GRID) return r;
   }
   const size_t n3 = (size_t)c->n * c->n * c->n, K = 2 * n3;

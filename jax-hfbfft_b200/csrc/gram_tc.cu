@@ -1,114 +1,148 @@
 // Single-precision Gram matrices on the tcgen05 tensor cores.
 //
-// C_a = wxyz Psi^H X_a (X = psi, hampsi, hmfpsi, v_pair psi; static.py:
-// 283-290, 380-387 and construct_hfb_matrices 484-577) for complex64 states.
-// The complex product is written as one real GEMM over the interleaved
-// (re, im) storage: with A' = [Psi ; Psi~] (Psi~ row = (-im, re) per
-// element), D = A' X^T gives Re C in rows 0..n-1 and Im C in rows n..2n-1.
-// Operands are split as x = hi + lo with hi = tf32(x), lo = x - hi (exact,
-// left unrounded: the MMA takes its tf32 part) and D accumulates hi*hi +
-// hi*lo + lo*hi (the three-term tf32 scheme, about 21 significant bits per
-// product).
+// C_a[i][j] = wxyz <psi_i | x_j> (X = psi, hampsi, hmfpsi, v_pair psi;
+// static.py:283-290, 380-387 and construct_hfb_matrices 484-577) for complex64
+// states.  Operands are split as x = hi + lo with hi = tf32(x), lo = x - hi
+// (exact, left unrounded: the MMA takes its tf32 part) and D accumulates
+// hi*hi + hi*lo + lo*hi (the three-term tf32 scheme, about 21 significant
+// bits per product).
 //
-// One CTA owns one 128-row block of A' for one matrix and one slice of K.
-// (Feeding the K blocks by TMA, with A split into tensor memory as the
-// rotation does, measured slower here: 2.9-3.2 ms against 2.0 ms for the
-// 140 Pb208 neutron states, with 8-row or 128-row boxes and with a deeper
-// raw ring; the split of B then sits on six warps instead of seven, four
-// of which also split A.)
-//   warps 0-6   load a 32-float K block of the rows from global memory,
+// A unit is 128 rows x_j (the requested matrices' vectors j, interleaved) by
+// up to 144 columns psi_i of one isospin.  Producers store real and imaginary
+// parts of 16 points side by side in a 128-byte row, so one staged block
+// serves both
+//   D_re = x_r psi_r + x_i psi_i   and   D_im = x_i psi_r - x_r psi_i
+// (the minus sign is the descriptor's).  Only one triangle is computed: i >= j
+// of S and of lambda (the eigensolver reads its lower triangle; all of lambda
+// when the caller wants it), i <= j of H and G, whose rows go by descending j.
+// The columns of a block start or end at its first row's j, which leaves 56 %
+// of them for two matrices of 140 states.
+//
+// Work items are (K slice, unit), handed out by a ticket to one CTA per SM
+// (fewer when the launch is to leave SMs to what runs beside it).  The slices
+// depend on the grid alone, so no sum's order depends on which matrices are
+// computed together.
+//   warps 0-6   load a block of 16 points of the rows from global memory (the
+//               next block's loads are in flight while this one is split),
 //               split it and store it into a 128-byte-swizzled stage
 //               (3-stage ring);
-//   warp 7      issues the MMAs (M = 128, N = n padded to 16, K = 8) into
-//               one of two TMEM accumulators, which starts from zero every
-//               four K blocks;
-//   warps 8-15  drain the finished accumulator into fp32 registers every
-//               four K blocks, so the tensor core's own fp32 accumulation
+//   warp 7      issues the MMAs (M = 128, N = columns, K = 8) into TMEM
+//               accumulators, three in rotation for D_re and D_im, which start
+//               from zero every four blocks;
+//   warps 8-15  drain the finished accumulator into fp32 registers, four warps
+//               D_re and four D_im, so the tensor core's own fp32 accumulation
 //               spans at most 48 MMAs and the sum over drains is rounded to
 //               nearest.
 // Per-slice partial sums are added in fp64 in a fixed order by a second
-// kernel, which also scatters Re/Im rows into the complex outputs.
+// kernel, which also writes the mirrored elements.
+// A row that is also a column (S, G) is loaded once and stored twice.
+// Bound by the producers: rows lie a state apart (1.8 MB at 48^3), every row of
+// a block is another page, and a block's 35 KB take 1.4 us to arrive although
+// its lines were brought into L2 four blocks before (MMAs alone: 1.0 us).
+// Pb208 (140 + 96 states,
+// 48^3), S + lambda and H + G: 3.04 ms with the real and imaginary rows in
+// units of their own (each loaded and split separately), 2.4 ms here.
+// (Feeding the blocks by TMA into a raw ring measured slower for that form.)
 // Every wait is bounded; a timeout latches HFB_ERR_CUDA, drains the MMAs
 // in flight and releases TMEM before returning.
 #include <math.h>
-#include "hfb_ctx.cuh"
+#include <algorithm>
+#include "diag.cuh"
 #include "tc_sm100.cuh"
 
 namespace hfb {
 
 namespace {
 
-constexpr int kTcProducerWarps = 7;   // 16 warps in all: 4 per SM sub-partition, 128 registers each
+constexpr int kTcProducerWarps = 7;
 constexpr int kTcEpilogueWarps = 8;
 constexpr int kTcThreads = 32 * (kTcProducerWarps + 1 + kTcEpilogueWarps);
+// registers: 512 x 128 at launch, then 256 x 72 + 256 x 184
+constexpr int kTcProducerRegs = 72, kTcEpilogueRegs = 184;
 constexpr int kTcStages = 3;
-constexpr int kTcMaxNp = 160;           // padded states per block handled here
-constexpr int kTcMaxGroups = 5;         // 16-column groups per epilogue thread
+constexpr int kTcMaxNp = 160;           // padded states per isospin handled here
+constexpr int kTcMaxCols = 144;         // columns of a unit: the epilogue's accumulator registers
 constexpr int kTcMaxUnits = 32;
-constexpr int kTcRowsPerPass = kTcProducerWarps * 32 / 8;   // 8 threads per 128-byte row
-constexpr int kTcItemsA = (128 + kTcRowsPerPass - 1) / kTcRowsPerPass;
-constexpr int kTcItemsB = (kTcMaxNp + kTcRowsPerPass - 1) / kTcRowsPerPass;
-constexpr int kTcTmemCols = 512;        // two accumulators at columns 0 and 256
+constexpr int kTcItems = 5;             // 32-byte row quarters per producer thread and block
+static_assert(kTcItems * kTcProducerWarps * 32 >= 4 * (128 + kTcMaxCols), "producer share");
+constexpr int kTcTmemCols = 512, kTcAccCols = 160;   // three accumulators
+// up to this many states hi*(hi|lo) is one MMA of twice the columns (Zr90, 61 +
+// 47 states, 40^3: 337 us against 360); by the states of the isospin, not the
+// columns of the unit, so that it depends on nothing else
+constexpr int kTcPairCols = kTcAccCols / 2;
 constexpr uint32_t kTcABytes = 128 * 128;   // 128 rows x 128 bytes
+constexpr uint32_t kTcStageBytes = 2 * kTcABytes + 2 * kTcMaxCols * 128;
 constexpr long long kTcWaitLimit = 2000000000LL;
-// K blocks accumulated in TMEM between drains into registers: 4 measured
-// 6 % faster than 1 on Pb208 (1.96 ms against 2.09 ms for the 140 neutron
-// states) and stays inside the 3e-6 bar of the single-precision Gram test
+// Blocks accumulated in TMEM between drains into registers: 4 measured 6 %
+// faster than 1 and stays inside the 3e-6 bar of the single-precision Gram
+// test
 constexpr int kTcDrain = 4;
+// blocks that a row's line is brought into L2 ahead of its load
+constexpr int kTcAhead = 4;
+// K slices: enough that the last wave of items is short, at least six drains
+constexpr int kTcMaxSlices = 148, kTcMinSlice = 24;
+constexpr int kTcMaxWin = 48 * 48 * 48 / 8 / kTcMaxSlices + 1;   // blocks of a slice of the largest grid
+constexpr size_t kTcSmem = 1024 + kTcStages * kTcStageBytes + sizeof(float) * 16 * kTcMaxWin;
+static_assert(kTcMaxWin > 2 * kTcMinSlice, "slices of small grids");
+
+constexpr uint32_t kNone = 0xffffffffu;
+enum TcGroup { TC_LOWER = 0, TC_UPPER = 1, TC_FULL = 2, TC_GROUPS = 3 };   // S and lambda; H and G; lambda
 
 struct TcUnit {
-  unsigned char b, a, mb, pad;
+  unsigned char b, group;      // isospin, TcGroup
+  short row0, col0, cols;      // first stacked row; first column and padded count
 };
 struct TcJob {
-  int nunit, kchunks, kb_total, n3;
-  int drain;                      // K blocks accumulated in TMEM between drains
+  int nunit, slices, kb_total, n3;
   TcUnit u[kTcMaxUnits];
-  int s0[2], ns[2], np[2];
+  int s0[2], ns[2];
+  int nm[2][TC_GROUPS];        // [isospin][group] matrices stacked
+  unsigned char mat[2][TC_GROUPS][2];   // their numbers
   const double* vp[2];
-  signed char unit_of[2][4][4];   // [block][matrix][m-block] -> unit
 };
 
-__device__ __forceinline__ uint32_t stage_bytes(int np) { return 2 * kTcABytes + 2 * (uint32_t)np * 128; }
+// volatile: the load stays where it is issued, a block ahead of its use
+__device__ __forceinline__ void ldg8(float4 (&v)[2], const float* p) {
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
+                 "=f"(v[1].w)
+               : "l"(p));
+}
+__device__ __forceinline__ void prefetch_l2(const float* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
+}
+__device__ __forceinline__ void tc_sync_all() { asm volatile("bar.sync 1, %0;" ::"n"(kTcThreads) : "memory"); }
 
 __global__ void __launch_bounds__(kTcThreads, 1)
-gram_tc_kernel(TcJob job, const float* __restrict__ psi, const float* __restrict__ hampsi,
-               const float* __restrict__ hmfpsi, float* __restrict__ part, int* status) {
+gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi, const float* __restrict__ hampsi,
+               const float* __restrict__ hmfpsi, float* __restrict__ part, int* ticket, int* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[kTcStages], empty[kTcStages], dfull[2], dempty[2], fin;
+  __shared__ uint64_t full[kTcStages], empty[kTcStages], dfull[3], dempty[3], fin;
   __shared__ uint32_t tbase;
   __shared__ volatile int abort_flag;
+  __shared__ volatile int next[2];
 
-  const int unit = blockIdx.x % job.nunit, chunk = blockIdx.x / job.nunit;
-  const TcUnit U = job.u[unit];
-  const int b = U.b, am = U.a, mb = U.mb;
-  const int n = job.ns[b], np = job.np[b];
-  const size_t K = 2 * (size_t)job.n3;                 // complex elements per state
-  const int kb0 = (int)((long long)job.kb_total * chunk / job.kchunks);
-  const int kb1 = (int)((long long)job.kb_total * (chunk + 1) / job.kchunks);
-  const int nwin = kb1 - kb0;
-  const uint32_t sbytes = stage_bytes(np);
+  float* vps = reinterpret_cast<float*>(smem + kTcStages * kTcStageBytes);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
-
+  const int items = job.nunit * job.slices;
   if (tid == 0) {
     for (int s = 0; s < kTcStages; ++s) {
       tc::mbar_init(&full[s], kTcProducerWarps);
       tc::mbar_init(&empty[s], 1);
     }
-    for (int d = 0; d < 2; ++d) {
+    for (int d = 0; d < 3; ++d) {
       tc::mbar_init(&dfull[d], 1);
-      tc::mbar_init(&dempty[d], kTcEpilogueWarps);
+      tc::mbar_init(&dempty[d], kTcEpilogueWarps / 2);
     }
     tc::mbar_init(&fin, 1);
     abort_flag = 0;
+    next[0] = atomicAdd(ticket, 1);
   }
   if (warp == kTcProducerWarps) {
     tc::tmem_alloc(&tbase, kTcTmemCols);
     tc::tmem_relinquish();
   }
-  // zero every stage once: padding rows are never written again
-  for (uint32_t e = tid; e < kTcStages * sbytes / 16; e += blockDim.x)
-    reinterpret_cast<float4*>(smem)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   tc::fence_before();
   __syncthreads();
@@ -128,151 +162,237 @@ gram_tc_kernel(TcJob job, const float* __restrict__ psi, const float* __restrict
     }
     return true;
   };
+  // The next item, or -1; every role calls it once per item, after its part of
+  // the last one.  The first block of the slice in kb0, their number in nwin.
+  auto take = [&](int it, int& kb0, int& nwin) -> int {
+    tc_sync_all();
+    const int item = next[it & 1];
+    if (item >= items || abort_flag) return -1;
+    const int slice = item / job.nunit;
+    kb0 = (int)((long long)job.kb_total * slice / job.slices);
+    nwin = (int)((long long)job.kb_total * (slice + 1) / job.slices) - kb0;
+    return item;
+  };
+  int kb0, nwin;
 
-  if (warp < kTcProducerWarps) {
-    // ---------------------------------------------------------- producers
-    const int c = tid & 7;            // 16-byte chunk of the 128-byte row
-    const int r0 = tid >> 3;          // first row; rows r0 + kTcRowsPerPass i
-    const size_t rowf = 2 * K;        // floats per state
-    // A' rows: state index (or -1) and whether the row is Psi~
-    int rowA[kTcItemsA];
-    unsigned tmask = 0;
+  if (warp <= kTcProducerWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcProducerRegs));
+    if (warp < kTcProducerWarps) {
+      // -------------------------------------------------------- producers
+      const size_t rowf = 4 * (size_t)job.n3;             // floats per state
+      const int q = tid & 3;                              // 32-byte quarter of the row
+      int w = 0;                                          // blocks since the start
+      for (int it = 0;; ++it) {
+        const int item = take(it, kb0, nwin);
+        if (item < 0) break;
+        if (tid == 0) next[(it + 1) & 1] = atomicAdd(ticket, 1);
+        const TcUnit U = job.u[item % job.nunit];
+        const int b = U.b, n = job.ns[b], nm = job.nm[b][U.group];
+        const size_t start = (size_t)job.s0[b] * rowf + (size_t)kb0 * 32 + 8 * q;
+        const float* src[kTcItems];
+        uint32_t dst[kTcItems], dup[kTcItems];   // place, and for a column that is also a row, that place
+        unsigned gmask = 0;
+        const bool shared_row = job.mat[b][U.group][U.group == TC_UPPER ? nm - 1 : 0] == (U.group == TC_UPPER ? 3 : 0);
 #pragma unroll
-    for (int i = 0; i < kTcItemsA; ++i) {
-      const int rl = r0 + kTcRowsPerPass * i, rg = mb * 128 + rl;
-      rowA[i] = rl >= 128 ? -1 : rg < n ? rg : (rg < 2 * n ? rg - n : -1);
-      if (rg >= n && rg < 2 * n) tmask |= 1u << i;
-    }
-    const float* pa = psi + (size_t)job.s0[b] * rowf;
-    const float* pb = (am == 1 ? hampsi : am == 2 ? hmfpsi : psi) + (size_t)job.s0[b] * rowf;
-    const double* vp = job.vp[b];
-    for (int w = 0; w < nwin; ++w) {
-      const int s = w % kTcStages;
-      if (w >= kTcStages && !wait(&empty[s], (uint32_t)((w / kTcStages - 1) & 1))) break;
-      const size_t off = (size_t)(kb0 + w) * 32 + 4 * c;
-      float4 va[kTcItemsA], vb[kTcItemsB];
-#pragma unroll
-      for (int i = 0; i < kTcItemsA; ++i)
-        if (rowA[i] >= 0) va[i] = __ldg(reinterpret_cast<const float4*>(pa + (size_t)rowA[i] * rowf + off));
-#pragma unroll
-      for (int i = 0; i < kTcItemsB; ++i) {
-        const int j = r0 + kTcRowsPerPass * i;
-        if (j < n) vb[i] = __ldg(reinterpret_cast<const float4*>(pb + (size_t)j * rowf + off));
-      }
-      float v0 = 1.f, v1 = 1.f;
-      if (am == 3) {
-        const size_t k = (off / 2) % (size_t)job.n3;
-        v0 = (float)vp[k];
-        v1 = (float)vp[k + 1];
-      }
-      unsigned char* st = smem + (size_t)s * sbytes;
-      auto put = [&](unsigned char* hi_base, uint32_t lo_delta, int row, float4 v) {
-        float4 h, l;
-        tc::split_tf32(v.x, h.x, l.x);
-        tc::split_tf32(v.y, h.y, l.y);
-        tc::split_tf32(v.z, h.z, l.z);
-        tc::split_tf32(v.w, h.w, l.w);
-        const uint32_t o = tc::sw128_offset(row, c);
-        *reinterpret_cast<float4*>(hi_base + o) = h;
-        *reinterpret_cast<float4*>(hi_base + lo_delta + o) = l;
-      };
-#pragma unroll
-      for (int i = 0; i < kTcItemsA; ++i) {
-        if (rowA[i] < 0) continue;
-        float4 v = va[i];
-        if ((tmask >> i) & 1) v = make_float4(-v.y, v.x, -v.w, v.z);
-        put(st, kTcABytes, r0 + kTcRowsPerPass * i, v);
-      }
-#pragma unroll
-      for (int i = 0; i < kTcItemsB; ++i) {
-        const int j = r0 + kTcRowsPerPass * i;
-        if (j >= n) continue;
-        float4 v = vb[i];
-        if (am == 3) v = make_float4(v0 * v.x, v0 * v.y, v1 * v.z, v1 * v.w);
-        put(st + 2 * kTcABytes, (uint32_t)np * 128, j, v);
-      }
-      tc::fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&full[s]);
-    }
-  } else if (warp == kTcProducerWarps) {
-    // ---------------------------------------------------------------- MMA
-    if (lane == 0) {
-      const uint32_t idesc = tc::idesc_tf32(128, np);
-      for (int w = 0; w < nwin; ++w) {
-        const int s = w % kTcStages, e = w / job.drain, d = e & 1;
-        const bool first = w % job.drain == 0, last = w % job.drain == job.drain - 1 || w == nwin - 1;
-        if (!wait(&full[s], (uint32_t)((w / kTcStages) & 1))) break;
-        if (first && e >= 2 && !wait(&dempty[d], (uint32_t)((e / 2 - 1) & 1))) break;
-        tc::fence_after();
-        const uint32_t sa = tc::smem_u32(smem + (size_t)s * sbytes);
-        const uint32_t ahi = sa, alo = sa + kTcABytes, bhi = sa + 2 * kTcABytes, blo = bhi + (uint32_t)np * 128;
-        const uint32_t dt = tmem + (uint32_t)(d * 256);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          tc::mma_tf32(dt, tc::sw128_desc(ahi + 32 * k), tc::sw128_desc(bhi + 32 * k), idesc, k > 0 || !first);
-          tc::mma_tf32(dt, tc::sw128_desc(ahi + 32 * k), tc::sw128_desc(blo + 32 * k), idesc, 1);
-          tc::mma_tf32(dt, tc::sw128_desc(alo + 32 * k), tc::sw128_desc(bhi + 32 * k), idesc, 1);
+        for (int p = 0; p < kTcItems; ++p) {
+          // eight threads store rows r and r + 4: their chunks fall on
+          // distinct banks
+          const int e = (p * kTcProducerWarps * 32 + tid) >> 2;
+          int r = (e & ~7) | ((e & 7) >> 1) | ((e & 1) << 2);
+          const float* base = nullptr;
+          dup[p] = kNone;
+          if (r < 128) {
+            const int g = U.row0 + r, j = U.group == TC_UPPER ? n - 1 - g / nm : g / nm;
+            if (g < n * nm) {
+              const int a = job.mat[b][U.group][g % nm];
+              const bool here = (a == 0 || a == 3) && j >= U.col0 && j < U.col0 + U.cols;
+              if (!here) base = (a == 1 ? hampsi : a == 2 ? hmfpsi : psi) + (size_t)j * rowf;
+              if (a == 3) gmask |= 1u << p;
+            }
+            dst[p] = tc::sw128_offset(r, q);
+          } else {
+            r -= 128;
+            const int i = U.col0 + r;
+            if (r < U.cols && i < n) {
+              base = psi + (size_t)i * rowf;
+              const int g = U.group == TC_UPPER ? (n - 1 - i) * nm + nm - 1 - U.row0 : i * nm - U.row0;
+              if (shared_row && g >= 0 && g < 128) dup[p] = tc::sw128_offset(g, q);
+            }
+            dst[p] = 2 * kTcABytes + tc::sw128_offset(r, q);
+          }
+          src[p] = base ? base + start : nullptr;
         }
-        tc::mma_commit(&empty[s]);
-        if (last) tc::mma_commit(&dfull[d]);
+        float4 d[kTcItems][2];
+        auto load = [&](int p) {
+          if (src[p]) {
+            ldg8(d[p], src[p]);
+            src[p] += 32;
+          }
+        };
+#pragma unroll
+        for (int p = 0; p < kTcItems; ++p) load(p);
+        if (job.mat[b][U.group][nm - 1] == 3) {   // v_pair of the slice
+          const double* vp = job.vp[b];
+          for (int e = tid; e < 16 * nwin; e += 32 * kTcProducerWarps)
+            vps[e] = (float)vp[((size_t)kb0 * 16 + e) % (size_t)job.n3];
+          asm volatile("bar.sync 2, %0;" ::"n"(32 * kTcProducerWarps) : "memory");
+        }
+        auto scale = [&](float4 (&x)[2], int i) {
+          const float4 v = *reinterpret_cast<const float4*>(vps + 16 * i + 4 * q);
+          x[0] = make_float4(v.x * x[0].x, v.x * x[0].y, v.y * x[0].z, v.y * x[0].w);
+          x[1] = make_float4(v.z * x[1].x, v.z * x[1].y, v.w * x[1].z, v.w * x[1].w);
+        };
+        auto put = [&](unsigned char* o, uint32_t lo, const float4 (&x)[2]) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {   // real parts, imaginary parts
+            float4 h, l;
+            tc::split_tf32(c ? x[0].y : x[0].x, h.x, l.x);
+            tc::split_tf32(c ? x[0].w : x[0].z, h.y, l.y);
+            tc::split_tf32(c ? x[1].y : x[1].x, h.z, l.z);
+            tc::split_tf32(c ? x[1].w : x[1].z, h.w, l.w);
+            unsigned char* t = reinterpret_cast<unsigned char*>((uintptr_t)o ^ (c ? 64u : 0u));
+            *reinterpret_cast<float4*>(t) = h;
+            *reinterpret_cast<float4*>(t + lo) = l;
+          }
+        };
+        for (int i = 0; i < nwin; ++i, ++w) {
+          const int s = w % kTcStages;
+          if (w >= kTcStages && !wait(&empty[s], (uint32_t)((w / kTcStages - 1) & 1))) break;
+          unsigned char* st = smem + (size_t)s * kTcStageBytes;
+#pragma unroll
+          for (int p = 0; p < kTcItems; ++p) {
+            if (!src[p]) continue;
+            const bool isb = dst[p] >= 2 * kTcABytes;
+            const uint32_t lo = isb ? (uint32_t)U.cols * 128 : kTcABytes;
+            if ((gmask >> p) & 1) scale(d[p], i);
+            put(st + dst[p], lo, d[p]);
+            if (dup[p] != kNone) {
+              if (U.group == TC_UPPER) scale(d[p], i);
+              put(st + dup[p], kTcABytes, d[p]);
+            }
+            if (i + 1 < nwin) load(p);
+            if (q == 0 && i + kTcAhead < nwin) prefetch_l2(src[p] + 32 * (kTcAhead - 2));
+          }
+          tc::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&full[s]);
+        }
       }
-      // every MMA issued above has completed once this arrives
-      tc::mma_commit(&fin);
-      if (!tc::mbar_wait(&fin, 0, kTcWaitLimit)) latch_error(status, HFB_ERR_CUDA);
+    } else {
+      // -------------------------------------------------------------- MMA
+      int w = 0, grp = 0, nfin = 0;
+      const bool one = tc::elect_one();
+      const uint64_t stage0 = tc::sw128_desc(tc::smem_u32(smem));
+      for (int it = 0;; ++it) {
+        const int item = take(it, kb0, nwin);
+        if (item < 0) break;
+        // the whole warp runs the loop, so that descriptors stay uniform
+        const uint32_t cols = __shfl_sync(0xffffffffu, (uint32_t)job.u[item % job.nunit].cols, 0);
+        const uint32_t idesc = tc::idesc_tf32(128, cols), ineg = idesc | tc::kNegateA, lob = (cols * 128) >> 4;
+        constexpr uint64_t loa = kTcABytes >> 4;
+        const bool pair = __shfl_sync(0xffffffffu, job.ns[job.u[item % job.nunit].b], 0) <= kTcPairCols;
+        const uint32_t idpair = tc::idesc_tf32(128, 2 * cols) - tc::idesc_tf32(128, cols);
+        bool ok = true;
+        for (int i = 0; i < nwin && ok; ++i, ++w) {
+          const int s = w % kTcStages, er = 2 * grp, ei = er + 1;
+          const bool first = i % kTcDrain == 0, last = i % kTcDrain == kTcDrain - 1 || i == nwin - 1;
+          ok = wait(&full[s], (uint32_t)((w / kTcStages) & 1));
+          if (first && er >= 3 && ok) ok = wait(&dempty[er % 3], (uint32_t)((er / 3 - 1) & 1));
+          if (!ok) break;
+          tc::fence_after();
+          const uint64_t da = stage0 + (uint64_t)((uint32_t)s * (kTcStageBytes >> 4)), db = da + 2 * loa;
+          const uint32_t dr = tmem + (uint32_t)(er % 3) * kTcAccCols, di = tmem + (uint32_t)(ei % 3) * kTcAccCols;
+          auto mma3 = [&](uint32_t dt, int ka, int kb, uint32_t id, uint32_t acc) {
+            if (pair) {
+              tc::mma_tf32(dt, da + 2 * ka, db + 2 * kb, id + idpair, acc);
+            } else {
+              tc::mma_tf32(dt, da + 2 * ka, db + 2 * kb, id, acc);
+              tc::mma_tf32(dt, da + 2 * ka, db + lob + 2 * kb, id, 1);
+            }
+            tc::mma_tf32(dt, da + loa + 2 * ka, db + 2 * kb, id, 1);
+          };
+          // k steps 0, 1 of a row: real parts, 2, 3: imaginary parts
+          if (one) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mma3(dr, k, k, idesc, k > 0 || !first);
+            if (last) tc::mma_commit(&dfull[er % 3]);
+          }
+          __syncwarp();
+          if (first && ei >= 3) ok = wait(&dempty[ei % 3], (uint32_t)((ei / 3 - 1) & 1));
+          if (!ok) break;
+          tc::fence_after();
+          if (one) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) mma3(di, 2 + k, k, idesc, k > 0 || !first);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) mma3(di, k, 2 + k, ineg, 1);
+            tc::mma_commit(&empty[s]);
+            if (last) tc::mma_commit(&dfull[ei % 3]);
+          }
+          __syncwarp();
+          if (last) ++grp;
+        }
+        // every MMA issued above has completed once this arrives
+        if (one) tc::mma_commit(&fin);
+        __syncwarp();
+        if (!tc::mbar_wait(&fin, (uint32_t)(nfin & 1), kTcWaitLimit)) {
+          abort_flag = 1;
+          latch_error(status, HFB_ERR_CUDA);
+        }
+        ++nfin;
+        __syncwarp();
+      }
     }
-    __syncwarp();
   } else {
     // ----------------------------------------------------------- epilogue
-    const int q = warp & 3;                       // TMEM lane quarter of this warp
-    const int half = (warp - kTcProducerWarps - 1) / 4;   // two warps per quarter split the columns
-    const int ng = np / 16, g0 = (ng + 1) / 2;
-    const int gbeg = half ? g0 : 0, gcnt = half ? ng - g0 : g0;
-    float acc[kTcMaxGroups][16];
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcEpilogueRegs));
+    const int qd = warp & 3;                              // TMEM lane quarter of this warp
+    const int im = (warp - kTcProducerWarps - 1) / 4;     // D_re or D_im
+    int grp = 0;
+    for (int it = 0;; ++it) {
+      const int item = take(it, kb0, nwin);
+      if (item < 0) break;
+      const int ng = job.u[item % job.nunit].cols / 16;
+      const bool pair = job.ns[job.u[item % job.nunit].b] <= kTcPairCols;
+      float acc[kTcMaxCols / 16][16];
 #pragma unroll
-    for (int g = 0; g < kTcMaxGroups; ++g)
+      for (int g = 0; g < kTcMaxCols / 16; ++g)
 #pragma unroll
-      for (int i = 0; i < 16; ++i) acc[g][i] = 0.f;
-    bool ok = true;
-    const int nep = (nwin + job.drain - 1) / job.drain;
-    for (int e = 0; e < nep; ++e) {
-      const int d = e & 1;
-      if (!wait(&dfull[d], (uint32_t)((e / 2) & 1))) { ok = false; break; }
-      tc::fence_after();
-      const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * 256);
-      // two groups per load where possible: fewer load-wait round trips
+        for (int i = 0; i < 16; ++i) acc[g][i] = 0.f;
+      bool ok = true;
+      for (int i = 0; i < nwin; i += kTcDrain, ++grp) {
+        const int e = 2 * grp + im;
+        if (!wait(&dfull[e % 3], (uint32_t)((e / 3) & 1))) { ok = false; break; }
+        tc::fence_after();
+        const uint32_t ta = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(e % 3) * kTcAccCols;
 #pragma unroll
-      for (int g = 0; g < kTcMaxGroups; g += 2) {
-        if (g + 1 < gcnt) {
-          float v[32];
-          tc::tmem_ld32(ta + (uint32_t)((gbeg + g) * 16), v);
+        for (int g = 0; g < kTcMaxCols / 16; ++g)
+          if (g < ng) {
+            float v[16];
+            tc::tmem_ld16(ta + (uint32_t)(g * 16), v);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            acc[g][i] += v[i];
-            acc[g + 1][i] += v[16 + i];
+            for (int c = 0; c < 16; ++c) acc[g][c] += v[c];
+            if (pair) {
+              tc::tmem_ld16(ta + (uint32_t)((ng + g) * 16), v);
+#pragma unroll
+              for (int c = 0; c < 16; ++c) acc[g][c] += v[c];
+            }
           }
-        } else if (g < gcnt) {
-          float v[16];
-          tc::tmem_ld16(ta + (uint32_t)((gbeg + g) * 16), v);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[g][i] += v[i];
-        }
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&dempty[e % 3]);
       }
-      tc::fence_before();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&dempty[d]);
-    }
-    if (ok && !abort_flag) {
-      const int row = q * 32 + lane;
-      float* o = part + ((size_t)blockIdx.x * 128 + row) * kTcMaxNp;
+      if (ok && !abort_flag) {
+        float* o = part + (((size_t)item * 2 + im) * 128 + qd * 32 + lane) * kTcMaxCols;
 #pragma unroll
-      for (int g = 0; g < kTcMaxGroups; ++g)
-        if (g < gcnt) {
+        for (int g = 0; g < kTcMaxCols / 16; ++g)
+          if (g < ng) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4)
-            *reinterpret_cast<float4*>(o + (gbeg + g) * 16 + i) =
-                make_float4(acc[g][i], acc[g][i + 1], acc[g][i + 2], acc[g][i + 3]);
-        }
+            for (int i = 0; i < 16; i += 4)
+              *reinterpret_cast<float4*>(o + g * 16 + i) =
+                  make_float4(acc[g][i], acc[g][i + 1], acc[g][i + 2], acc[g][i + 3]);
+          }
+      }
     }
   }
   tc::fence_before();
@@ -287,28 +407,54 @@ struct TcOut {
   double2* p[8];   // [block * 4 + matrix]
 };
 
-// out_a[b][i][j] = wxyz * (Re, Im) from rows i and n + i of A' X^T, the
-// K slices summed in fp64 in order; Hermitian matrices mirror the upper
-// triangle.
-__global__ void gram_tc_reduce_kernel(TcJob job, const float* __restrict__ part, double scale, TcOut outs, int ldo,
-                                      int bq, int aq) {
-  const int b = bq, am = aq;
-  const int n = job.ns[b];
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n * n) return;
-  const int i = e / n, j = e % n;
-  const bool herm = am != 1;
-  if (herm && i > j) return;
-  const int rre = i, rim = n + i;
-  const int ure = job.unit_of[b][am][rre / 128], uim = job.unit_of[b][am][rim / 128];
-  double re = 0.0, im = 0.0;
-  for (int c = 0; c < job.kchunks; ++c) {
-    re += (double)part[(((size_t)c * job.nunit + ure) * 128 + (rre % 128)) * kTcMaxNp + j];
-    im += (double)part[(((size_t)c * job.nunit + uim) * 128 + (rim % 128)) * kTcMaxNp + j];
+// out_a[b][i][j] = wxyz (D_re, D_im)[row of j][column of i], the K slices
+// summed in fp64 in a fixed order (six interleaved sums, then those in turn).
+// One block per row of a unit: four columns a thread, six threads over the
+// slices.  (A launch per matrix and isospin with one thread per element: 73 us
+// of a 2.3 ms Zr90 step.)
+constexpr int kTcRedLanes = 6, kTcRedCols = kTcMaxCols / 4;
+__global__ void __launch_bounds__(kTcRedLanes* kTcRedCols)
+gram_tc_reduce_kernel(const __grid_constant__ TcJob job, const float* __restrict__ part, double scale,
+                      const __grid_constant__ TcOut outs, int ldo, int* ticket) {
+  __shared__ double red[kTcRedLanes][kTcRedCols][8];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *ticket = 0;   // for the next launch
+  const TcUnit U = job.u[blockIdx.y];
+  const int row = blockIdx.x, b = U.b, n = job.ns[b], nm = job.nm[b][U.group];
+  const int g = U.row0 + row;
+  if (g >= n * nm) return;
+  const int j = U.group == TC_UPPER ? n - 1 - g / nm : g / nm, am = job.mat[b][U.group][g % nm];
+  const int c4 = threadIdx.x % kTcRedCols, sl = threadIdx.x / kTcRedCols;
+  const bool on = 4 * c4 < U.cols;
+  double s[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s[i] = 0.0;
+  if (on) {
+    const float* p = part + ((size_t)blockIdx.y * 2 * 128 + row) * kTcMaxCols + 4 * c4;
+#pragma unroll 4
+    for (int c = sl; c < job.slices; c += kTcRedLanes) {
+      const float* o = p + (size_t)c * job.nunit * 2 * 128 * kTcMaxCols;
+      const float4 re = *reinterpret_cast<const float4*>(o);
+      const float4 im = *reinterpret_cast<const float4*>(o + 128 * kTcMaxCols);
+      s[0] += re.x; s[1] += re.y; s[2] += re.z; s[3] += re.w;
+      s[4] += im.x; s[5] += im.y; s[6] += im.z; s[7] += im.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) red[sl][c4][i] = s[i];
   }
+  __syncthreads();
+  if (sl != 0 || !on) return;
+#pragma unroll
+  for (int q = 1; q < kTcRedLanes; ++q)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] += red[q][c4][i];
   double2* out = outs.p[b * 4 + am];
-  out[(size_t)i * ldo + j] = make_double2(scale * re, scale * im);
-  if (herm && i != j) out[(size_t)j * ldo + i] = make_double2(scale * re, -scale * im);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = U.col0 + 4 * c4 + k;
+    if (i >= n || (U.group == TC_LOWER && i < j) || (U.group == TC_UPPER && i > j)) continue;
+    out[(size_t)i * ldo + j] = make_double2(scale * s[k], scale * s[4 + k]);
+    if (am != 1 && i != j) out[(size_t)j * ldo + i] = make_double2(scale * s[k], -scale * s[4 + k]);
+  }
 }
 
 }  // namespace
@@ -317,61 +463,52 @@ __global__ void gram_tc_reduce_kernel(TcJob job, const float* __restrict__ part,
 // (the caller then uses the CUDA-core kernel).
 int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
                    const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz,
-                   double2* const* outs_host, int ldo, cudaStream_t st) {
+                   double2* const* outs_host, int ldo, int leave, cudaStream_t st) {
   TcJob job{};
   job.n3 = c->n * c->n * c->n;
-  job.kb_total = (int)(4 * (size_t)job.n3 / 32);
-  for (int b = 0; b < 2; ++b)
-    for (int a = 0; a < 4; ++a)
-      for (int m = 0; m < 4; ++m) job.unit_of[b][a][m] = -1;
+  job.kb_total = job.n3 / 8;
   for (int b = 0; b < nblk; ++b) {
     if (ns[b] <= 0) continue;
+    const int n = ns[b];
     job.s0[b] = s0[b];
-    job.ns[b] = ns[b];
-    job.np[b] = (ns[b] + 15) / 16 * 16;
+    job.ns[b] = n;
     job.vp[b] = vp ? vp[b] : nullptr;
-    if (job.np[b] > kTcMaxNp) return HFB_ERR_UNSUPPORTED_GRID;
-    const int nmb = (2 * ns[b] + 127) / 128;
+    if ((n + 15) / 16 * 16 > kTcMaxNp) return HFB_ERR_UNSUPPORTED_GRID;
     for (int a = 0; a < 4; ++a) {
       if (!(masks[b] & (1 << a))) continue;
-      for (int m = 0; m < nmb; ++m) {
-        if (job.nunit >= kTcMaxUnits) return HFB_ERR_UNSUPPORTED_GRID;
-        job.unit_of[b][a][m] = (signed char)job.nunit;
-        job.u[job.nunit++] = TcUnit{(unsigned char)b, (unsigned char)a, (unsigned char)m, 0};
+      const int g = a >= 2 ? TC_UPPER : a == 1 && !(masks[b] & kGramLowerLambda) ? TC_FULL : TC_LOWER;
+      job.mat[b][g][job.nm[b][g]++] = (unsigned char)a;
+    }
+    for (int g = 0; g < TC_GROUPS; ++g) {
+      const int nm = job.nm[b][g];
+      for (int row0 = 0; row0 < n * nm; row0 += 128) {
+        const int first = g == TC_LOWER ? row0 / nm / 16 * 16 : 0, end = g == TC_UPPER ? n - row0 / nm : n;
+        const int all = (end - first + 15) / 16 * 16;
+        const int parts = (all + kTcMaxCols - 1) / kTcMaxCols, cols = (all / 16 + parts - 1) / parts * 16;
+        for (int col0 = first; col0 < end; col0 += cols) {
+          if (job.nunit >= kTcMaxUnits) return HFB_ERR_UNSUPPORTED_GRID;
+          job.u[job.nunit++] = TcUnit{(unsigned char)b, (unsigned char)g, (short)row0, (short)col0,
+                                      (short)std::min(cols, (end - col0 + 15) / 16 * 16)};
+        }
       }
     }
   }
   if (job.nunit == 0) return HFB_OK;
-  // about one wave of single-CTA SMs
-  int nsm = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  }
-  job.drain = kTcDrain;
-  job.kchunks = nsm / job.nunit;
-  if (job.kchunks < 1) job.kchunks = 1;
-  if (job.kchunks > job.kb_total) job.kchunks = job.kb_total;
-  const int ncta = job.nunit * job.kchunks;
-  float* part = (float*)scratch(c, hfb_ctx_s::S_GRAM, sizeof(float) * (size_t)ncta * 128 * kTcMaxNp);
+  // the widest units first, so that the last items of a launch are short
+  std::stable_sort(job.u, job.u + job.nunit, [](const TcUnit& x, const TcUnit& y) { return x.cols > y.cols; });
+  job.slices = std::max(1, std::min(kTcMaxSlices, job.kb_total / kTcMinSlice));
+  const int items = job.nunit * job.slices, sms = c->sms - leave;
+  float* part = (float*)scratch(c, hfb_ctx_s::S_GRAM, sizeof(float) * (size_t)items * 2 * 128 * kTcMaxCols);
   if (!part) return HFB_ERR_ALLOC;
-  int npmax = 16;
-  for (int b = 0; b < nblk; ++b) npmax = job.np[b] > npmax ? job.np[b] : npmax;
-  const size_t smem = 1024 + (size_t)kTcStages * (2 * kTcABytes + 2 * (size_t)npmax * 128);
+  int* ticket = c->counters + 1;
   allow_max_dynamic_smem(gram_tc_kernel);
-  gram_tc_kernel<<<ncta, kTcThreads, smem, st>>>(job, (const float*)psi, (const float*)hampsi,
-                                                 (const float*)hmfpsi, part, c->dev_status);
+  gram_tc_kernel<<<std::min(items, sms), kTcThreads, kTcSmem, st>>>(job, (const float*)psi, (const float*)hampsi,
+                                                                   (const float*)hmfpsi, part, ticket, c->dev_status);
   HFB_CHECK_LAUNCH();
   TcOut ot;
   for (int q = 0; q < 8; ++q) ot.p[q] = outs_host[q];
-  for (int b = 0; b < nblk; ++b)
-    for (int a = 0; a < 4; ++a) {
-      if (ns[b] <= 0 || !(masks[b] & (1 << a))) continue;
-      const int nn = ns[b] * ns[b];
-      gram_tc_reduce_kernel<<<(nn + 255) / 256, 256, 0, st>>>(job, part, wxyz, ot, ldo, b, a);
-      HFB_CHECK_LAUNCH();
-    }
+  gram_tc_reduce_kernel<<<dim3(128, job.nunit), kTcRedLanes * kTcRedCols, 0, st>>>(job, part, wxyz, ot, ldo, ticket);
+  HFB_CHECK_LAUNCH();
   return HFB_OK;
 }
 
