@@ -6,424 +6,525 @@
 // D the real n x n first-derivative matrix with its k = 0 and n/2 bins zero,
 // B the effective mass, L_d the pointwise 2x2 current / spin-orbit operator
 // of the axis and the Nyquist term (pi/d)^2 mean_line(B) (-1)^j
-// sum_l (-1)^l x_l / n of cderv02 (levels.py:314-330).  D on the N lines of
-// a staged plane is a real GEMM, D (N x N) times the plane's values (N
-// points x N lines x 2 spinor components x re/im), run as 8 x 8 x 4 FP64
-// MMAs: an MMA tile is 8 points x 4 lines x re/im, with both spinor
-// components in two accumulators, so after GEMM 1 a thread holds e for one
-// point and line in both components -- what the pointwise step needs.  w =
-// L_d x - B e goes to a second plane buffer for GEMM 2; the thread's own
-// tiles come back from GEMM 2 in the same positions.
+// sum_l (-1)^l x_l / n of cderv02 (levels.py:314-330).
 //
-// Kernels as in the FFT path: A (one CTA per state and x-plane) runs the z
-// lines with the local upot / spin terms and then the y lines, accumulating
-// in global memory (L2-resident between passes); B (one CTA per state and
-// y-plane) runs the x lines and the final weights and overlaps.  The
-// derivative matrices (one per axis) are built in double on the host at
-// context creation.
+// D changes sign when both its indices are reversed (j -> n-1-j), so with
+// x-[l] = x[l] - x[n-1-l], x+[l] = x[l] + x[n-1-l] for l < n/2,
+//     (D x)[j] = (Dm x-)[j] + (Dp x+)[j],  (D x)[n-1-j] = (Dm x-)[j] - (Dp x+)[j],
+//     Dm[j][l] = (D[j][l] - D[j][n-1-l]) / 2,  Dp[j][l] = (D[j][l] + D[j][n-1-l]) / 2,
+// two products with (n/2) x (n/2) matrices: half the MMAs of D itself.
+//
+// A warp owns one MMA tile of a staged plane, 8 points j < n/2 and their
+// mirrors on 8 lines, both spinor components: after GEMM 1 a thread holds
+// D x at 4 (point, line) positions in both components, does the pointwise
+// step on them, stores w+- for GEMM 2 and gets the same positions back.
+//
+// Two kernels: X (x-planes: z lines with the local terms, then y lines; what
+// the z lines give waits in the w buffer, at the thread's own positions) and
+// Y (y-planes: x lines, the final weights and overlaps).  Both are
+// persistent: the derivative matrices stay in shared memory, and the next
+// plane is copied in (cp.async) from the moment the plane's last reader has
+// passed, behind GEMM 2.  In the z pass only the warps of the same lines wait
+// for one another, so that some warps' MMAs run beside others' pointwise
+// step.  (A warp of its own for the copies took registers from the others:
+// 2.0 ms for X at 48^3 against 1.5.)  Planes are stored without padding, 16-byte elements
+// XOR-swizzled by row so that fragment loads along rows and columns hit
+// distinct banks.
+//
+// Bound by the tensor pipe and the pointwise FP64 work in turn.  Pb208 (236
+// states, 48^3): 4.87 ms a call with the full D, eight warps on five rounds
+// of tiles and the partial sums in global memory; 2.5 ms here.
 #include <math.h>
 #include <vector>
-#include "hfb_ctx.cuh"
+#include "diag.cuh"
 #include "hpsi.cuh"
 
 namespace hfb {
 
 namespace {
 
-constexpr int kHdWarps = 8;
-constexpr int kHdThreads = 32 * kHdWarps;
-
 template <int N>
 struct HdGeo {
-  static constexpr int LD = N + 4;                     // complex elements per staged row (rows half a bank set apart)
-  static constexpr int MB = N / 8;                     // 8-point blocks of a line
-  static constexpr int LG = N / 8;                     // 8-line groups of a plane
-  static constexpr int NT = MB * LG;                   // MMA tiles per pass
-  static constexpr int TMAX = (NT + kHdWarps - 1) / kHdWarps;
-  static constexpr int KS = N / 4;                     // k steps
-  static constexpr size_t PLANE = (size_t)2 * N * LD;  // complex elements of one staged plane
-  static constexpr int DLD = N + 4;                    // row stride of a staged D: rows 8 banks apart
-  // plane, w buffer, alternating sums [2][N]; two derivative matrices, line means of B
-  static constexpr size_t SMEM = sizeof(double2) * (2 * PLANE + 2 * N) + sizeof(double) * (2 * (size_t)N * DLD + N);
-  static_assert(N % 8 == 0, "grid size");
+  static constexpr int H = N / 2;                     // points of a half line
+  static constexpr int MB = (H + 7) / 8;              // 8-point blocks of it
+  static constexpr int LG = N / 8;                    // 8-line groups of a plane
+  static constexpr int WARPS = MB * LG, THREADS = 32 * WARPS;   // one warp per tile
+  static constexpr int KS = H / 4;                    // MMA k steps
+  static constexpr int HP = 8 * MB;                   // rows of Dm, Dp (zero past H)
+  static constexpr int LDH = H % 16 == 4 || H % 16 == 12 ? H : H + 4;   // row stride: rows on distinct banks
+  static constexpr int DSZ = 2 * HP * LDH;            // doubles of Dm, Dp of one axis
+  static constexpr size_t PLANE = (size_t)2 * N * N;  // complex elements of a plane
+  static constexpr size_t smem(int axes) { return sizeof(double2) * (2 * PLANE + axes * 2 * N) + sizeof(double) * axes * (DSZ + N); }
+  // CTAs per SM that shared memory and the registers allow for
+  static constexpr int CTAS = N >= 40 ? 1 : N == 32 ? 2 : N == 24 ? 4 : 8;
+  static_assert(N % 8 == 0 && (LDH % 16 == 4 || LDH % 16 == 12), "grid size");
 };
 
-__device__ __forceinline__ void hd_mma(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
+// Element (component, row, column) of a plane.
+template <int N>
+__device__ __forceinline__ int hd_el(int c, int row, int col) {
+  return (c * N + row) * N + (col ^ (((row & 1) * 5) | (row & 2)));
 }
-
-// Staged plane buf[c][a][b] (row stride LD); a "line" of the pass runs along
-// b (ROW) or along a, and pt is the position along it.
+// A "line" of a pass runs along the columns (ROW) or along the rows; pt is
+// the position along it.
 template <int N, bool ROW>
 __device__ __forceinline__ int hd_at(int c, int line, int pt) {
-  using G = HdGeo<N>;
-  return ROW ? (c * N + line) * G::LD + pt : (c * N + pt) * G::LD + line;
+  return ROW ? hd_el<N>(c, line, pt) : hd_el<N>(c, pt, line);
 }
 
-}  // namespace
-
-namespace {
-
+// A thread's place in its warp's tile: point j (mirror N-1-j), lines l and
+// l + 1; fragment row / line fr, k index fk.
+struct HdTile {
+  int j0, l0, fr, fk, j, l;
+  bool on;    // j is a point (not padding)
+};
 template <int N>
-constexpr int hd_dld() { return HdGeo<N>::DLD; }
+__device__ __forceinline__ HdTile hd_tile() {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  HdTile t;
+  t.fr = lane >> 2;
+  t.fk = lane & 3;
+  t.j0 = 8 * (warp % HdGeo<N>::MB);
+  t.l0 = 8 * (warp / HdGeo<N>::MB);
+  t.j = t.j0 + t.fr;
+  t.l = t.l0 + 2 * t.fk;
+  t.on = t.j < HdGeo<N>::H;
+  return t;
+}
 
-// One axis pass over the N lines of the staged plane X: emits the axis's
-// contribution to h x at every point of the plane, both spinor components,
-// through emit(line, j, g, out0, out1, pre(g)) (g the point's index in the
-// state; pre's global loads are issued before the tile's GEMM 2 MMAs).
-// Dm is D for the axis (row stride hd_dld), W a second plane buffer, alt and
-// bbar per-line scratch; lines start at base + line * sa (ROW) or base +
-// line * sb, points are sb (ROW) or sa apart.  Ends with a CTA barrier.
-template <int N, int AXIS, bool ROW, bool LOCAL, class Pre, class Emit>
-__device__ __forceinline__ void hd_pass(const double2* X, double2* W, const double* Dm, double2* alt, double* bbar,
-                                        const double* pot, size_t base, size_t sa, size_t sb, double nq, Pre&& pre,
-                                        Emit&& emit) {
+// d[half][line][component] = D applied along the lines; S holds the values
+// themselves (PLAIN; ``alt`` then gets sum (-1)^l x_l of line l0 + fr) or
+// their +- combinations at positions l and N-1-l.
+template <int N, bool ROW, bool PLAIN>
+__device__ __forceinline__ void hd_gemm(const double2* S, const double* Dm, const HdTile& t, double2 (&d)[2][2][2],
+                                        double2 (&alt)[2]) {
   using G = HdGeo<N>;
-  constexpr size_t N3 = (size_t)N * N * N;
-  constexpr int DLD = hd_dld<N>();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  auto gidx = [&](int line, int j) -> size_t {
-    return ROW ? base + (size_t)line * sa + (size_t)j * sb : base + (size_t)j * sa + (size_t)line * sb;
-  };
-  // Nyquist ingredients per line (levels.py:314-330): sum_l (-1)^l x_l of
-  // both components and the line mean of B; one warp per line, lanes over
-  // the points, a fixed shuffle tree
-  for (int line = warp; line < N; line += kHdWarps) {
-    double ax0 = 0.0, ay0 = 0.0, ax1 = 0.0, ay1 = 0.0, bs = 0.0;
-    for (int l = lane; l < N; l += 32) {
-      const double sgn = (l & 1) ? -1.0 : 1.0;
-      const double2 v0 = X[hd_at<N, ROW>(0, line, l)], v1 = X[hd_at<N, ROW>(1, line, l)];
-      ax0 += sgn * v0.x;
-      ay0 += sgn * v0.y;
-      ax1 += sgn * v1.x;
-      ay1 += sgn * v1.y;
-      bs += pot[1 * N3 + gidx(line, l)];
-    }
+  const double* am = Dm + t.j * G::LDH + t.fk;
+  const double* ap = am + G::HP * G::LDH;
+  double m[4][2], p[4][2];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ax0 += __shfl_xor_sync(0xffffffffu, ax0, o);
-      ay0 += __shfl_xor_sync(0xffffffffu, ay0, o);
-      ax1 += __shfl_xor_sync(0xffffffffu, ax1, o);
-      ay1 += __shfl_xor_sync(0xffffffffu, ay1, o);
-      bs += __shfl_xor_sync(0xffffffffu, bs, o);
+  for (int i = 0; i < 4; ++i) m[i][0] = m[i][1] = p[i][0] = p[i][1] = 0.0;
+  if (PLAIN) alt[0] = alt[1] = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int ks = 0; ks < G::KS; ++ks) {
+    const int pt = 4 * ks + t.fk, line = t.l0 + t.fr;
+    const double a = am[4 * ks], b = ap[4 * ks];
+    double2 u[2], v[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      u[c] = S[hd_at<N, ROW>(c, line, pt)];
+      v[c] = S[hd_at<N, ROW>(c, line, N - 1 - pt)];
+      if (PLAIN) {
+        const double2 s = u[c] + v[c], r = u[c] - v[c];
+        u[c] = s;
+        v[c] = r;
+        alt[c] = alt[c] + r;
+      }
     }
-    if (lane == 0) {
-      alt[line] = make_double2(ax0, ay0);
-      alt[N + line] = make_double2(ax1, ay1);
-      bbar[line] = bs / N;
+    gd_mma(m[0], a, v[0].x);
+    gd_mma(p[0], b, u[0].x);
+    gd_mma(m[1], a, v[0].y);
+    gd_mma(p[1], b, u[0].y);
+    gd_mma(m[2], a, v[1].x);
+    gd_mma(p[2], b, u[1].x);
+    gd_mma(m[3], a, v[1].y);
+    gd_mma(p[3], b, u[1].y);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      d[0][u][c] = make_double2(m[2 * c][u] + p[2 * c][u], m[2 * c + 1][u] + p[2 * c + 1][u]);
+      d[1][u][c] = make_double2(m[2 * c][u] - p[2 * c][u], m[2 * c + 1][u] - p[2 * c + 1][u]);
+    }
+  if (PLAIN) {
+    // (-1)^l = (-1)^fk, the mirror's sign is opposite; sum over the four k lanes
+    const double sg = (t.fk & 1) ? -1.0 : 1.0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      alt[c] = sg * alt[c];
+#pragma unroll
+      for (int o = 1; o <= 2; o *= 2) {
+        alt[c].x += __shfl_xor_sync(0xffffffffu, alt[c].x, o);
+        alt[c].y += __shfl_xor_sync(0xffffffffu, alt[c].y, o);
+      }
     }
   }
-  // Tile: 8 points x 8 lines.  MMA fragments: A = D row j0 + lane/4, k =
-  // lane%4; B = line l0 + lane/4 at point k, one MMA each for the re and im
-  // parts of the two spinor components (one double2 load gives both parts);
-  // C = point j0 + lane/4, lines l0 + 2 (lane%4) + {0, 1}.
+}
+
+// The pointwise step of an axis at one point: q = L_d e (+ local terms) and
+// n = L_d a (w without its -B e).
+template <int AXIS, bool LOCAL>
+__device__ __forceinline__ void hd_point(const double* pot, size_t n3, size_t g, const double2 (&a)[2],
+                                         const double2 (&e)[2], double2 (&q)[2], double2 (&w)[2]) {
   const double h = 0.5;
-  double2 o[G::TMAX][2][2];   // [tile][line of the pair][component]
-  // ---- GEMM 1: e = D x, then o = L_d e (+ local terms), w = L_d x - B e
-#pragma unroll
-  for (int ti = 0; ti < G::TMAX; ++ti) {
-    const int t = warp + ti * kHdWarps;
-    if (t < G::NT) {
-      const int j0 = (t / G::LG) * 8, l0 = (t % G::LG) * 8;
-      const int j = j0 + (lane >> 2), lp = l0 + 2 * (lane & 3);
-      // this tile's pointwise inputs are loaded before its MMAs, which hide
-      // their latency
-      double bm[2], aqd[2], w0[2], w1[2], w2[2], up[2], s0[2], s1[2], s2[2];
-      size_t g[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        g[u] = gidx(lp + u, j);
-        bm[u] = pot[1 * N3 + g[u]];
-        aqd[u] = pot[(3 + AXIS) * N3 + g[u]];
-        w0[u] = pot[9 * N3 + g[u]];
-        w1[u] = pot[10 * N3 + g[u]];
-        w2[u] = pot[11 * N3 + g[u]];
-        up[u] = LOCAL ? pot[g[u]] : 0.0;
-        s0[u] = LOCAL ? pot[6 * N3 + g[u]] : 0.0;
-        s1[u] = LOCAL ? pot[7 * N3 + g[u]] : 0.0;
-        s2[u] = LOCAL ? pot[8 * N3 + g[u]] : 0.0;
-      }
-      double acc[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-      for (int ks = 0; ks < G::KS; ++ks) {
-        const int pt = ks * 4 + (lane & 3);
-        const double a = Dm[(j0 + (lane >> 2)) * DLD + pt];
-        const double2 x0 = X[hd_at<N, ROW>(0, l0 + (lane >> 2), pt)];
-        const double2 x1 = X[hd_at<N, ROW>(1, l0 + (lane >> 2), pt)];
-        hd_mma(acc[0], a, x0.x);
-        hd_mma(acc[1], a, x0.y);
-        hd_mma(acc[2], a, x1.x);
-        hd_mma(acc[3], a, x1.y);
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int line = lp + u;
-        const double2 e0 = make_double2(acc[0][u], acc[1][u]), e1 = make_double2(acc[2][u], acc[3][u]);
-        const double2 a0 = X[hd_at<N, ROW>(0, line, j)], a1 = X[hd_at<N, ROW>(1, line, j)];
-        double2 q0, q1, n0, n1;
-        if (LOCAL) {
-          // upot psi + sigma.spot psi (meanfield.py:47-58)
-          q0 = (up[u] + s2[u]) * a0 + cmulri(s0[u], -s1[u], a1);
-          q1 = (up[u] - s2[u]) * a1 + cmulri(s0[u], s1[u], a0);
-        } else {
-          q0 = make_double2(0.0, 0.0);
-          q1 = make_double2(0.0, 0.0);
-        }
-        const double aq = aqd[u], v0 = w0[u], v1 = w1[u], v2 = w2[u];
-        if (AXIS == 0) {
-          // meanfield.py:63-83
-          q0 = q0 + cmulri(0.0, -(h * aq - h * v1), e0) - (h * v2) * e1;
-          q1 = q1 + cmulri(0.0, -(h * aq + h * v1), e1) + (h * v2) * e0;
-          n0 = cmulri(0.0, -h * (aq - v1), a0) - (h * v2) * a1;
-          n1 = cmulri(0.0, -h * (aq + v1), a1) + (h * v2) * a0;
-        } else if (AXIS == 1) {
-          // meanfield.py:92-112
-          q0 = q0 + cmulri(0.0, -(h * aq + h * v0), e0) + cmulri(0.0, h * v2, e1);
-          q1 = q1 + cmulri(0.0, -(h * aq - h * v0), e1) + cmulri(0.0, h * v2, e0);
-          n0 = cmulri(0.0, -h * (aq + v0), a0) + cmulri(0.0, h * v2, a1);
-          n1 = cmulri(0.0, -h * (aq - v0), a1) + cmulri(0.0, h * v2, a0);
-        } else {
-          // meanfield.py:121-141
-          q0 = q0 + cmulri(0.0, -(h * aq), e0) + cmulri(h * v0, -(h * v1), e1);
-          q1 = q1 + cmulri(0.0, -(h * aq), e1) + cmulri(-(h * v0), -(h * v1), e0);
-          n0 = cmulri(0.0, -h * aq, a0) + cmulri(h * v0, -(h * v1), a1);
-          n1 = cmulri(0.0, -h * aq, a1) + cmulri(-(h * v0), -(h * v1), a0);
-        }
-        o[ti][u][0] = q0;
-        o[ti][u][1] = q1;
-        W[hd_at<N, ROW>(0, line, j)] = n0 - bm[u] * e0;
-        W[hd_at<N, ROW>(1, line, j)] = n1 - bm[u] * e1;
-      }
-    }
+  const double bm = pot[1 * n3 + g], aq = pot[(3 + AXIS) * n3 + g];
+  const double v0 = AXIS != 0 ? pot[9 * n3 + g] : 0.0, v1 = AXIS != 1 ? pot[10 * n3 + g] : 0.0,
+               v2 = AXIS != 2 ? pot[11 * n3 + g] : 0.0;
+  q[0] = q[1] = make_double2(0.0, 0.0);
+  if (LOCAL) {
+    // upot psi + sigma.spot psi (meanfield.py:47-58)
+    const double up = pot[g], s0 = pot[6 * n3 + g], s1 = pot[7 * n3 + g], s2 = pot[8 * n3 + g];
+    q[0] = (up + s2) * a[0] + cmulri(s0, -s1, a[1]);
+    q[1] = (up - s2) * a[1] + cmulri(s0, s1, a[0]);
   }
-  __syncthreads();
-  // ---- GEMM 2: r = D w; out = o + r + Nyquist term
-#pragma unroll
-  for (int ti = 0; ti < G::TMAX; ++ti) {
-    const int t = warp + ti * kHdWarps;
-    if (t < G::NT) {
-      const int j0 = (t / G::LG) * 8, l0 = (t % G::LG) * 8;
-      const int j = j0 + (lane >> 2), lp = l0 + 2 * (lane & 3);
-      const size_t g0 = gidx(lp, j), g1 = gidx(lp + 1, j);
-      const auto pv0 = pre(g0);
-      const auto pv1 = pre(g1);
-      double acc[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-      for (int ks = 0; ks < G::KS; ++ks) {
-        const int pt = ks * 4 + (lane & 3);
-        const double a = Dm[(j0 + (lane >> 2)) * DLD + pt];
-        const double2 x0 = W[hd_at<N, ROW>(0, l0 + (lane >> 2), pt)];
-        const double2 x1 = W[hd_at<N, ROW>(1, l0 + (lane >> 2), pt)];
-        hd_mma(acc[0], a, x0.x);
-        hd_mma(acc[1], a, x0.y);
-        hd_mma(acc[2], a, x1.x);
-        hd_mma(acc[3], a, x1.y);
-      }
-      const double nqj = (j & 1) ? -nq : nq;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int line = lp + u;
-        const double sg = nqj * bbar[line];
-        const double2 r0 = o[ti][u][0] + make_double2(acc[0][u], acc[1][u]) + sg * alt[line];
-        const double2 r1 = o[ti][u][1] + make_double2(acc[2][u], acc[3][u]) + sg * alt[N + line];
-        emit(line, j, u == 0 ? g0 : g1, r0, r1, u == 0 ? pv0 : pv1);
-      }
-    }
+  if (AXIS == 0) {
+    // meanfield.py:63-83
+    q[0] = q[0] + cmulri(0.0, -(h * aq - h * v1), e[0]) - (h * v2) * e[1];
+    q[1] = q[1] + cmulri(0.0, -(h * aq + h * v1), e[1]) + (h * v2) * e[0];
+    w[0] = cmulri(0.0, -h * (aq - v1), a[0]) - (h * v2) * a[1];
+    w[1] = cmulri(0.0, -h * (aq + v1), a[1]) + (h * v2) * a[0];
+  } else if (AXIS == 1) {
+    // meanfield.py:92-112
+    q[0] = q[0] + cmulri(0.0, -(h * aq + h * v0), e[0]) + cmulri(0.0, h * v2, e[1]);
+    q[1] = q[1] + cmulri(0.0, -(h * aq - h * v0), e[1]) + cmulri(0.0, h * v2, e[0]);
+    w[0] = cmulri(0.0, -h * (aq + v0), a[0]) + cmulri(0.0, h * v2, a[1]);
+    w[1] = cmulri(0.0, -h * (aq - v0), a[1]) + cmulri(0.0, h * v2, a[0]);
+  } else {
+    // meanfield.py:121-141
+    q[0] = q[0] + cmulri(0.0, -(h * aq), e[0]) + cmulri(h * v0, -(h * v1), e[1]);
+    q[1] = q[1] + cmulri(0.0, -(h * aq), e[1]) + cmulri(-(h * v0), -(h * v1), e[0]);
+    w[0] = cmulri(0.0, -h * aq, a[0]) + cmulri(h * v0, -(h * v1), a[1]);
+    w[1] = cmulri(0.0, -h * aq, a[1]) + cmulri(-(h * v0), -(h * v1), a[0]);
   }
-  __syncthreads();
+  w[0] = w[0] - bm * e[0];
+  w[1] = w[1] - bm * e[1];
 }
 
-}  // namespace
+// First half of an axis pass: GEMM 1, the lines' alternating sums into alts,
+// the pointwise step and w+- into W; out[half][line][component] = L_d D x
+// (+ local terms) (+ what W held at the thread's positions, ADD).  The point
+// (line, pt) of the plane is element base + line * sl + pt * sp of a field.
+template <int N, int AXIS, bool ROW, bool LOCAL, bool ADD>
+__device__ __forceinline__ void hd_first(const double2* X, double2* W, const double* Dm, double2* alts, const HdTile& t,
+                                         const double* pot, size_t base, size_t sl, size_t sp,
+                                         double2 (&out)[2][2][2]) {
+  constexpr size_t N3 = (size_t)N * N * N;
+  double2 e[2][2][2], alt[2];
+  hd_gemm<N, ROW, true>(X, Dm, t, e, alt);
+  if (t.j0 == 0 && t.fk == 0) {
+    alts[t.l0 + t.fr] = alt[0];
+    alts[N + t.l0 + t.fr] = alt[1];
+  }
+  if (!t.on) return;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int line = t.l + u;
+    double2 w[2][2];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      const int pt = f ? N - 1 - t.j : t.j;
+      const double2 a[2] = {X[hd_at<N, ROW>(0, line, pt)], X[hd_at<N, ROW>(1, line, pt)]};
+      hd_point<AXIS, LOCAL>(pot, N3, base + line * sl + pt * sp, a, e[f][u], out[f][u], w[f]);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (ADD) out[f][u][c] = out[f][u][c] + W[hd_at<N, ROW>(c, line, pt)];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      W[hd_at<N, ROW>(c, line, t.j)] = w[0][c] + w[1][c];
+      W[hd_at<N, ROW>(c, line, N - 1 - t.j)] = w[0][c] - w[1][c];
+    }
+  }
+}
 
-namespace {
+// Second half: GEMM 2 on w+-, and the Nyquist term, added to out; bb is the
+// line mean of B of the plane's lines, nq = (pi/d)^2 / n.
+template <int N, bool ROW>
+__device__ __forceinline__ void hd_second(const double2* W, const double* Dm, const double2* alts, const double* bb,
+                                          double nq, const HdTile& t, double2 (&out)[2][2][2]) {
+  double2 r[2][2][2], none[2];
+  hd_gemm<N, ROW, false>(W, Dm, t, r, none);
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const double sg = ((t.j & 1) ? -nq : nq) * bb[t.l + u];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const double2 al = sg * alts[c * N + t.l + u];   // the mirror's sign is opposite
+      out[0][u][c] = out[0][u][c] + r[0][u][c] + al;
+      out[1][u][c] = out[1][u][c] + r[1][u][c] - al;
+    }
+  }
+}
 
+// Barrier of the warps of a line group (tiles of the same lines).
 template <int N>
-__device__ __forceinline__ void hd_load_d(double* dst, const double* src) {
-  constexpr int DLD = hd_dld<N>();
-#pragma unroll 4
-  for (int e = threadIdx.x; e < N * N; e += kHdThreads) dst[(e / N) * DLD + e % N] = src[e];
+__device__ __forceinline__ void hd_sync_group() {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x >> 5) / HdGeo<N>::MB), "n"(32 * HdGeo<N>::MB) : "memory");
+}
+// Start the copy of a plane: rows of N elements ``pitch`` apart, components
+// N^3 apart.
+template <int N>
+__device__ __forceinline__ void hd_stage(double2* X, const double2* src, size_t pitch) {
+  for (int e = threadIdx.x; e < 2 * N * N; e += HdGeo<N>::THREADS) {
+    const int c = e / (N * N), r = e / N % N, q = e % N;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(X + hd_el<N>(c, r, q))),
+                 "l"(src + (size_t)c * N * N * N + r * pitch + q)
+                 : "memory");
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+// The line means of B of the plane's lines: from the launch's table, or, when
+// a CTA has few planes, from the plane of B (element b[line * sl + i * sp]).
+template <int N>
+__device__ __forceinline__ void hd_means(double* dst, const double* __restrict__ table, const double* __restrict__ b,
+                                         size_t sl, size_t sp, int tid) {
+  for (int line = tid; line >= 0 && line < N; line += HdGeo<N>::THREADS) {
+    double m = 0.0;
+    if (table) {
+      m = table[line];
+    } else {
+#pragma unroll 8
+      for (int i = 0; i < N; ++i) m += b[line * sl + i * sp];
+      m /= N;
+    }
+    dst[line] = m;
+  }
+}
+__device__ __forceinline__ void hd_staged() {
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
 }
 
-// Values an emit step reads from global memory, loaded before its MMAs.
-struct HdPre {
-  double2 m0, m1;   // the state's partial h psi, both components
-  double vp;        // v_pair
+struct HdArgs {
+  const double* pot;
+  const double* bbar;      // [iq][axis][line], or null
+  const double2* psi;
+  double2* acc;
+  int s0, ns, nneut;
+  const double* dmat;      // [axis][Dm, Dp]
+  double nq[3];
+  const double *weight, *weightuv;
+  double2 *pout, *pout_mf, *pout_del;
+  double* ovl;
 };
 
-// A: one x-plane of one state; z lines with the local terms, then y lines.
+// X: an x-plane of a state; z lines with the local terms, then y lines.
 template <int N>
-__global__ void __launch_bounds__(kHdThreads)
-hpsi_dmma_x_kernel(const double* __restrict__ pot, const double2* __restrict__ psi, double2* acc, int s0, int nneut,
-                   const double* __restrict__ dmat, double nq_y, double nq_z) {
+__global__ void __launch_bounds__(HdGeo<N>::THREADS, HdGeo<N>::CTAS) hpsi_dmma_x_kernel(const __grid_constant__ HdArgs a) {
   using G = HdGeo<N>;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
-  constexpr int DLD = hd_dld<N>();
   extern __shared__ __align__(16) unsigned char hd_smem[];
-  double2* plane = reinterpret_cast<double2*>(hd_smem);
-  double2* wb = plane + G::PLANE;
-  double2* alt = wb + G::PLANE;
-  double* dz = reinterpret_cast<double*>(alt + 2 * N);
-  double* dy = dz + N * DLD;
-  double* bbar = dy + N * DLD;
-  const int x0 = blockIdx.x, s = s0 + blockIdx.y;
-  const double* potq = pot + (size_t)(s >= nneut ? 1 : 0) * 12 * N3;
-  const double2* src = psi + (size_t)s * 2 * N3 + (size_t)x0 * N2;
-#pragma unroll 6
-  for (int e = threadIdx.x; e < 2 * N * N; e += kHdThreads) {
-    const int c = e / (N * N), r = e - c * N * N;
-    plane[(c * N + r / N) * G::LD + r % N] = src[(size_t)c * N3 + r];
+  double2* X = reinterpret_cast<double2*>(hd_smem);
+  double2* W = X + G::PLANE;
+  double* dz = reinterpret_cast<double*>(W + G::PLANE);
+  double* dy = dz + G::DSZ;
+  double* bz = dy + G::DSZ;
+  double* by = bz + N;
+  double2* az = reinterpret_cast<double2*>(by + N);
+  double2* ay = az + 2 * N;
+  const HdTile t = hd_tile<N>();
+  const int items = a.ns * N;
+  auto source = [&](int it) { return a.psi + (size_t)(a.s0 + it / N) * 2 * N3 + (size_t)(it % N) * N2; };
+  int it = blockIdx.x;
+  hd_stage<N>(X, source(it), N);
+  for (int e = threadIdx.x; e < G::DSZ; e += G::THREADS) {
+    dz[e] = a.dmat[2 * G::DSZ + e];
+    dy[e] = a.dmat[G::DSZ + e];
   }
-  hd_load_d<N>(dz, dmat + 2 * N2);
-  hd_load_d<N>(dy, dmat + 1 * N2);
-  __syncthreads();
-  double2* dst = acc + (size_t)s * 2 * N3;
-  const size_t base = (size_t)x0 * N2;
-  hd_pass<N, 2, true, true>(
-      plane, wb, dz, alt, bbar, potq, base, N, 1, nq_z, [](size_t) { return 0; },
-      [&](int, int, size_t g, double2 q0, double2 q1, int) {
-        dst[g] = q0;
-        dst[N3 + g] = q1;
-      });
-  hd_pass<N, 1, false, false>(
-      plane, wb, dy, alt, bbar, potq, base, N, 1, nq_y,
-      [&](size_t g) { return HdPre{dst[g], dst[N3 + g], 0.0}; },
-      [&](int, int, size_t g, double2 q0, double2 q1, const HdPre& pv) {
-        dst[g] = pv.m0 + q0;
-        dst[N3 + g] = pv.m1 + q1;
-      });
-}
-
-// B: one y-plane of one state; x lines, then pout = weight * h psi -
-// weightuv * v_pair psi, pout_del = v_pair psi and the plane's overlaps.
-template <int N>
-__global__ void __launch_bounds__(kHdThreads)
-hpsi_dmma_y_kernel(const double* __restrict__ pot, const double2* __restrict__ psi, double2* acc, int s0, int nneut,
-                   const double* __restrict__ dmat, double nq_x, const double* __restrict__ weight,
-                   const double* __restrict__ weightuv, double2* pout, double2* pout_mf, double2* pout_del,
-                   double* ovl) {
-  using G = HdGeo<N>;
-  constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
-  constexpr int DLD = hd_dld<N>();
-  extern __shared__ __align__(16) unsigned char hd_smem[];
-  __shared__ double red[2][kHdWarps];
-  double2* plane = reinterpret_cast<double2*>(hd_smem);
-  double2* wb = plane + G::PLANE;
-  double2* alt = wb + G::PLANE;
-  double* dx = reinterpret_cast<double*>(alt + 2 * N);
-  double* bbar = dx + 2 * N * DLD;
-  const int y0 = blockIdx.x, s = s0 + blockIdx.y;
-  const double* potq = pot + (size_t)(s >= nneut ? 1 : 0) * 12 * N3;
-  const double2* src = psi + (size_t)s * 2 * N3 + (size_t)y0 * N;
-  // plane (a = x, b = z) at fixed y0
-#pragma unroll 6
-  for (int e = threadIdx.x; e < 2 * N * N; e += kHdThreads) {
-    const int c = e / (N * N), r = e - c * N * N;
-    const int a = r / N, b = r % N;
-    plane[(c * N + a) * G::LD + b] = src[(size_t)c * N3 + (size_t)a * N2 + b];
-  }
-  hd_load_d<N>(dx, dmat);
-  __syncthreads();
-  const double wt = weight ? weight[s] : 1.0;
-  const double wu = weightuv ? weightuv[s] : 0.0;
-  const double2* a_s = acc + (size_t)s * 2 * N3;
-  const size_t so = (size_t)s * 2 * N3;
-  double ov_mf = 0.0, ov_po = 0.0;
-  hd_pass<N, 0, false, false>(plane, wb, dx, alt, bbar, potq, (size_t)y0 * N, N2, 1, nq_x,
-                              [&](size_t g) { return HdPre{a_s[g], a_s[N3 + g], potq[2 * N3 + g]}; },
-                              [&](int line, int j, size_t g, double2 q0, double2 q1, const HdPre& pv) {
-                                const double vp = pv.vp;
-#pragma unroll
-                                for (int c = 0; c < 2; ++c) {
-                                  const size_t gi = (size_t)c * N3 + g;
-                                  const double2 mf = (c == 0 ? pv.m0 : pv.m1) + (c == 0 ? q0 : q1);
-                                  const double2 ps = plane[hd_at<N, false>(c, line, j)];
-                                  const double2 dl = vp * ps;
-                                  const double2 po = wt * mf - wu * dl;
-                                  if (pout_mf) pout_mf[so + gi] = mf;
-                                  if (pout) pout[so + gi] = po;
-                                  if (pout_del) pout_del[so + gi] = dl;
-                                  ov_mf += ps.x * mf.x + ps.y * mf.y;
-                                  ov_po += ps.x * po.x + ps.y * po.y;
-                                }
-                              });
-  if (ovl) {
-    // deterministic block reduction: warp shuffles, then thread 0
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      ov_mf += __shfl_xor_sync(0xffffffffu, ov_mf, o);
-      ov_po += __shfl_xor_sync(0xffffffffu, ov_po, o);
+  for (; it < items; it += gridDim.x) {
+    const int s = a.s0 + it / N, x0 = it % N, iq = s >= a.nneut ? 1 : 0;
+    const double* pot = a.pot + (size_t)iq * 12 * N3;
+    {
+      const double* tb = a.bbar ? a.bbar + (size_t)iq * 3 * N2 + (size_t)x0 * N : nullptr;
+      hd_means<N>(bz, tb ? tb + 2 * N2 : nullptr, pot + N3 + (size_t)x0 * N2, N, 1, threadIdx.x);
+      hd_means<N>(by, tb ? tb + N2 : nullptr, pot + N3 + (size_t)x0 * N2, 1, N, (int)threadIdx.x - G::THREADS / 2);
     }
-    const int w = threadIdx.x / 32, l = threadIdx.x % 32;
-    if (l == 0) {
-      red[0][w] = ov_mf;
-      red[1][w] = ov_po;
+    hd_staged();
+    double2 out[2][2][2];
+    hd_first<N, 2, true, true, false>(X, W, dz, az, t, pot, (size_t)x0 * N2, N, 1, out);
+    hd_sync_group<N>();
+    hd_second<N, true>(W, dz, az, bz, a.nq[2], t, out);
+    hd_sync_group<N>();
+    if (t.on) {
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) W[hd_at<N, true>(c, t.l + u, f ? N - 1 - t.j : t.j)] = out[f][u][c];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double a = 0.0, b = 0.0;
-      for (int i = 0; i < kHdWarps; ++i) {
-        a += red[0][i];
-        b += red[1][i];
+    hd_first<N, 1, false, false, true>(X, W, dy, ay, t, pot, (size_t)x0 * N2, 1, N, out);
+    __syncthreads();
+    if (it + (int)gridDim.x < items) hd_stage<N>(X, source(it + gridDim.x), N);
+    hd_second<N, false>(W, dy, ay, by, a.nq[1], t, out);
+    if (t.on) {
+      double2* dst = a.acc + (size_t)s * 2 * N3 + (size_t)x0 * N2 + t.l;
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) dst[c * N3 + (size_t)(f ? N - 1 - t.j : t.j) * N + u] = out[f][u][c];
+    }
+    __syncthreads();   // the means are rewritten
+  }
+}
+
+// Y: a y-plane of a state; x lines, then pout = weight * h psi - weightuv *
+// v_pair psi, pout_del = v_pair psi and the plane's overlaps.
+template <int N>
+__global__ void __launch_bounds__(HdGeo<N>::THREADS, HdGeo<N>::CTAS) hpsi_dmma_y_kernel(const __grid_constant__ HdArgs a) {
+  using G = HdGeo<N>;
+  constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
+  extern __shared__ __align__(16) unsigned char hd_smem[];
+  __shared__ double red[2][G::WARPS];
+  double2* X = reinterpret_cast<double2*>(hd_smem);   // row x, column z
+  double2* W = X + G::PLANE;
+  double* dx = reinterpret_cast<double*>(W + G::PLANE);
+  double* bx = dx + G::DSZ;
+  double2* ax = reinterpret_cast<double2*>(bx + N);
+  const HdTile t = hd_tile<N>();
+  const int items = a.ns * N;
+  auto source = [&](int it) { return a.psi + (size_t)(a.s0 + it / N) * 2 * N3 + (size_t)(it % N) * N; };
+  int it = blockIdx.x;
+  hd_stage<N>(X, source(it), N2);
+  for (int e = threadIdx.x; e < G::DSZ; e += G::THREADS) dx[e] = a.dmat[e];
+  for (; it < items; it += gridDim.x) {
+    const int s = a.s0 + it / N, y0 = it % N, iq = s >= a.nneut ? 1 : 0;
+    const double* pot = a.pot + (size_t)iq * 12 * N3;
+    hd_means<N>(bx, a.bbar ? a.bbar + (size_t)iq * 3 * N2 + (size_t)y0 * N : nullptr, pot + N3 + (size_t)y0 * N, 1, N2,
+                threadIdx.x);
+    hd_staged();
+    double2 out[2][2][2];
+    hd_first<N, 0, false, false, false>(X, W, dx, ax, t, pot, (size_t)y0 * N, 1, N2, out);
+    __syncthreads();
+    if (it + (int)gridDim.x < items) hd_stage<N>(X, source(it + gridDim.x), N2);
+    hd_second<N, false>(W, dx, ax, bx, a.nq[0], t, out);
+    const double wt = a.weight ? a.weight[s] : 1.0, wu = a.weightuv ? a.weightuv[s] : 0.0;
+    double ov_mf = 0.0, ov_po = 0.0;
+    if (t.on) {
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        const size_t g = (size_t)y0 * N + (size_t)(f ? N - 1 - t.j : t.j) * N2 + t.l, gs = (size_t)s * 2 * N3 + g;
+        double2 ps[2][2], pm[2][2];
+        double vp[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          vp[u] = pot[2 * N3 + g + u];
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            ps[u][c] = a.psi[gs + c * N3 + u];   // the plane itself may be gone
+            pm[u][c] = a.acc[gs + c * N3 + u];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const size_t gi = gs + c * N3 + u;
+            const double2 mf = pm[u][c] + out[f][u][c];
+            const double2 dl = vp[u] * ps[u][c];
+            const double2 po = wt * mf - wu * dl;
+            if (a.pout_mf) a.pout_mf[gi] = mf;
+            if (a.pout) a.pout[gi] = po;
+            if (a.pout_del) a.pout_del[gi] = dl;
+            ov_mf += ps[u][c].x * mf.x + ps[u][c].y * mf.y;
+            ov_po += ps[u][c].x * po.x + ps[u][c].y * po.y;
+          }
       }
-      ovl[((size_t)blockIdx.y * N + y0) * 2 + 0] = a;
-      ovl[((size_t)blockIdx.y * N + y0) * 2 + 1] = b;
+    }
+    if (a.ovl) {
+      // fixed order: warp shuffles, then one thread per sum
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        ov_mf += __shfl_xor_sync(0xffffffffu, ov_mf, o);
+        ov_po += __shfl_xor_sync(0xffffffffu, ov_po, o);
+      }
+      if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x / 32] = ov_mf;
+        red[1][threadIdx.x / 32] = ov_po;
+      }
+    }
+    __syncthreads();   // red is complete; the means are rewritten
+    if (a.ovl && threadIdx.x < 2) {
+      double p = 0.0;
+      for (int i = 0; i < G::WARPS; ++i) p += red[threadIdx.x][i];
+      a.ovl[((size_t)(s - a.s0) * N + y0) * 2 + threadIdx.x] = p;
     }
   }
 }
 
+// bbar[iq][axis][line] = mean of B along the line; lines numbered by their two
+// other coordinates in increasing order.
+__global__ void __launch_bounds__(128) hd_bbar_kernel(int n, const double* __restrict__ pot, double* __restrict__ bbar) {
+  const int n2 = n * n, line = blockIdx.x * 128 + threadIdx.x, ax = blockIdx.y, iq = blockIdx.z;
+  if (line >= n2) return;
+  const int u = line / n, v = line % n;
+  const double* b = pot + ((size_t)iq * 12 + 1) * n2 * n + (ax == 0 ? (size_t)line : ax == 1 ? (size_t)u * n2 + v : (size_t)line * n);
+  const size_t st = ax == 0 ? n2 : ax == 1 ? n : 1;
+  double s = 0.0;
+#pragma unroll 8
+  for (int j = 0; j < n; ++j) s += b[j * st];
+  bbar[((size_t)iq * 3 + ax) * n2 + line] = s / n;
+}
+
 template <int N>
-int hpsi_dmma_launch_t(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, const void* psi,
-                       const double* weight, const double* weightuv, void* acc, void* pout, void* pout_mf,
-                       void* pout_del, double* ovl, cudaStream_t st) {
+int hpsi_dmma_launch_t(hfb_ctx_s* c, HdArgs a, cudaStream_t st) {
   using G = HdGeo<N>;
-  if (ns <= 0) return HFB_OK;
-  double nq[3];
-  for (int a = 0; a < 3; ++a) nq[a] = (M_PI / c->d[a]) * (M_PI / c->d[a]) / N;
+  if (a.ns <= 0) return HFB_OK;
+  for (int ax = 0; ax < 3; ++ax) a.nq[ax] = (M_PI / c->d[ax]) * (M_PI / c->d[ax]) / N;
   allow_max_dynamic_smem(hpsi_dmma_x_kernel<N>);
   allow_max_dynamic_smem(hpsi_dmma_y_kernel<N>);
-  const dim3 grid(N, ns);
-  hpsi_dmma_x_kernel<N><<<grid, kHdThreads, G::SMEM, st>>>((const double*)pot, (const double2*)psi, (double2*)acc,
-                                                           s0, nneut, c->hpsi_d64, nq[1], nq[2]);
+  const long items = (long)a.ns * N, places = (long)G::CTAS * c->sms;
+  const unsigned grid = (unsigned)(items < places ? items : places);
+  // a table of the line means (one launch, about 8 us with its gap) pays from
+  // a few planes a CTA on (about 1 us each without it)
+  a.bbar = nullptr;
+  if (items > 8 * places) {
+    double* bbar = (double*)scratch(c, hfb_ctx_s::S_HPT, sizeof(double) * 6 * N * N);
+    if (!bbar) return HFB_ERR_ALLOC;
+    hd_bbar_kernel<<<dim3((N * N + 127) / 128, 3, 2), 128, 0, st>>>(N, a.pot, bbar);
+    HFB_CHECK_LAUNCH();
+    a.bbar = bbar;
+  }
+  hpsi_dmma_x_kernel<N><<<grid, G::THREADS, G::smem(2), st>>>(a);
   HFB_CHECK_LAUNCH();
-  hpsi_dmma_y_kernel<N><<<grid, kHdThreads, G::SMEM, st>>>((const double*)pot, (const double2*)psi, (double2*)acc,
-                                                           s0, nneut, c->hpsi_d64, nq[0], weight, weightuv,
-                                                           (double2*)pout, (double2*)pout_mf, (double2*)pout_del,
-                                                           ovl);
+  hpsi_dmma_y_kernel<N><<<grid, G::THREADS, G::smem(1), st>>>(a);
   HFB_CHECK_LAUNCH();
   return HFB_OK;
 }
 
 }  // namespace
 
-// D of each axis (levels.py:132-189 as a matrix): D[j][l] = -(2 kf / n)
+// Dm and Dp of each axis, rows padded and strided as the kernels read them,
+// from D (levels.py:132-189 as a matrix): D[j][l] = -(2 kf / n)
 // sum_{k=1}^{n/2-1} k sin(2 pi k (j - l) / n), kf = 2 pi / (n d), in double.
 int hpsi_dmma_prepare(hfb_ctx_s* c) {
   c->hpsi_d64 = nullptr;
-  const int n = c->n;
-  if (n % 8 != 0 || n > 48) return HFB_OK;
-  std::vector<double> d((size_t)3 * n * n);
-  for (int ax = 0; ax < 3; ++ax) {
-    const double kf = 2.0 * M_PI / (n * c->d[ax]);
-    for (int j = 0; j < n; ++j)
-      for (int l = 0; l < n; ++l) {
+  return dispatch_n(c->n, [&](auto nn) -> int {
+    constexpr int N = decltype(nn)::value;
+    using G = HdGeo<N>;
+    std::vector<double> d((size_t)3 * G::DSZ, 0.0);
+    for (int ax = 0; ax < 3; ++ax) {
+      const double kf = 2.0 * M_PI / (N * c->d[ax]);
+      auto el = [&](int j, int l) {
         double v = 0.0;
-        for (int k = 1; k < n / 2; ++k) {
-          const int ph = (((k * (j - l)) % n) + n) % n;
-          v += k * sin(2.0 * M_PI * ph / n);
+        for (int k = 1; k < N / 2; ++k) {
+          const int ph = (((k * (j - l)) % N) + N) % N;
+          v += k * sin(2.0 * M_PI * ph / N);
         }
-        d[((size_t)ax * n + j) * n + l] = -2.0 * kf / n * v;
-      }
-  }
-  if (cudaMalloc(&c->hpsi_d64, d.size() * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    c->hpsi_d64 = nullptr;
-    return HFB_ERR_ALLOC;
-  }
-  if (cudaMemcpy(c->hpsi_d64, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
-    return HFB_ERR_CUDA;
-  return HFB_OK;
+        return -2.0 * kf / N * v;
+      };
+      for (int j = 0; j < G::H; ++j)
+        for (int l = 0; l < G::H; ++l) {
+          const double p = el(j, l), q = el(j, N - 1 - l);
+          d[(size_t)ax * G::DSZ + j * G::LDH + l] = 0.5 * (p - q);
+          d[(size_t)ax * G::DSZ + (G::HP + j) * G::LDH + l] = 0.5 * (p + q);
+        }
+    }
+    if (cudaMalloc(&c->hpsi_d64, d.size() * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();
+      c->hpsi_d64 = nullptr;
+      return HFB_ERR_ALLOC;
+    }
+    if (cudaMemcpy(c->hpsi_d64, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+      return HFB_ERR_CUDA;
+    return HFB_OK;
+  });
 }
 
 bool hpsi_dmma_available(hfb_ctx_s* c, int prec) { return prec == HFB_F64 && c->f64_hpsi == 1 && c->hpsi_d64; }
@@ -431,10 +532,16 @@ bool hpsi_dmma_available(hfb_ctx_s* c, int prec) { return prec == HFB_F64 && c->
 int hpsi_dmma_launch(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, const void* psi, const double* weight,
                      const double* weightuv, void* acc, void* pout, void* pout_mf, void* pout_del, double* ovl,
                      cudaStream_t st) {
-  return dispatch_n(c->n, [&](auto nn) -> int {
-    constexpr int N = decltype(nn)::value;
-    return hpsi_dmma_launch_t<N>(c, pot, s0, ns, nneut, psi, weight, weightuv, acc, pout, pout_mf, pout_del, ovl, st);
-  });
+  HdArgs a{};
+  a.pot = (const double*)pot;
+  a.psi = (const double2*)psi;
+  a.acc = (double2*)acc;
+  a.s0 = s0; a.ns = ns; a.nneut = nneut;
+  a.dmat = c->hpsi_d64;
+  a.weight = weight; a.weightuv = weightuv;
+  a.pout = (double2*)pout; a.pout_mf = (double2*)pout_mf; a.pout_del = (double2*)pout_del;
+  a.ovl = ovl;
+  return dispatch_n(c->n, [&](auto nn) -> int { return hpsi_dmma_launch_t<decltype(nn)::value>(c, a, st); });
 }
 
 }  // namespace hfb
