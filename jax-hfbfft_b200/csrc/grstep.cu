@@ -4,11 +4,21 @@
 //
 // The preconditioner is a 3-D FFT, a division by
 //   (max(wg,.1) (E0 + h2ma k^2) + 0.5 max(wguv,.1) vmax) * Ntot
-// and an inverse 3-D FFT.  It runs as three plane kernels:
+// and an inverse 3-D FFT.  It runs as three kernels over planes of one
+// component of a state:
 //   A (x-plane):  v = ps1 - lagrange (or - <h> psi), norms for efluct, z and y
 //                 forward line FFTs;
 //   B (y-plane):  x forward FFT, divide, x inverse FFT (stays in registers);
 //   C (x-plane):  y and z inverse line FFTs, psi -= x0 * result.
+// Bound by the latency of the lines' exchanges: what helps is more of them in
+// flight.  So a plane is in shared memory only between its two line passes
+// (z lines start or end in global memory, rows of it; y lines columns), its
+// rows double as the lines' exchange buffers, and B needs no plane at all:
+// 44 kB a CTA at 48^3 FP64 against 123 kB with both components staged on the
+// way in and out (one CTA per SM).  Pb208 (236 states, 48^3), A + B + C: FP64
+// 1.29 + 0.97 + 1.27 ms before, 0.70 + 0.63 + 0.57 ms here; FP32 0.46 + 0.32 + 0.49 ms
+// before, 0.37 + 0.19 + 0.25 ms here (the bytes alone: 0.51 + 0.26 + 0.38 and
+// half of that).
 #include "hfb_ctx.cuh"
 #include "hpsi.cuh"
 
@@ -19,50 +29,36 @@ struct PlaneGeo {
   static constexpr int P = PencilSplit<R, N>::P;
   static constexpr int M = N / P;
   static constexpr int T = (M + P - 1) / P;
-  static constexpr int LD = N + 4;
-  static constexpr int NB = Pencil<R, N, P>::XB;
   static constexpr int THREADS = ((N * P + 31) / 32) * 32;
   static constexpr int LINES = THREADS / P;
-  static constexpr size_t SMEM = sizeof(cplx<R>) * (size_t)(2 * N * LD + LINES * NB + N);
+  static constexpr int XB = Pencil<R, N, P>::XB;
+  // Row pitch of the plane: a row holds a line's exchange buffer, and the
+  // lanes that share a memory transaction (8 in FP64, 16 in FP32: consecutive
+  // lines of P lanes) fall on distinct banks in column reads and, for P = 8 and
+  // FP32, in the exchange.
+  static constexpr int Q = sizeof(R) == 8 ? 8 : 16, WANT = P == 8 ? 1 : sizeof(R) == 8 && P == 4 ? 2 : 4;
+  static constexpr int NEED = XB > N ? XB : N;
+  static constexpr int LD = NEED + (Q + WANT - NEED % Q) % Q;
+  // 36 warps an SM for A (56 registers): FP64 0.70 ms at 48^3 against 0.81 with
+  // what the compiler takes, equal at 32^3, 15 % slower at 24^3; B and C equal
+  static constexpr int A_CTAS = N >= 32 ? 1152 / THREADS : 1;
+  static constexpr size_t SMEM = sizeof(cplx<R>) * (size_t)(LINES * LD + N);
+  static constexpr size_t SMEM_B = sizeof(cplx<R>) * (size_t)(LINES * XB + N);
 };
 
-// Forward (DIR = -1) or inverse (+1) transform of every line of one staged
-// component ``pl`` ([N][LD]); data stays in natural order in the plane.
-template <class R, int N, bool ROW, int DIR>
-__device__ __forceinline__ void plane_lines(cplx<R>* pl, cplx<R>* xb, const cplx<R>* tw, int line, int p,
-                                            bool active) {
-  using G = PlaneGeo<R, N>;
-  using PC = Pencil<R, N, G::P>;
-  using Z = cplx<R>;
-  constexpr int M = G::M, T = G::T, P = G::P;
-  auto at = [&](int j) -> Z& { return ROW ? pl[line * G::LD + j] : pl[j * G::LD + line]; };
-  Z v[M];
-  Z f[T][P];
-  if (DIR < 0) {
-#pragma unroll
-    for (int m = 0; m < M; ++m) v[m] = at(p + P * m);
-    PC::forward(v, f, xb, tw, p, 0xffffffffu);
-    if (active) {
-#pragma unroll
-      for (int t = 0; t < T; ++t)
-        if (PC::valid(p, t)) {
-#pragma unroll
-          for (int k1 = 0; k1 < P; ++k1) at(PC::freq(p, t, k1)) = f[t][k1];
-        }
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < T; ++t) {
-#pragma unroll
-      for (int k1 = 0; k1 < P; ++k1) f[t][k1] = PC::valid(p, t) ? at(PC::freq(p, t, k1)) : czero<Z>();
-    }
-    PC::inverse(f, v, xb, tw, p, 0xffffffffu);
-    if (active) {
-#pragma unroll
-      for (int m = 0; m < M; ++m) at(p + P * m) = v[m];
-    }
+// A thread's line and place in it; threads past the last line (n = 8) work on
+// line 0 in a buffer of their own and store nothing.
+template <class R, int N>
+struct LinePlace {
+  int raw, p, line;
+  bool active;
+  __device__ __forceinline__ LinePlace() {
+    raw = threadIdx.x / PlaneGeo<R, N>::P;
+    p = threadIdx.x % PlaneGeo<R, N>::P;
+    active = raw < N;
+    line = active ? raw : 0;
   }
-}
+};
 
 template <class R>
 __device__ __forceinline__ void block_sum2(double& a, double& b, double (*red)[32]) {
@@ -82,64 +78,81 @@ __device__ __forceinline__ void block_sum2(double& a, double& b, double (*red)[3
   }
 }
 
-// A: x-plane, build v and transform along z and y.
+// A: x-plane of one component, build v and transform along z and y.
 template <class R, int N>
-__global__ void __launch_bounds__(PlaneGeo<R, N>::THREADS)
-precond_a_kernel(const cplx<R>* __restrict__ src, const cplx<R>* __restrict__ lag, int use_lag,
-                 const cplx<R>* __restrict__ psi, const double* __restrict__ coef, cplx<R>* tmp, double* fluct) {
+__global__ void __launch_bounds__(PlaneGeo<R, N>::THREADS, PlaneGeo<R, N>::A_CTAS)
+precond_a_kernel(const cplx<R>* src, const cplx<R>* __restrict__ lag, int use_lag, const cplx<R>* __restrict__ psi,
+                 const double* __restrict__ coef, cplx<R>* tmp, double* fluct) {
   using G = PlaneGeo<R, N>;
+  using PC = Pencil<R, N, G::P>;
   using Z = cplx<R>;
+  constexpr int M = G::M, T = G::T, P = G::P, LD = G::LD;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[2][32];
   Z* plane = reinterpret_cast<Z*>(smem_raw);
-  Z* xball = plane + 2 * N * G::LD;
-  Z* tw = xball + G::LINES * G::NB;
-  const int x0 = blockIdx.x, s = blockIdx.y;
-  fill_twiddles<R>(tw, N);
-  const size_t off = (size_t)s * 2 * N3 + (size_t)x0 * N2;
-  const R cf = coef ? (R)coef[s] : R(0);
+  Z* tw = plane + G::LINES * LD;
+  const int x0 = blockIdx.x % N, sc = blockIdx.x / N;   // sc = 2 state + component
+  const LinePlace<R, N> l;
+  const size_t off = (size_t)sc * N3 + (size_t)x0 * N2;
+  const R cf = coef ? (R)coef[sc / 2] : R(0);
+  const bool use_ps = psi && (!use_lag || fluct), use_lg = psi && lag && (use_lag || fluct);
   double n1 = 0, n2 = 0;
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    size_t g = off + (size_t)c * N3 + r;
-    Z v = src[g];
+  Z v[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const size_t g = off + (size_t)l.line * N + l.p + P * m;
+    v[m] = src[g];
+    const Z lg = use_lg ? lag[g] : czero<Z>();
+    const Z hp = use_ps ? cf * psi[g] : czero<Z>();
     if (psi) {
-      Z ps = psi[g];
-      Z lg = lag ? lag[g] : czero<Z>();
-      Z hp = cf * ps;
-      v = use_lag ? v - lg : v - hp;
-      if (fluct) {
-        Z e2 = lg - hp;
-        n1 += (double)v.x * v.x + (double)v.y * v.y;
+      v[m] = use_lag ? v[m] - lg : v[m] - hp;
+      if (fluct && l.active) {
+        const Z e2 = lg - hp;
+        n1 += (double)v[m].x * v[m].x + (double)v[m].y * v[m].y;
         n2 += (double)e2.x * e2.x + (double)e2.y * e2.y;
       }
     }
-    plane[(c * N + r / N) * G::LD + r % N] = v;
   }
+  fill_twiddles<R>(tw, N);
+  __syncthreads();
+  Z* row = plane + l.raw * LD;
+  {
+    Z f[T][P];
+    PC::forward(v, f, row, tw, l.p, 0xffffffffu);
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+      if (PC::valid(l.p, t)) {
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) row[PC::freq(l.p, t, k1)] = f[t][k1];
+      }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < M; ++m) v[m] = plane[(l.p + P * m) * LD + l.line];
   if (fluct) {
-    block_sum2<R>(n1, n2, red);
+    block_sum2<R>(n1, n2, red);   // (its barrier also ends the column reads)
     if (threadIdx.x == 0) {
-      fluct[((size_t)s * N + x0) * 2 + 0] = n1;
-      fluct[((size_t)s * N + x0) * 2 + 1] = n2;
+      double* o = fluct + (((size_t)(sc / 2) * 2 + sc % 2) * N + x0) * 2;
+      o[0] = n1;
+      o[1] = n2;
     }
+  } else {
+    __syncthreads();
   }
-  __syncthreads();
-  const int line_raw = threadIdx.x / G::P, p = threadIdx.x % G::P;
-  const bool active = line_raw < N;
-  const int line = active ? line_raw : 0;
-  Z* xb = xball + line_raw * G::NB;
-  for (int c = 0; c < 2; ++c) plane_lines<R, N, true, -1>(plane + c * N * G::LD, xb, tw, line, p, active);
-  __syncthreads();
-  for (int c = 0; c < 2; ++c) plane_lines<R, N, false, -1>(plane + c * N * G::LD, xb, tw, line, p, active);
-  __syncthreads();
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    tmp[off + (size_t)c * N3 + r] = plane[(c * N + r / N) * G::LD + r % N];
-  }
+  Z f[T][P];
+  PC::forward(v, f, row, tw, l.p, 0xffffffffu);
+  if (!l.active) return;
+#pragma unroll
+  for (int t = 0; t < T; ++t)
+    if (PC::valid(l.p, t)) {
+#pragma unroll
+      for (int k1 = 0; k1 < P; ++k1) tmp[off + (size_t)PC::freq(l.p, t, k1) * N + l.line] = f[t][k1];
+    }
 }
 
-// B: y-plane (fixed ky), transform along x, divide, transform back.
+// B: y-plane (fixed ky) of one component, transform along x, divide, transform
+// back; lines are independent.
 template <class R, int N>
 __global__ void __launch_bounds__(PlaneGeo<R, N>::THREADS)
 precond_b_kernel(cplx<R>* tmp, int nneut, const double* __restrict__ wg, const double* __restrict__ wu,
@@ -151,102 +164,87 @@ precond_b_kernel(cplx<R>* tmp, int nneut, const double* __restrict__ wg, const d
   constexpr int M = G::M, T = G::T, P = G::P;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Z* plane = reinterpret_cast<Z*>(smem_raw);
-  Z* xball = plane + 2 * N * G::LD;
-  Z* tw = xball + G::LINES * G::NB;
-  const int y0 = blockIdx.x, s = blockIdx.y;
+  Z* xball = reinterpret_cast<Z*>(smem_raw);
+  Z* tw = xball + G::LINES * G::XB;
+  const int y0 = blockIdx.x % N, sc = blockIdx.x / N, s = sc / 2;
   const int iq = s >= nneut ? 1 : 0;
+  const LinePlace<R, N> l;  // line = kz
+  Z* io = tmp + (size_t)sc * N3 + (size_t)y0 * N + l.line;
+  Z v[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) v[m] = io[(size_t)(l.p + P * m) * N2];
   fill_twiddles<R>(tw, N);
-  const size_t off = (size_t)s * 2 * N3 + (size_t)y0 * N;
-  // compile-time trip count, unrolled: several loads in flight per thread
-#pragma unroll 8
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    int a = r / N, b = r % N;
-    plane[(c * N + a) * G::LD + b] = tmp[off + (size_t)c * N3 + (size_t)a * N2 + b];
-  }
   __syncthreads();
-  const int line_raw = threadIdx.x / P, p = threadIdx.x % P;
-  const bool active = line_raw < N;
-  const int line = active ? line_raw : 0;  // line = kz
-  Z* xb = xball + line_raw * G::NB;
+  Z* xb = xball + l.raw * G::XB;
   const double wgm = fmax(wg ? wg[s] : 1.0, 0.1);
   const double wum = fmax(wu ? wu[s] : 0.0, 0.1);
   const double vm = vmax_dev ? vmax_dev[iq] : vmax_host;
-  const int kyi = signed_k(y0, N), kzi = signed_k(line, N);
+  const int kyi = signed_k(y0, N), kzi = signed_k(l.line, N);
   const double kyz2 = (kyi * kfy) * (kyi * kfy) + (kzi * kfz) * (kzi * kfz);
   const double shift = wgm * e0 + 0.5 * wum * vm;
-  for (int c = 0; c < 2; ++c) {
-    Z* pl = plane + c * N * G::LD;
-    Z v[M];
-    Z f[T][P];
+  Z f[T][P];
+  PC::forward(v, f, xb, tw, l.p, 0xffffffffu);
 #pragma unroll
-    for (int m = 0; m < M; ++m) v[m] = pl[(p + P * m) * G::LD + line];
-    PC::forward(v, f, xb, tw, p, 0xffffffffu);
+  for (int t = 0; t < T; ++t) {
+    if (!PC::valid(l.p, t)) continue;
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-#pragma unroll
-      for (int k1 = 0; k1 < P; ++k1) {
-        int kxi = signed_k(PC::freq(p, t, k1), N);
-        double k2 = (kxi * kfx) * (kxi * kfx) + kyz2;
-        double den = (shift + wgm * h2ma * k2) * (double)N3;
-        f[t][k1] = (R)(1.0 / den) * f[t][k1];
-      }
-    }
-    PC::inverse(f, v, xb, tw, p, 0xffffffffu);
-    if (active) {
-#pragma unroll
-      for (int m = 0; m < M; ++m) pl[(p + P * m) * G::LD + line] = v[m];
+    for (int k1 = 0; k1 < P; ++k1) {
+      int kxi = signed_k(PC::freq(l.p, t, k1), N);
+      double k2 = (kxi * kfx) * (kxi * kfx) + kyz2;
+      double den = (shift + wgm * h2ma * k2) * (double)N3;
+      f[t][k1] = (R)(1.0 / den) * f[t][k1];
     }
   }
-  __syncthreads();
-  // compile-time trip count, unrolled: several loads in flight per thread
-#pragma unroll 8
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    int a = r / N, b = r % N;
-    tmp[off + (size_t)c * N3 + (size_t)a * N2 + b] = plane[(c * N + a) * G::LD + b];
-  }
+  PC::inverse(f, v, xb, tw, l.p, 0xffffffffu);
+  if (!l.active) return;
+#pragma unroll
+  for (int m = 0; m < M; ++m) io[(size_t)(l.p + P * m) * N2] = v[m];
 }
 
-// C: x-plane, inverse along y and z, then write or update.
+// C: x-plane of one component, inverse along y and z, then write or update.
 template <class R, int N>
 __global__ void __launch_bounds__(PlaneGeo<R, N>::THREADS)
 precond_c_kernel(const cplx<R>* tmp, int mode, double x0, const double* x0_dev, cplx<R>* dst) {
   using G = PlaneGeo<R, N>;
+  using PC = Pencil<R, N, G::P>;
   using Z = cplx<R>;
+  constexpr int M = G::M, T = G::T, P = G::P, LD = G::LD;
   constexpr size_t N2 = (size_t)N * N, N3 = N2 * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Z* plane = reinterpret_cast<Z*>(smem_raw);
-  Z* xball = plane + 2 * N * G::LD;
-  Z* tw = xball + G::LINES * G::NB;
-  const int xp = blockIdx.x, s = blockIdx.y;
+  Z* tw = plane + G::LINES * LD;
+  const int xp = blockIdx.x % N, sc = blockIdx.x / N;
+  const LinePlace<R, N> l;
+  const size_t off = (size_t)sc * N3 + (size_t)xp * N2;
+  Z f[T][P], v[M];
+#pragma unroll
+  for (int t = 0; t < T; ++t)
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1)
+      f[t][k1] = PC::valid(l.p, t) ? tmp[off + (size_t)PC::freq(l.p, t, k1) * N + l.line] : czero<Z>();
   fill_twiddles<R>(tw, N);
-  const size_t off = (size_t)s * 2 * N3 + (size_t)xp * N2;
-  // compile-time trip count, unrolled: several loads in flight per thread
-#pragma unroll 8
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    plane[(c * N + r / N) * G::LD + r % N] = tmp[off + (size_t)c * N3 + r];
+  __syncthreads();
+  Z* row = plane + l.raw * LD;
+  PC::inverse(f, v, row, tw, l.p, 0xffffffffu);
+  __syncthreads();
+  if (l.active) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) plane[(l.p + P * m) * LD + l.line] = v[m];
   }
   __syncthreads();
-  const int line_raw = threadIdx.x / G::P, p = threadIdx.x % G::P;
-  const bool active = line_raw < N;
-  const int line = active ? line_raw : 0;
-  Z* xb = xball + line_raw * G::NB;
-  for (int c = 0; c < 2; ++c) plane_lines<R, N, false, +1>(plane + c * N * G::LD, xb, tw, line, p, active);
-  __syncthreads();
-  for (int c = 0; c < 2; ++c) plane_lines<R, N, true, +1>(plane + c * N * G::LD, xb, tw, line, p, active);
-  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < T; ++t)
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) f[t][k1] = PC::valid(l.p, t) ? row[PC::freq(l.p, t, k1)] : czero<Z>();
+  __syncwarp();
+  PC::inverse(f, v, row, tw, l.p, 0xffffffffu);
+  if (!l.active) return;
   const R xr = (R)(x0_dev ? *x0_dev : x0);
-  // compile-time trip count, unrolled: several loads in flight per thread
-#pragma unroll 8
-  for (int e = threadIdx.x; e < 2 * N * N; e += G::THREADS) {
-    int c = e / (N * N), r = e - c * N * N;
-    size_t g = off + (size_t)c * N3 + r;
-    Z v = plane[(c * N + r / N) * G::LD + r % N];
-    if (mode == 0) dst[g] = v;
-    else dst[g] = dst[g] - xr * v;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const size_t g = off + (size_t)l.line * N + l.p + P * m;
+    if (mode == 0) dst[g] = v[m];
+    else dst[g] = dst[g] - xr * v[m];
   }
 }
 
@@ -261,12 +259,12 @@ int precond_launch_t(hfb_ctx_s* c, int ns, int nneut, const void* src, const voi
   allow_max_dynamic_smem(precond_a_kernel<R, N>);
   allow_max_dynamic_smem(precond_b_kernel<R, N>);
   allow_max_dynamic_smem(precond_c_kernel<R, N>);
-  dim3 grid(N, ns);
+  const unsigned grid = 2u * ns * N;
   precond_a_kernel<R, N><<<grid, G::THREADS, G::SMEM, st>>>((const Z*)src, (const Z*)lag, use_lag, (const Z*)psi,
                                                             coef, (Z*)tmp, fluct);
   HFB_CHECK_LAUNCH();
   const double kf[3] = {2.0 * kPi / (c->d[0] * N), 2.0 * kPi / (c->d[1] * N), 2.0 * kPi / (c->d[2] * N)};
-  precond_b_kernel<R, N><<<grid, G::THREADS, G::SMEM, st>>>((Z*)tmp, nneut, wg, wu, vmax_dev, vmax_host, e0, h2ma,
+  precond_b_kernel<R, N><<<grid, G::THREADS, G::SMEM_B, st>>>((Z*)tmp, nneut, wg, wu, vmax_dev, vmax_host, e0, h2ma,
                                                             kf[0], kf[1], kf[2]);
   HFB_CHECK_LAUNCH();
   precond_c_kernel<R, N><<<grid, G::THREADS, G::SMEM, st>>>((const Z*)tmp, mode, x0, x0_dev, (Z*)dst);
@@ -449,7 +447,7 @@ extern "C" int hfb_grstep(hfb_ctx_t ctx, int prec, const hfb_grstep_args* a, voi
   if (ns <= 0) return HFB_OK;
   const size_t n3 = (size_t)n * n * n;
   const int nov = hpsi_ovl_parts(ctx, prec);
-  double* part = (double*)scratch(ctx, hfb_ctx_s::S_PART, sizeof(double) * (size_t)ns * (nov + n) * 2);
+  double* part = (double*)scratch(ctx, hfb_ctx_s::S_PART, sizeof(double) * (size_t)ns * (nov + 2 * n) * 2);
   double* vec = (double*)scratch(ctx, hfb_ctx_s::S_SMALL, sizeof(double) * ((size_t)ns * 6 + 8 + 2 * kVmaxBlocks));
   if (!part || !vec) return HFB_ERR_ALLOC;
   double* ovl = part;
@@ -483,7 +481,7 @@ extern "C" int hfb_grstep(hfb_ctx_t ctx, int prec, const hfb_grstep_args* a, voi
           ns, n3, spe_new, a->sp_energy, a->x0dmp, a->x0dmp_dev, (const float2*)a->hmfpsi, (float2*)a->psi);
     HFB_CHECK_LAUNCH();
   }
-  grstep_finish_kernel<<<1, 1024, 0, st>>>(ns, a->do_fluct && a->e0dmp > 0.0, n, (const double2*)fl, a->wxyz, spe_new, a->wocc,
+  grstep_finish_kernel<<<1, 1024, 0, st>>>(ns, a->do_fluct && a->e0dmp > 0.0, 2 * n, (const double2*)fl, a->wxyz, spe_new, a->wocc,
                                           a->wstates, a->sp_energy, a->sp_efluct1, a->sp_efluct2, a->sums);
   HFB_CHECK_LAUNCH();
   // 3) h psi_new into hmfpsi (and v_pair psi_new into delpsi when requested)

@@ -47,7 +47,7 @@ int hpsi_ovl_parts(hfb_ctx_s* c, int prec);
 //  mode 0: dst = out;  mode 1: dst -= x0 * out   (dst = psi in the gradient step)
 // ``tmp`` holds the intermediate spectrum (may alias src or dst).  ``x0_dev``
 // (optional) is a device double read in place of x0.
-// ``fluct`` (optional) receives per-(state, x-plane) partial sums [ns][n][2]
+// ``fluct`` (optional) receives per-(state, component, x-plane) partial sums [ns][2][n][2]
 // of |v|^2 and |lag - coef psi|^2.  ``wg``, ``wu`` are per-state weights
 // before the max(., 0.1) floor; the pairing shift uses vmax_dev[iq] when
 // given, else vmax_host.
