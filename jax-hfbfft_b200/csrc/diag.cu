@@ -4,7 +4,7 @@
 //  * Gram contractions C_a = wxyz Psi^H X_a (X = psi, hampsi, hmfpsi,
 //    v_pair psi) over K = 2 n^3: one kernel reads each psi tile once for all
 //    requested matrices; split-K partials are summed in a fixed order.
-//  * Hermitian eigensolver: cyclic two-sided Jacobi in one CTA on the packed
+//  * Hermitian eigensolver: cyclic two-sided Jacobi in one CTA on the folded
 //    lower triangle held in shared memory (round-robin ordering, n/2 disjoint
 //    rotations per round); the rotations are recorded and replayed onto the
 //    eigenvector matrix by a row-parallel kernel.  Eigenvalues ascending.
@@ -213,34 +213,56 @@ int gram_launch(hfb_ctx_s* c, int prec, int nblk, const int* s0, const int* ns, 
 }
 
 // ============================================================== Jacobi ====
-// Packed lower triangle: element (k, l), k >= l, at k (k + 1) / 2 + l.
-__device__ __forceinline__ int pk(int k, int l) { return k * (k + 1) / 2 + l; }
-__device__ __forceinline__ double2 ld_h(const double2* a, int k, int l) {
-  if (k >= l) return a[pk(k, l)];
-  double2 v = a[pk(l, k)];
-  return make_double2(v.x, -v.y);
-}
-__device__ __forceinline__ void st_h(double2* a, int k, int l, double2 v) {
-  if (k >= l) a[pk(k, l)] = v;
-  else a[pk(l, k)] = make_double2(v.x, -v.y);
+// The strict lower triangle of a Hermitian matrix of even size m folded into
+// m - 1 rows of h = m / 2: columns l < h below one another, the rest of the
+// triangle transposed into the corner that they leave free.  Walks along rows
+// and along columns are contiguous or ``ld`` apart (odd where it fits), so the
+// lanes of a warp fall on distinct banks; packed row by row, column walks
+// collided.
+struct Folded {
+  double2* p;
+  int h, ld;
+  __device__ __forceinline__ double2& at(int k, int l) const {   // k > l
+    return l < h ? p[(k - 1) * ld + l] : p[(l - h) * ld + k - h];
+  }
+  __device__ __forceinline__ double2 get(int k, int l) const {
+    if (k > l) return at(k, l);
+    const double2 v = at(l, k);
+    return make_double2(v.x, -v.y);
+  }
+  __device__ __forceinline__ void set(int k, int l, double2 v) const {
+    if (k > l) at(k, l) = v;
+    else at(l, k) = make_double2(v.x, -v.y);
+  }
+};
+// Row and column of entry e of a packed lower triangle with its diagonal.
+__device__ __forceinline__ void unpack_lower(int e, int& k, int& l) {
+  k = (int)((sqrt(8.0 * e + 1.0) - 1.0) / 2.0);
+  while (k * (k + 1) / 2 > e) --k;
+  while ((k + 1) * (k + 2) / 2 <= e) ++k;
+  l = e - k * (k + 1) / 2;
 }
 
-// Round-robin tournament: round r of m-1 (m even), pair index q < m/2.
+// Round-robin tournament: round r < m - 1 (m even), pair index q < m / 2.
 __device__ __forceinline__ void rr_pair(int m, int r, int q, int& a, int& b) {
-  if (q == 0) { a = r % (m - 1); b = m - 1; }
-  else { a = (r + q) % (m - 1); b = (r + m - 1 - q) % (m - 1); }
+  a = r + q;
+  b = q == 0 ? m - 1 : r + m - 1 - q;
+  if (a >= m - 1) a -= m - 1;
+  if (q != 0 && b >= m - 1) b -= m - 1;
   if (a > b) { int t = a; a = b; b = t; }
 }
 
 struct JacRot {
-  double cs, sn;
-  double2 om;   // exp(-i phi)
+  double cs, sn;   // sn == 0: the identity
+  double2 om;      // exp(-i phi)
 };
 
 constexpr int kJacMaxSweeps = 40;
 constexpr int kEighMax = 4;     // matrices per batched launch
-constexpr int kJacThreads = 1024;
-constexpr int kJacBlk = 4;      // 2x2 blocks per thread (half*(half+1)/2 <= 4096 -> n <= 180)
+constexpr int kJacThreads = 1024, kJacSmall = 512;
+constexpr int kJacBlk = 4;      // 2x2 blocks per thread: 84 * 85 / 2 over 928 threads
+constexpr int kJacMaxN = 168;   // what shared memory holds
+constexpr int kJacAhead = 32;   // pairs from which a round's rotations are computed in the round before
 
 // One batched solve: up to kEighMax independent matrices, one CTA each.
 struct EighBatch {
@@ -257,12 +279,23 @@ struct EighBatch {
   const int* gate;             // optional device flags [nb]: matrix b is solved only when gate[b] != 0
 };
 
-// One CTA per matrix: cyclic two-sided Jacobi on the packed lower triangle.
-// Each round applies n/2 disjoint rotations (round-robin pairing); thread t
-// owns fixed 2x2 blocks (pair q1 rows x pair q2 columns, q1 >= q2) for the
-// whole solve, and skips a block when both of its rotations are the
-// identity.  Rotations are recorded for the eigenvector replay.
-__global__ void __launch_bounds__(kJacThreads)
+// One CTA per matrix: cyclic two-sided Jacobi on the folded lower triangle and
+// the diagonal.  Each round applies n/2 disjoint rotations (round-robin
+// pairing) as updates of the 2x2 blocks (pair q1 rows x pair q2 columns, q1 >
+// q2), and skips a block when both of its rotations are the identity.  A
+// round's own latency is its rotations (hypot, roots and quotients one after
+// the other, for one pair per thread), so from kJacAhead pairs on the first
+// warps compute the next round's behind the update: the elements that pair up next lie in blocks
+// (1, 0), (q + 1, q - 1) and (half - 1, half - 2), which these warps update
+// first.  With fewer pairs the update is as short as that part of it.  The
+// other threads own fixed blocks for the whole solve.  Rotations are recorded for
+// the eigenvector replay.  Lambda of Pb208 (140 + 96 states): 2.46 ms with
+// the rotations between two block barriers, 1.88 ms here (single-precision
+// threshold 1.51, 1.20).
+// TH: the block's largest size (up to kJacSmall threads the loop keeps out of
+// local memory: 32 + 32 states 150 us against 172).
+template <int TH>
+__global__ void __launch_bounds__(TH)
 jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t rot_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int b = blockIdx.x;
@@ -270,11 +303,11 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
   const int n = eb.n[b], lda = eb.lda[b];
   const int m = n + (n & 1);   // pad odd sizes with a decoupled index
   const int half = m / 2;
-  double2* a = reinterpret_cast<double2*>(smem_raw);
-  JacRot* rr = reinterpret_cast<JacRot*>(a + (size_t)m * (m + 1) / 2);
-  int* rp = reinterpret_cast<int*>(rr + half);
-  int* rq = rp + half;
-  int* act = rq + half;
+  const Folded a{reinterpret_cast<double2*>(smem_raw), half, m == kJacMaxN ? half : half | 1};
+  double2* rcs = a.p + (size_t)(m - 1) * a.ld;                 // (cs, sn) [2][half], by the round's parity
+  double2* rom = rcs + 2 * half;                               // om
+  double* dg = reinterpret_cast<double*>(rom + 2 * half);      // diagonal
+  const bool ahead = half >= kJacAhead;
   __shared__ int any_rot;
   __shared__ int round_rot[2];   // a rotation in round r (parity r & 1)
   const double2* Ab = eb.a[b];
@@ -282,28 +315,24 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
   // the lower triangle (eigh with symmetrize_input=False reads only it; the
   // diagonal's imaginary part is ignored as by LAPACK heevd)
   for (int e = threadIdx.x; e < m * (m + 1) / 2; e += blockDim.x) {
-    int k = (int)((sqrt(8.0 * e + 1.0) - 1.0) / 2.0);
-    while (k * (k + 1) / 2 > e) --k;
-    while ((k + 1) * (k + 2) / 2 <= e) ++k;
-    const int l = e - k * (k + 1) / 2;
-    double2 v = make_double2(0.0, 0.0);
-    if (k < n && l < n) v = Ab[(size_t)k * lda + l];
-    if (k == l) v.y = 0.0;
-    a[e] = v;
+    int k, l;
+    unpack_lower(e, k, l);
+    const double2 v = k < n && l < n ? Ab[(size_t)k * lda + l] : make_double2(0.0, 0.0);
+    if (k == l) dg[k] = v.x;
+    else a.at(k, l) = v;
   }
   // Frobenius norm (invariant under the rotations): an off-diagonal element
   // below eps ||A||_F is at the rounding-noise level the rotations
   // themselves create, so it is not rotated (the eigenvalue error this
-  // leaves is second order in it)
-  __shared__ double red_f[32];
+  // leaves is second order in it).  Summed as by kJacThreads threads whatever
+  // the block's size.
+  __shared__ double red_f[kJacThreads / 32];
   __shared__ double tol_abs;
-  {
+  for (int w = threadIdx.x / 32; w < kJacThreads / 32; w += blockDim.x / 32) {
     double f2 = 0.0;
-    for (int e = threadIdx.x; e < m * (m + 1) / 2; e += blockDim.x) {
-      int k = (int)((sqrt(8.0 * e + 1.0) - 1.0) / 2.0);
-      while (k * (k + 1) / 2 > e) --k;
-      while ((k + 1) * (k + 2) / 2 <= e) ++k;
-      const int l = e - k * (k + 1) / 2;
+    for (int e = 32 * w + threadIdx.x % 32; e < m * (m + 1) / 2; e += kJacThreads) {
+      int k, l;
+      unpack_lower(e, k, l);
       double v = 0.0;
       if (k < n && l < n) {
         const double2 x = Ab[(size_t)k * lda + l];
@@ -313,32 +342,107 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) f2 += __shfl_xor_sync(0xffffffffu, f2, o);
-    if ((threadIdx.x & 31) == 0) red_f[threadIdx.x / 32] = f2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x / 32); ++w) t += red_f[w];
-      tol_abs = (eb.tol_rel > 0.0 ? eb.tol_rel : 2.220446049250313e-16) * sqrt(t);
-    }
+    if ((threadIdx.x & 31) == 0) red_f[w] = f2;
   }
-  // this thread's blocks (round independent)
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int w = 0; w < kJacThreads / 32; ++w) t += red_f[w];
+    tol_abs = (eb.tol_rel > 0.0 ? eb.tol_rel : 2.220446049250313e-16) * sqrt(t);
+  }
+  const int rotators = (half + 31) / 32 * 32;   // threads of the rotating warps
+  // the other threads' blocks (round independent)
   const int nblk = half * (half + 1) / 2;
-  int bq1[kJacBlk], bq2[kJacBlk];
+  int blk[kJacBlk];   // q1 << 8 | q2, or -1
 #pragma unroll
   for (int j = 0; j < kJacBlk; ++j) {
-    const int e = threadIdx.x + j * kJacThreads;
-    bq1[j] = bq2[j] = -1;
-    if (e < nblk) {
-      int q1 = (int)((sqrt(8.0 * e + 1.0) - 1.0) / 2.0);
-      while (q1 * (q1 + 1) / 2 > e) --q1;
-      while ((q1 + 1) * (q1 + 2) / 2 <= e) ++q1;
-      bq1[j] = q1;
-      bq2[j] = e - q1 * (q1 + 1) / 2;
+    const int e = (int)threadIdx.x - rotators + j * ((int)blockDim.x - rotators);
+    blk[j] = -1;
+    if ((int)threadIdx.x >= rotators && e < nblk) {
+      int q1, q2;
+      unpack_lower(e, q1, q2);
+      const bool next = q1 - q2 == 2 || (q1 == 1 && q2 == 0) || (q1 == half - 1 && q2 == half - 2);
+      if (q1 != q2 && !(ahead && next)) blk[j] = q1 << 8 | q2;
     }
   }
   __syncthreads();
   int rounds = 0;
   int sweep = 0;
+  auto negligible = [&](double app, double aqq, double mag) {
+    // off-diagonal element at the noise level or negligible beside both
+    // diagonal entries
+    return mag <= tol_abs || (fabs(app) + 100.0 * mag == fabs(app) && fabs(aqq) + 100.0 * mag == fabs(aqq));
+  };
+  // rotation of pair q of round r, number ``at`` of the record; what it does to
+  // the pair itself follows in diagonal(), beside the update of other blocks
+  struct { double cs, sn, app, aqq, mag; } mine;
+  auto rotation = [&](int r, int q, int at) {
+    int p_, q_;
+    rr_pair(m, r, q, p_, q_);
+    JacRot g;
+    g.cs = 1.0; g.sn = 0.0; g.om = make_double2(1.0, 0.0);
+    const double app = dg[p_], aqq = dg[q_];
+    const double2 apq = a.get(p_, q_);
+    const double mag = hypot(apq.x, apq.y);
+    if (!negligible(app, aqq, mag)) {
+      const double theta = (aqq - app) / (2.0 * mag);
+      double t = 1.0 / (fabs(theta) + sqrt(theta * theta + 1.0));
+      if (theta < 0.0) t = -t;
+      g.cs = 1.0 / sqrt(t * t + 1.0);
+      g.sn = t * g.cs;
+      g.om = make_double2(apq.x / mag, -apq.y / mag);
+      any_rot = 1;
+      round_rot[r & 1] = 1;
+    }
+    mine.cs = g.cs; mine.sn = g.sn; mine.app = app; mine.aqq = aqq; mine.mag = mag;
+    rcs[(r & 1) * half + q] = make_double2(g.cs, g.sn);
+    rom[(r & 1) * half + q] = g.om;
+    rotb[(size_t)at * half + q] = g;
+  };
+  auto diagonal = [&](int r, int q) {
+    if (mine.sn == 0.0) return;
+    int p_, q_;
+    rr_pair(m, r, q, p_, q_);
+    const double u = mine.sn / mine.cs;
+    dg[p_] = mine.app - u * mine.mag;
+    dg[q_] = mine.aqq + u * mine.mag;
+    a.set(q_, p_, make_double2(0.0, 0.0));
+  };
+  // block (q1, q2) under the rotations of round r
+  auto update = [&](int r, int q1, int q2) {
+    const int o = (r & 1) * half;
+    const double2 s1 = rcs[o + q1], s2 = rcs[o + q2];
+    const bool a1 = s1.y != 0.0, a2 = s2.y != 0.0;
+    if (!a1 && !a2) return;
+    int k0, k1, l0, l1;
+    rr_pair(m, r, q1, k0, k1);
+    rr_pair(m, r, q2, l0, l1);
+    // G = [[cs, sn], [-sn om, cs om]] (rows: old index, cols: new index)
+    const JacRot g1{s1.x, s1.y, rom[o + q1]}, g2{s2.x, s2.y, rom[o + q2]};
+    double2 B00 = a.get(k0, l0), B01 = a.get(k0, l1), B10 = a.get(k1, l0), B11 = a.get(k1, l1);
+    auto cm = [](double2 x, double2 y) { return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x); };
+    if (a2) {   // right multiply by G2 (columns l0, l1)
+      const double2 t10 = cm(B01, g2.om), t11 = cm(B11, g2.om);
+      const double2 c00 = make_double2(g2.cs * B00.x - g2.sn * t10.x, g2.cs * B00.y - g2.sn * t10.y);
+      const double2 c01 = make_double2(g2.sn * B00.x + g2.cs * t10.x, g2.sn * B00.y + g2.cs * t10.y);
+      const double2 c10 = make_double2(g2.cs * B10.x - g2.sn * t11.x, g2.cs * B10.y - g2.sn * t11.y);
+      const double2 c11 = make_double2(g2.sn * B10.x + g2.cs * t11.x, g2.sn * B10.y + g2.cs * t11.y);
+      B00 = c00; B01 = c01; B10 = c10; B11 = c11;
+    }
+    if (a1) {   // left multiply by G1^H = [[cs, -sn conj(om)], [sn, cs conj(om)]] (rows k0, k1)
+      const double2 oc = make_double2(g1.om.x, -g1.om.y);
+      const double2 u0 = cm(B10, oc), u1 = cm(B11, oc);
+      const double2 d00 = make_double2(g1.cs * B00.x - g1.sn * u0.x, g1.cs * B00.y - g1.sn * u0.y);
+      const double2 d01 = make_double2(g1.cs * B01.x - g1.sn * u1.x, g1.cs * B01.y - g1.sn * u1.y);
+      const double2 d10 = make_double2(g1.sn * B00.x + g1.cs * u0.x, g1.sn * B00.y + g1.cs * u0.y);
+      const double2 d11 = make_double2(g1.sn * B01.x + g1.cs * u1.x, g1.sn * B01.y + g1.cs * u1.y);
+      B00 = d00; B01 = d01; B10 = d10; B11 = d11;
+    }
+    a.set(k0, l0, B00);
+    a.set(k0, l1, B01);
+    a.set(k1, l0, B10);
+    a.set(k1, l1, B11);
+  };
   for (; sweep < kJacMaxSweeps; ++sweep) {
     if (threadIdx.x == 0) any_rot = 0;
     __syncthreads();
@@ -348,115 +452,62 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
     {
       int need = 0;
       for (int e = threadIdx.x; e < m * (m - 1) / 2 && !need; e += blockDim.x) {
-        int k = (int)((sqrt(8.0 * e + 1.0) - 1.0) / 2.0);
-        while (k * (k + 1) / 2 > e) --k;
-        while ((k + 1) * (k + 2) / 2 <= e) ++k;
-        const int p_ = k + 1, q_ = e - k * (k + 1) / 2;   // p_ > q_
-        const double app = a[pk(p_, p_)].x, aqq = a[pk(q_, q_)].x;
-        const double2 apq = ld_h(a, p_, q_);
-        const double mag = hypot(apq.x, apq.y);
-        const bool negl = (mag <= tol_abs) ||
-                          (fabs(app) + 100.0 * mag == fabs(app) && fabs(aqq) + 100.0 * mag == fabs(aqq));
-        if (!negl) need = 1;
+        int p_, q_;
+        unpack_lower(e, p_, q_);
+        ++p_;   // p_ > q_
+        const double2 apq = a.at(p_, q_);
+        if (!negligible(dg[p_], dg[q_], hypot(apq.x, apq.y))) need = 1;
       }
       if (need) any_rot = 1;
       __syncthreads();
       const int go = any_rot;
       __syncthreads();
       if (!go) break;
-      if (threadIdx.x == 0) any_rot = 0;
-      __syncthreads();
     }
-    if (threadIdx.x == 0) round_rot[0] = round_rot[1] = 0;
+    if (threadIdx.x == 0) any_rot = round_rot[0] = 0;
     __syncthreads();
-    for (int r = 0; r < m - 1; ++r) {
-      // the next round's flag is cleared here; no thread reads it before
-      // this round's barrier
-      if (threadIdx.x == 0) round_rot[(r + 1) & 1] = 0;
-      for (int q = threadIdx.x; q < half; q += blockDim.x) {
-        int p_, q_;
-        rr_pair(m, r, q, p_, q_);
-        JacRot g;
-        g.cs = 1.0; g.sn = 0.0; g.om = make_double2(1.0, 0.0);
-        const double app = a[pk(p_, p_)].x, aqq = a[pk(q_, q_)].x;
-        const double2 apq = ld_h(a, p_, q_);
-        const double mag = hypot(apq.x, apq.y);
-        // negligible off-diagonal element relative to both diagonal entries
-        const bool negl = (mag <= tol_abs) ||
-                          (fabs(app) + 100.0 * mag == fabs(app) && fabs(aqq) + 100.0 * mag == fabs(aqq));
-        int on = 0;
-        if (!negl) {
-          const double theta = (aqq - app) / (2.0 * mag);
-          double t = 1.0 / (fabs(theta) + sqrt(theta * theta + 1.0));
-          if (theta < 0.0) t = -t;
-          g.cs = 1.0 / sqrt(t * t + 1.0);
-          g.sn = t * g.cs;
-          g.om = make_double2(apq.x / mag, -apq.y / mag);
-          on = 1;
-          any_rot = 1;
-          round_rot[r & 1] = 1;
-        }
-        rr[q] = g;
-        rp[q] = p_;
-        rq[q] = q_;
-        act[q] = on;
-        rotb[(size_t)rounds * half + q] = g;
-      }
-      __syncthreads();
-      // a round without rotations leaves the matrix as it is: no update
-      // pass and no second barrier (the next round's first writes to the
-      // rotation arrays come after every thread has passed this test)
-      if (!round_rot[r & 1]) {
-        ++rounds;
-        continue;
-      }
+    if (!ahead) {
+      for (int r = 0; r < m - 1; ++r, ++rounds) {
+        const int q = threadIdx.x;
+        // the next round's flag is cleared here; no thread reads it before
+        // this round's barrier
+        if (q == 0) round_rot[(r + 1) & 1] = 0;
+        if (q < half) rotation(r, q, rounds);
+        __syncthreads();
+        // a round without rotations leaves the matrix as it is: no update
+        // pass and no second barrier
+        if (!round_rot[r & 1]) continue;
+        if (q < half) diagonal(r, q);
 #pragma unroll
-      for (int j = 0; j < kJacBlk; ++j) {
-        const int q1 = bq1[j], q2 = bq2[j];
-        if (q1 < 0) continue;
-        const int a1 = act[q1], a2 = act[q2];
-        if (!a1 && !a2) continue;
-        const int k0 = rp[q1], k1 = rq[q1];
-        const JacRot g1 = rr[q1];
-        if (q1 == q2) {
-          const double app = a[pk(k0, k0)].x, aqq = a[pk(k1, k1)].x;
-          const double2 apq = ld_h(a, k0, k1);
-          const double mag = hypot(apq.x, apq.y);
-          const double t = g1.sn / g1.cs;
-          a[pk(k0, k0)] = make_double2(app - t * mag, 0.0);
-          a[pk(k1, k1)] = make_double2(aqq + t * mag, 0.0);
-          st_h(a, k1, k0, make_double2(0.0, 0.0));
-          continue;
+        for (int j = 0; j < kJacBlk; ++j)
+          if (blk[j] >= 0) update(r, blk[j] >> 8, blk[j] & 255);
+        __syncthreads();
+      }
+      const int cont = any_rot;
+      __syncthreads();
+      if (!cont) break;
+      continue;
+    }
+    if ((int)threadIdx.x < half) rotation(0, threadIdx.x, rounds);
+    __syncthreads();
+    for (int r = 0; r < m - 1; ++r, ++rounds) {
+      // a round without rotations leaves the matrix as it is
+      const int on = round_rot[r & 1];
+      if ((int)threadIdx.x < rotators) {
+        const int q = threadIdx.x;
+        if (q == 0) round_rot[(r + 1) & 1] = 0;   // all have read the last round's
+        if (on && q < half) {
+          diagonal(r, q);
+          update(r, q == half - 1 ? q : q + 1, q == 0 ? 0 : q - 1);
         }
-        const int l0 = rp[q2], l1 = rq[q2];
-        const JacRot g2 = rr[q2];
-        // G = [[cs, sn], [-sn om, cs om]] (rows: old index, cols: new index)
-        double2 B00 = ld_h(a, k0, l0), B01 = ld_h(a, k0, l1), B10 = ld_h(a, k1, l0), B11 = ld_h(a, k1, l1);
-        auto cm = [](double2 x, double2 y) { return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x); };
-        if (a2) {   // right multiply by G2 (columns l0, l1)
-          const double2 t10 = cm(B01, g2.om), t11 = cm(B11, g2.om);
-          const double2 c00 = make_double2(g2.cs * B00.x - g2.sn * t10.x, g2.cs * B00.y - g2.sn * t10.y);
-          const double2 c01 = make_double2(g2.sn * B00.x + g2.cs * t10.x, g2.sn * B00.y + g2.cs * t10.y);
-          const double2 c10 = make_double2(g2.cs * B10.x - g2.sn * t11.x, g2.cs * B10.y - g2.sn * t11.y);
-          const double2 c11 = make_double2(g2.sn * B10.x + g2.cs * t11.x, g2.sn * B10.y + g2.cs * t11.y);
-          B00 = c00; B01 = c01; B10 = c10; B11 = c11;
-        }
-        if (a1) {   // left multiply by G1^H = [[cs, -sn conj(om)], [sn, cs conj(om)]] (rows k0, k1)
-          const double2 oc = make_double2(g1.om.x, -g1.om.y);
-          const double2 u0 = cm(B10, oc), u1 = cm(B11, oc);
-          const double2 d00 = make_double2(g1.cs * B00.x - g1.sn * u0.x, g1.cs * B00.y - g1.sn * u0.y);
-          const double2 d01 = make_double2(g1.cs * B01.x - g1.sn * u1.x, g1.cs * B01.y - g1.sn * u1.y);
-          const double2 d10 = make_double2(g1.sn * B00.x + g1.cs * u0.x, g1.sn * B00.y + g1.cs * u0.y);
-          const double2 d11 = make_double2(g1.sn * B01.x + g1.cs * u1.x, g1.sn * B01.y + g1.cs * u1.y);
-          B00 = d00; B01 = d01; B10 = d10; B11 = d11;
-        }
-        st_h(a, k0, l0, B00);
-        st_h(a, k0, l1, B01);
-        st_h(a, k1, l0, B10);
-        st_h(a, k1, l1, B11);
+        asm volatile("bar.sync 1, %0;" ::"r"(rotators) : "memory");
+        if (q < half && r + 1 < m - 1) rotation(r + 1, q, rounds + 1);
+      } else if (on) {
+#pragma unroll
+        for (int j = 0; j < kJacBlk; ++j)
+          if (blk[j] >= 0) update(r, blk[j] >> 8, blk[j] & 255);
       }
       __syncthreads();
-      ++rounds;
     }
     const int cont = any_rot;
     __syncthreads();
@@ -468,7 +519,7 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
     if (sweep >= kJacMaxSweeps) latch_error(status, HFB_ERR_NO_CONVERGENCE);
   }
   double* wb = eb.w[b];
-  for (int k = threadIdx.x; k < n; k += blockDim.x) wb[k] = a[pk(k, k)].x;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) wb[k] = dg[k];
 }
 
 // Replay V = I G_1 G_2 ... onto blocks of kVecRows rows, then order the
@@ -476,7 +527,7 @@ jacobi_kernel(EighBatch eb, JacRot* rot, int* nrounds_out, int* status, size_t r
 // are streamed through shared memory kVecChunk rounds at a time with
 // cp.async double buffering, so each round costs one block barrier instead
 // of one global-memory latency.
-constexpr int kVecRows = 8;
+constexpr int kVecRows = 2;   // Pb208 (236 states): 8 rows 0.46 ms, 4 0.33 ms, 2 0.22 ms
 constexpr int kVecChunk = 8;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -590,16 +641,20 @@ int eigh_batch(hfb_ctx_s* c, EighBatch eb, cudaStream_t st) {
     eb.vblk0[i + 1] = eb.vblk0[i] + (eb.n[i] + kVecRows - 1) / kVecRows;
   }
   const int half = mmax / 2;
-  if (half * (half + 1) / 2 > kJacBlk * kJacThreads) return HFB_ERR_ARG;
-  const size_t smem = sizeof(double2) * (size_t)mmax * (mmax + 1) / 2 + (sizeof(JacRot) + 3 * sizeof(int)) * half;
-  if (smem > 227 * 1024) return HFB_ERR_ARG;
+  if (mmax > kJacMaxN) return HFB_ERR_ARG;
+  const size_t smem = sizeof(double2) * (size_t)(mmax - 1) * (mmax == kJacMaxN ? half : half | 1) +
+                      sizeof(JacRot) * 2 * half + sizeof(double) * mmax;
+  // a thread per block of the largest matrix beside the rotating warps
+  const int want = (half + 31) / 32 * 32 + (half * (half + 1) / 2 + 31) / 32 * 32;
+  const int threads = want < kJacThreads ? want : kJacThreads;
   const size_t rot_stride = (size_t)kJacMaxSweeps * (mmax - 1) * half;
   char* buf = (char*)scratch(c, hfb_ctx_s::S_MAT, sizeof(JacRot) * rot_stride * eb.nb + sizeof(int) * kEighMax + 64);
   if (!buf) return HFB_ERR_ALLOC;
   JacRot* rot = (JacRot*)buf;
   int* nr = (int*)(buf + sizeof(JacRot) * rot_stride * eb.nb);
-  allow_max_dynamic_smem(jacobi_kernel);
-  jacobi_kernel<<<eb.nb, kJacThreads, smem, st>>>(eb, rot, nr, c->dev_status, rot_stride);
+  const auto kernel = threads <= kJacSmall ? jacobi_kernel<kJacSmall> : jacobi_kernel<kJacThreads>;
+  allow_max_dynamic_smem(kernel);
+  kernel<<<eb.nb, threads, smem, st>>>(eb, rot, nr, c->dev_status, rot_stride);
   HFB_CHECK_LAUNCH();
   eb.stage_half = half;
   const size_t smem2 =
