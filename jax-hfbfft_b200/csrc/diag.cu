@@ -732,13 +732,14 @@ int zgemm_small_one(int n, int ld, int ta, int tb, const double2* A, const doubl
 // eigenvectors in the columns of V + b sV, by refinement (diag_cluster.cu);
 // Jacobi for the matrices it does not apply to.
 static int eigh_refine(hfb_ctx_s* c, int nb, Pair2 nper, int ld, const double2* A, size_t sA, double* W, size_t sW,
-                       double2* V, size_t sV, double tol_rel, cudaStream_t st) {
+                       double2* V, size_t sV, double tol_rel, cudaStream_t st,
+                       cudaEvent_t begun = nullptr) {
   const size_t wb = (refine_bytes(nb, ld) + 15) / 16 * 16;
   char* buf = (char*)scratch(c, hfb_ctx_s::S_EIG, wb + sizeof(int) * nb);
   if (!buf) return HFB_ERR_ALLOC;
   int* fallback = (int*)(buf + wb);
   const RefineArgs a{nper, ld, A, sA, W, sW, V, sV, tol_rel > 0.0 ? tol_rel : 1e-13, fallback};
-  const int r = refine_launch(nb, a, buf, st);
+  const int r = refine_launch(nb, a, buf, begun, st);
   if (r) return r;
   EighBatch eb{};
   eb.tol_rel = tol_rel;
@@ -1050,6 +1051,7 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
   if (a->construct && a->ipair) mask |= 8;
   const bool beside = a->diagonalize && ctx->side && ctx->side2;
   const bool split = beside && a->construct && ctx->gram_split;
+  const bool refine = a->diagonalize && ctx->lambda_refine && prec == HFB_F64;
   const double* vp[2] = {a->v_pair, a->v_pair ? a->v_pair + n3 : nullptr};
   double2* outs[8];
   for (int iq = 0; iq < 2; ++iq)
@@ -1064,7 +1066,7 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
   if (beside) {
     cudaEventRecord(ctx->ev_fork, st);
     cudaStreamWaitEvent(ctx->side2, ctx->ev_fork, 0);
-    if (split) cudaEventRecord(ctx->ev_fork2, ctx->side2);
+    if (split && !refine) cudaEventRecord(ctx->ev_fork2, ctx->side2);
     nst = ctx->side2;
   }
   r = loewdin_launch(LoewdinArgs{nper, off, ld, gm, 4 * sm, Ur, a->sp_norm, ctx->dev_status}, work, !split, nst);
@@ -1078,8 +1080,8 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
     // converges in a few sweeps and measured faster (11.4 ms against 12.0
     // ms per Pb208 iteration: in the bulk the refinement's acceptance test
     // fails and the Jacobi runs after it)
-    if (ctx->lambda_refine && prec == HFB_F64) {
-      r = eigh_refine(ctx, 2, nper, ld, gm + sm, 4 * sm, w, ld, Vl, sm, tol_rel, st);
+    if (refine) {
+      r = eigh_refine(ctx, 2, nper, ld, gm + sm, 4 * sm, w, ld, Vl, sm, tol_rel, st, split ? ctx->ev_fork2 : nullptr);
     } else {
       EighBatch eb{};
       eb.tol_rel = tol_rel;

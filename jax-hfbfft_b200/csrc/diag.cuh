@@ -40,7 +40,7 @@ struct RefineArgs {
   int* fallback;      // [nb]: set when the refinement does not apply to matrix b
 };
 size_t refine_bytes(int nb, int ld);
-int refine_launch(int nb, const RefineArgs& a, void* work, cudaStream_t st);
+int refine_launch(int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st);   // begun: every CTA runs (or null)
 
 struct LoewdinArgs {
   Pair2 nper, off;

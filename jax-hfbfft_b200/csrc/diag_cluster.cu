@@ -744,18 +744,25 @@ int cluster_size(int n, int most = 8) {
   return c;
 }
 
+// ``begun`` (optional) is recorded once every CTA of the launch runs.
 template <class... KA, class... A>
-int cluster_launch(void (*kern)(KA...), int nb, int size, cudaStream_t st, A... args) {
+int cluster_launch(void (*kern)(KA...), int nb, int size, cudaEvent_t begun, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(nb * size));
   cfg.blockDim = dim3(kClThreads);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)size;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  if (begun) {
+    at[1].id = cudaLaunchAttributeLaunchCompletionEvent;
+    at[1].val.launchCompletionEvent.event = begun;
+    at[1].val.launchCompletionEvent.flags = 0;
+    cfg.numAttrs = 2;
+  }
   count_launch();
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   if (e != cudaSuccess) {
@@ -778,7 +785,7 @@ int loewdin_launch(const LoewdinArgs& a, void* work, bool alone, cudaStream_t st
   LoewdinWork w;
   w.Y[0] = m; w.Y[1] = m + sm; w.Z[0] = m + 2 * sm; w.Z[1] = m + 3 * sm; w.T = m + 4 * sm;
   w.slots = (double*)(m + 5 * sm);
-  return cluster_launch(loewdin_kernel, 2, alone ? cluster_size(max2(a.nper)) : 1, st, a, w);
+  return cluster_launch(loewdin_kernel, 2, alone ? cluster_size(max2(a.nper)) : 1, nullptr, st, a, w);
 }
 
 size_t refine_bytes(int nb, int ld) {
@@ -786,7 +793,7 @@ size_t refine_bytes(int nb, int ld) {
          sizeof(double) * ((size_t)nb * ld + 12 * kClMax) + sizeof(int) * (size_t)nb * ld * 4;
 }
 
-int refine_launch(int nb, const RefineArgs& a, void* work, cudaStream_t st) {
+int refine_launch(int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st) {
   if (a.ld > kRefMaxN) return HFB_ERR_UNSUPPORTED_GRID;
   const size_t sm = (size_t)nb * a.ld * a.ld;
   double2* m = (double2*)work;
@@ -799,7 +806,7 @@ int refine_launch(int nb, const RefineArgs& a, void* work, cudaStream_t st) {
   static const bool wide =
       cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
   const int n = nb > 1 ? max2(a.nper) : a.nper.v[0];
-  return cluster_launch(refine_kernel, 1, cluster_size(n, wide ? 16 : 8), st, a, w, nb);
+  return cluster_launch(refine_kernel, 1, cluster_size(n, wide ? 16 : 8), begun, st, a, w, nb);
 }
 
 size_t construct_bytes(int ld) { return sizeof(double2) * 2 * 2 * (size_t)ld * ld + sizeof(double) * 2 * 4 * kClMax; }
@@ -810,7 +817,7 @@ int construct_launch(const ConstructArgs& a, void* work, cudaStream_t st) {
   w.TH = (double2*)work;
   w.TG = w.TH + sm;
   w.slots = (double*)(w.TG + sm);
-  return cluster_launch(construct_kernel, 2, cluster_size(max2(a.nper)), st, a, w);
+  return cluster_launch(construct_kernel, 2, cluster_size(max2(a.nper)), nullptr, st, a, w);
 }
 
 }  // namespace hfb
