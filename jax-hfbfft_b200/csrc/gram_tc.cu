@@ -22,10 +22,12 @@
 // (fewer when the launch is to leave SMs to what runs beside it).  The slices
 // depend on the grid alone, so no sum's order depends on which matrices are
 // computed together.
-//   warps 0-6   load a block of 16 points of the rows from global memory (the
-//               next block's loads are in flight while this one is split),
-//               split it and store it into a 128-byte-swizzled stage
-//               (3-stage ring);
+//   warps 0-5   split a block of 16 points of the rows from the raw ring into
+//               a 128-byte-swizzled stage (two of them);
+//   warp 6      fills the raw ring by TMA, 16 rows a copy (two blocks and up
+//               in flight: rows lie a state apart, 1.8 MB at 48^3, so every
+//               row of a block is another page and a block takes 1.4 us to
+//               arrive; a block ahead in registers left the MMAs waiting);
 //   warp 7      issues the MMAs (M = 128, N = columns, K = 8) into TMEM
 //               accumulators, three in rotation for D_re and D_im, which start
 //               from zero every four blocks;
@@ -36,13 +38,10 @@
 // Per-slice partial sums are added in fp64 in a fixed order by a second
 // kernel, which also writes the mirrored elements.
 // A row that is also a column (S, G) is loaded once and stored twice.
-// Bound by the producers: rows lie a state apart (1.8 MB at 48^3), every row of
-// a block is another page, and a block's 35 KB take 1.4 us to arrive although
-// its lines were brought into L2 four blocks before (MMAs alone: 1.0 us).
-// Pb208 (140 + 96 states,
-// 48^3), S + lambda and H + G: 3.04 ms with the real and imaginary rows in
-// units of their own (each loaded and split separately), 2.4 ms here.
-// (Feeding the blocks by TMA into a raw ring measured slower for that form.)
+// Pb208 (140 + 96 states, 48^3), S + lambda and H + G: 3.04 ms with the real
+// and imaginary rows in units of their own (each loaded and split separately),
+// 2.4 ms with the rows loaded through registers, 1.37 ms here; Zr90 (61 + 47
+// states, 40^3, S + H + G): 329, 337, 262 us.
 // Every wait is bounded; a timeout latches HFB_ERR_CUDA, drains the MMAs
 // in flight and releases TMEM before returning.
 #include <math.h>
@@ -54,35 +53,34 @@ namespace hfb {
 
 namespace {
 
-constexpr int kTcProducerWarps = 7;
-constexpr int kTcEpilogueWarps = 8;
-constexpr int kTcThreads = 32 * (kTcProducerWarps + 1 + kTcEpilogueWarps);
+constexpr int kTcSplitWarps = 6, kTcLoadWarp = 6, kTcMmaWarp = 7, kTcEpilogueWarps = 8;
+constexpr int kTcThreads = 32 * (kTcMmaWarp + 1 + kTcEpilogueWarps);
 // registers: 512 x 128 at launch, then 256 x 72 + 256 x 184
 constexpr int kTcProducerRegs = 72, kTcEpilogueRegs = 184;
-constexpr int kTcStages = 3;
+constexpr int kTcStages = 2, kTcMaxRaw = 8;   // split and raw stages
 constexpr int kTcMaxNp = 160;           // padded states per isospin handled here
 constexpr int kTcMaxCols = 144;         // columns of a unit: the epilogue's accumulator registers
 constexpr int kTcMaxUnits = 32;
-constexpr int kTcItems = 5;             // 32-byte row quarters per producer thread and block
-static_assert(kTcItems * kTcProducerWarps * 32 >= 4 * (128 + kTcMaxCols), "producer share");
+constexpr int kTcBoxRows = 16, kTcBoxBytes = kTcBoxRows * 128;
+constexpr int kTcMaxBoxes = 18;         // columns, rows among them or not, other rows: 9 + 8 at most
+constexpr int kTcItems = 6;             // 32-byte row quarters per splitting thread and block
+static_assert(kTcItems * kTcSplitWarps * 32 >= 4 * kTcBoxRows * kTcMaxBoxes, "splitters' share");
 constexpr int kTcTmemCols = 512, kTcAccCols = 160;   // three accumulators
 // up to this many states hi*(hi|lo) is one MMA of twice the columns (Zr90, 61 +
 // 47 states, 40^3: 337 us against 360); by the states of the isospin, not the
 // columns of the unit, so that it depends on nothing else
 constexpr int kTcPairCols = kTcAccCols / 2;
 constexpr uint32_t kTcABytes = 128 * 128;   // 128 rows x 128 bytes
-constexpr uint32_t kTcStageBytes = 2 * kTcABytes + 2 * kTcMaxCols * 128;
 constexpr long long kTcWaitLimit = 2000000000LL;
 // Blocks accumulated in TMEM between drains into registers: 4 measured 6 %
 // faster than 1 and stays inside the 3e-6 bar of the single-precision Gram
 // test
 constexpr int kTcDrain = 4;
-// blocks that a row's line is brought into L2 ahead of its load
-constexpr int kTcAhead = 4;
 // K slices: enough that the last wave of items is short, at least six drains
 constexpr int kTcMaxSlices = 148, kTcMinSlice = 24;
 constexpr int kTcMaxWin = 48 * 48 * 48 / 8 / kTcMaxSlices + 1;   // blocks of a slice of the largest grid
-constexpr size_t kTcSmem = 1024 + kTcStages * kTcStageBytes + sizeof(float) * 16 * kTcMaxWin;
+constexpr size_t kTcVps = sizeof(float) * 16 * kTcMaxWin;
+constexpr size_t kTcSmem = 226 * 1024;   // the rings take what they get
 static_assert(kTcMaxWin > 2 * kTcMinSlice, "slices of small grids");
 
 constexpr uint32_t kNone = 0xffffffffu;
@@ -91,9 +89,19 @@ enum TcGroup { TC_LOWER = 0, TC_UPPER = 1, TC_FULL = 2, TC_GROUPS = 3 };   // S 
 struct TcUnit {
   unsigned char b, group;      // isospin, TcGroup
   short row0, col0, cols;      // first stacked row; first column and padded count
+  short extra0, extra_n;       // psi rows of S or G that are not columns
+  short x0, x_n, xmap;         // rows of lambda or H, and their array
+  __host__ __device__ int boxes() const {
+    return cols / kTcBoxRows + (extra_n + kTcBoxRows - 1) / kTcBoxRows + (x_n + kTcBoxRows - 1) / kTcBoxRows;
+  }
+};
+struct TcMaps {
+  CUtensorMap m[2][3];         // [isospin][psi, hampsi, hmfpsi]
 };
 struct TcJob {
   int nunit, slices, kb_total, n3;
+  uint32_t stage_bytes, raw_bytes;
+  int raw_stages;
   TcUnit u[kTcMaxUnits];
   int s0[2], ns[2];
   int nm[2][TC_GROUPS];        // [isospin][group] matrices stacked
@@ -101,35 +109,30 @@ struct TcJob {
   const double* vp[2];
 };
 
-// volatile: the load stays where it is issued, a block ahead of its use
-__device__ __forceinline__ void ldg8(float4 (&v)[2], const float* p) {
-  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[0].z), "=f"(v[0].w), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[1].z),
-                 "=f"(v[1].w)
-               : "l"(p));
-}
-__device__ __forceinline__ void prefetch_l2(const float* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
-}
 __device__ __forceinline__ void tc_sync_all() { asm volatile("bar.sync 1, %0;" ::"n"(kTcThreads) : "memory"); }
 
 __global__ void __launch_bounds__(kTcThreads, 1)
-gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi, const float* __restrict__ hampsi,
-               const float* __restrict__ hmfpsi, float* __restrict__ part, int* ticket, int* status) {
+gram_tc_kernel(const __grid_constant__ TcJob job, const __grid_constant__ TcMaps maps, float* __restrict__ part,
+               int* ticket, int* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ uint64_t full[kTcStages], empty[kTcStages], dfull[3], dempty[3], fin;
+  __shared__ uint64_t full[kTcStages], empty[kTcStages], rfull[kTcMaxRaw], rempty[kTcMaxRaw], dfull[3], dempty[3], fin;
   __shared__ uint32_t tbase;
   __shared__ volatile int abort_flag;
   __shared__ volatile int next[2];
 
-  float* vps = reinterpret_cast<float*>(smem + kTcStages * kTcStageBytes);
+  unsigned char* raw = smem + kTcStages * job.stage_bytes;
+  float* vps = reinterpret_cast<float*>(raw + job.raw_stages * job.raw_bytes);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
   const int items = job.nunit * job.slices;
   if (tid == 0) {
     for (int s = 0; s < kTcStages; ++s) {
-      tc::mbar_init(&full[s], kTcProducerWarps);
+      tc::mbar_init(&full[s], kTcSplitWarps);
       tc::mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < kTcMaxRaw; ++s) {
+      tc::mbar_init(&rfull[s], 1);
+      tc::mbar_init(&rempty[s], kTcSplitWarps);
     }
     for (int d = 0; d < 3; ++d) {
       tc::mbar_init(&dfull[d], 1);
@@ -139,7 +142,7 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
     abort_flag = 0;
     next[0] = atomicAdd(ticket, 1);
   }
-  if (warp == kTcProducerWarps) {
+  if (warp == kTcMmaWarp) {
     tc::tmem_alloc(&tbase, kTcTmemCols);
     tc::tmem_relinquish();
   }
@@ -175,11 +178,10 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
   };
   int kb0, nwin;
 
-  if (warp <= kTcProducerWarps) {
+  if (warp <= kTcMmaWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcProducerRegs));
-    if (warp < kTcProducerWarps) {
-      // -------------------------------------------------------- producers
-      const size_t rowf = 4 * (size_t)job.n3;             // floats per state
+    if (warp < kTcSplitWarps) {
+      // -------------------------------------------------------- splitters
       const int q = tid & 3;                              // 32-byte quarter of the row
       int w = 0;                                          // blocks since the start
       for (int it = 0;; ++it) {
@@ -188,61 +190,53 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
         if (tid == 0) next[(it + 1) & 1] = atomicAdd(ticket, 1);
         const TcUnit U = job.u[item % job.nunit];
         const int b = U.b, n = job.ns[b], nm = job.nm[b][U.group];
-        const size_t start = (size_t)job.s0[b] * rowf + (size_t)kb0 * 32 + 8 * q;
-        const float* src[kTcItems];
+        const int cb = U.cols, eb = (U.extra_n + kTcBoxRows - 1) / kTcBoxRows * kTcBoxRows;
+        const int count = (U.boxes() * kTcBoxRows * 4 + kTcSplitWarps * 32 - 1) / (kTcSplitWarps * 32);
+        const bool upper = U.group == TC_UPPER, sg = job.mat[b][U.group][upper ? nm - 1 : 0] == (upper ? 3 : 0);
+        // place of row j of S or G / of lambda or H among the stacked rows
+        auto row_sg = [&](int j) { return (upper ? (n - 1 - j) * nm + nm - 1 : j * nm) - U.row0; };
+        auto row_x = [&](int j) { return (upper ? (n - 1 - j) * nm : j * nm + nm - 1) - U.row0; };
         uint32_t dst[kTcItems], dup[kTcItems];   // place, and for a column that is also a row, that place
         unsigned gmask = 0;
-        const bool shared_row = job.mat[b][U.group][U.group == TC_UPPER ? nm - 1 : 0] == (U.group == TC_UPPER ? 3 : 0);
-#pragma unroll
-        for (int p = 0; p < kTcItems; ++p) {
-          // eight threads store rows r and r + 4: their chunks fall on
-          // distinct banks
-          const int e = (p * kTcProducerWarps * 32 + tid) >> 2;
-          int r = (e & ~7) | ((e & 7) >> 1) | ((e & 1) << 2);
-          const float* base = nullptr;
-          dup[p] = kNone;
-          if (r < 128) {
-            const int g = U.row0 + r, j = U.group == TC_UPPER ? n - 1 - g / nm : g / nm;
-            if (g < n * nm) {
-              const int a = job.mat[b][U.group][g % nm];
-              const bool here = (a == 0 || a == 3) && j >= U.col0 && j < U.col0 + U.cols;
-              if (!here) base = (a == 1 ? hampsi : a == 2 ? hmfpsi : psi) + (size_t)j * rowf;
-              if (a == 3) gmask |= 1u << p;
-            }
-            dst[p] = tc::sw128_offset(r, q);
-          } else {
-            r -= 128;
-            const int i = U.col0 + r;
-            if (r < U.cols && i < n) {
-              base = psi + (size_t)i * rowf;
-              const int g = U.group == TC_UPPER ? (n - 1 - i) * nm + nm - 1 - U.row0 : i * nm - U.row0;
-              if (shared_row && g >= 0 && g < 128) dup[p] = tc::sw128_offset(g, q);
-            }
-            dst[p] = 2 * kTcABytes + tc::sw128_offset(r, q);
-          }
-          src[p] = base ? base + start : nullptr;
-        }
-        float4 d[kTcItems][2];
-        auto load = [&](int p) {
-          if (src[p]) {
-            ldg8(d[p], src[p]);
-            src[p] += 32;
-          }
+        auto raw_row = [&](int p) {
+          // eight threads take rows r and r ^ 5: both the raw chunks and the
+          // split ones fall on distinct banks
+          const int e = (p * kTcSplitWarps * 32 + tid) >> 2;
+          return (e & ~7) | (((e & 7) >> 1) ^ ((e & 1) * 5));
         };
 #pragma unroll
-        for (int p = 0; p < kTcItems; ++p) load(p);
-        if (job.mat[b][U.group][nm - 1] == 3) {   // v_pair of the slice
+        for (int p = 0; p < kTcItems; ++p) {
+          const int r = raw_row(p);
+          dst[p] = dup[p] = kNone;
+          if (r < cb) {
+            const int i = U.col0 + r, g = row_sg(i);
+            if (i < n) {
+              dst[p] = 2 * kTcABytes + tc::sw128_offset(r, q);
+              if (sg && g >= 0 && g < 128) dup[p] = tc::sw128_offset(g, q);
+            }
+          } else if (r < cb + eb) {
+            const int k = r - cb, j = U.extra0 + k;
+            if (k < U.extra_n && !(j >= U.col0 && j < U.col0 + U.cols)) {
+              dst[p] = tc::sw128_offset(row_sg(j), q);
+              if (upper) gmask |= 1u << p;
+            }
+          } else {
+            const int k = r - cb - eb;
+            if (k < U.x_n) dst[p] = tc::sw128_offset(row_x(U.x0 + k), q);
+          }
+        }
+        if (upper && sg) {   // v_pair of the slice
           const double* vp = job.vp[b];
-          for (int e = tid; e < 16 * nwin; e += 32 * kTcProducerWarps)
+          for (int e = tid; e < 16 * nwin; e += 32 * kTcSplitWarps)
             vps[e] = (float)vp[((size_t)kb0 * 16 + e) % (size_t)job.n3];
-          asm volatile("bar.sync 2, %0;" ::"n"(32 * kTcProducerWarps) : "memory");
+          asm volatile("bar.sync 2, %0;" ::"n"(32 * kTcSplitWarps) : "memory");
         }
         auto scale = [&](float4 (&x)[2], int i) {
           const float4 v = *reinterpret_cast<const float4*>(vps + 16 * i + 4 * q);
           x[0] = make_float4(v.x * x[0].x, v.x * x[0].y, v.y * x[0].z, v.y * x[0].w);
           x[1] = make_float4(v.z * x[1].x, v.z * x[1].y, v.w * x[1].z, v.w * x[1].w);
         };
-        auto put = [&](unsigned char* o, uint32_t lo, const float4 (&x)[2]) {
+        auto put = [&](unsigned char* st, uint32_t at, uint32_t lo, const float4 (&x)[2]) {
 #pragma unroll
           for (int c = 0; c < 2; ++c) {   // real parts, imaginary parts
             float4 h, l;
@@ -250,34 +244,75 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
             tc::split_tf32(c ? x[0].w : x[0].z, h.y, l.y);
             tc::split_tf32(c ? x[1].y : x[1].x, h.z, l.z);
             tc::split_tf32(c ? x[1].w : x[1].z, h.w, l.w);
-            unsigned char* t = reinterpret_cast<unsigned char*>((uintptr_t)o ^ (c ? 64u : 0u));
+            unsigned char* t = st + (at ^ (c ? 64u : 0u));
             *reinterpret_cast<float4*>(t) = h;
             *reinterpret_cast<float4*>(t + lo) = l;
           }
         };
         for (int i = 0; i < nwin; ++i, ++w) {
-          const int s = w % kTcStages;
+          const int s = w % kTcStages, rs = w % job.raw_stages;
+          if (!wait(&rfull[rs], (uint32_t)((w / job.raw_stages) & 1))) break;
           if (w >= kTcStages && !wait(&empty[s], (uint32_t)((w / kTcStages - 1) & 1))) break;
-          unsigned char* st = smem + (size_t)s * kTcStageBytes;
+          unsigned char* st = smem + (size_t)s * job.stage_bytes;
+          const unsigned char* rw = raw + (size_t)rs * job.raw_bytes;
 #pragma unroll
-          for (int p = 0; p < kTcItems; ++p) {
-            if (!src[p]) continue;
-            const bool isb = dst[p] >= 2 * kTcABytes;
-            const uint32_t lo = isb ? (uint32_t)U.cols * 128 : kTcABytes;
-            if ((gmask >> p) & 1) scale(d[p], i);
-            put(st + dst[p], lo, d[p]);
-            if (dup[p] != kNone) {
-              if (U.group == TC_UPPER) scale(d[p], i);
-              put(st + dup[p], kTcABytes, d[p]);
+          for (int h = 0; h < kTcItems; h += 3) {
+            float4 d[3][2];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              if (h + k < count) {
+                const int r = raw_row(h + k);
+                d[k][0] = *reinterpret_cast<const float4*>(rw + tc::sw128_offset(r, 2 * q));
+                d[k][1] = *reinterpret_cast<const float4*>(rw + tc::sw128_offset(r, 2 * q + 1));
+              }
+            if (h + 3 >= kTcItems) {
+              __syncwarp();
+              if (lane == 0) tc::mbar_arrive(&rempty[rs]);
             }
-            if (i + 1 < nwin) load(p);
-            if (q == 0 && i + kTcAhead < nwin) prefetch_l2(src[p] + 32 * (kTcAhead - 2));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const int p = h + k;
+              if (p >= count || dst[p] == kNone) continue;
+              if ((gmask >> p) & 1) scale(d[k], i);
+              put(st, dst[p], dst[p] >= 2 * kTcABytes ? (uint32_t)U.cols * 128 : kTcABytes, d[k]);
+              if (dup[p] != kNone) {
+                if (upper) scale(d[k], i);
+                put(st, dup[p], kTcABytes, d[k]);
+              }
+            }
           }
           tc::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(&full[s]);
         }
       }
+    } else if (warp == kTcLoadWarp) {
+      // ------------------------------------------------------------ loads
+      int w = 0;
+      for (int it = 0;; ++it) {
+        const int item = take(it, kb0, nwin);
+        if (item < 0) break;
+        const TcUnit U = job.u[item % job.nunit];
+        const int boxes = U.boxes(), cbox = U.cols / kTcBoxRows, ebox = (U.extra_n + kTcBoxRows - 1) / kTcBoxRows;
+        // this lane's box: its array and first row (rows past the last read as zero)
+        const CUtensorMap* map = &maps.m[U.b][lane < cbox + ebox ? 0 : U.xmap];
+        const int y = lane < cbox          ? U.col0 + kTcBoxRows * lane
+                      : lane < cbox + ebox ? U.extra0 + kTcBoxRows * (lane - cbox)
+                                           : U.x0 + kTcBoxRows * (lane - cbox - ebox);
+        for (int i = 0; i < nwin; ++i, ++w) {
+          const int rs = w % job.raw_stages;
+          if (w >= job.raw_stages && !wait(&rempty[rs], (uint32_t)((w / job.raw_stages - 1) & 1))) break;
+          if (lane == 0) tc::mbar_arrive_expect_tx(&rfull[rs], (uint32_t)(boxes * kTcBoxBytes));
+          __syncwarp();
+          if (lane < boxes)
+            tc::tma_load_2d(raw + (size_t)rs * job.raw_bytes + lane * kTcBoxBytes, map, (kb0 + i) * 32, y, &rfull[rs]);
+          __syncwarp();
+        }
+      }
+      // no copy is in flight when the CTA ends
+      for (int k = w > job.raw_stages ? w - job.raw_stages : 0; k < w; ++k)
+        if (!tc::mbar_wait(&rfull[k % job.raw_stages], (uint32_t)((k / job.raw_stages) & 1), kTcWaitLimit))
+          latch_error(status, HFB_ERR_CUDA);
     } else {
       // -------------------------------------------------------------- MMA
       int w = 0, grp = 0, nfin = 0;
@@ -300,7 +335,7 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
           if (first && er >= 3 && ok) ok = wait(&dempty[er % 3], (uint32_t)((er / 3 - 1) & 1));
           if (!ok) break;
           tc::fence_after();
-          const uint64_t da = stage0 + (uint64_t)((uint32_t)s * (kTcStageBytes >> 4)), db = da + 2 * loa;
+          const uint64_t da = stage0 + (uint64_t)((uint32_t)s * (job.stage_bytes >> 4)), db = da + 2 * loa;
           const uint32_t dr = tmem + (uint32_t)(er % 3) * kTcAccCols, di = tmem + (uint32_t)(ei % 3) * kTcAccCols;
           auto mma3 = [&](uint32_t dt, int ka, int kb, uint32_t id, uint32_t acc) {
             if (pair) {
@@ -347,7 +382,7 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
     // ----------------------------------------------------------- epilogue
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcEpilogueRegs));
     const int qd = warp & 3;                              // TMEM lane quarter of this warp
-    const int im = (warp - kTcProducerWarps - 1) / 4;     // D_re or D_im
+    const int im = (warp - kTcMmaWarp - 1) / 4;     // D_re or D_im
     int grp = 0;
     for (int it = 0;; ++it) {
       const int item = take(it, kb0, nwin);
@@ -397,7 +432,7 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const float* __restrict__ psi,
   }
   tc::fence_before();
   __syncthreads();
-  if (warp == kTcProducerWarps) {
+  if (warp == kTcMmaWarp) {
     tc::fence_after();
     tc::tmem_dealloc(tmem, kTcTmemCols);
   }
@@ -459,7 +494,8 @@ gram_tc_reduce_kernel(const __grid_constant__ TcJob job, const float* __restrict
 
 }  // namespace
 
-// Returns HFB_ERR_UNSUPPORTED_GRID when a block exceeds kTcMaxNp states
+// Returns HFB_ERR_UNSUPPORTED_GRID when a block exceeds kTcMaxNp states or its
+// arrays have no tensor map (base not 16-byte aligned)
 // (the caller then uses the CUDA-core kernel).
 int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const int* masks, const void* psi,
                    const void* hampsi, const void* hmfpsi, const double* const* vp, double wxyz,
@@ -467,6 +503,8 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
   TcJob job{};
   job.n3 = c->n * c->n * c->n;
   job.kb_total = job.n3 / 8;
+  TcMaps maps{};
+  int boxes = 0, widest = 0;
   for (int b = 0; b < nblk; ++b) {
     if (ns[b] <= 0) continue;
     const int n = ns[b];
@@ -479,6 +517,14 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
       const int g = a >= 2 ? TC_UPPER : a == 1 && !(masks[b] & kGramLowerLambda) ? TC_FULL : TC_LOWER;
       job.mat[b][g][job.nm[b][g]++] = (unsigned char)a;
     }
+    const void* arrays[3] = {psi, hampsi, hmfpsi};
+    for (int a = 0; a < 3; ++a)
+      if (a == 0 || (masks[b] & (1 << a))) {
+        const float* base = (const float*)arrays[a] + (size_t)s0[b] * 4 * job.n3;
+        // (the CUDA-core kernel takes any alignment)
+        if (!encode_fp32_rows_map(&maps.m[b][a], base, 4 * (uint64_t)job.n3, n, kTcBoxRows))
+          return HFB_ERR_UNSUPPORTED_GRID;
+      }
     for (int g = 0; g < TC_GROUPS; ++g) {
       const int nm = job.nm[b][g];
       for (int row0 = 0; row0 < n * nm; row0 += 128) {
@@ -487,8 +533,26 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
         const int parts = (all + kTcMaxCols - 1) / kTcMaxCols, cols = (all / 16 + parts - 1) / parts * 16;
         for (int col0 = first; col0 < end; col0 += cols) {
           if (job.nunit >= kTcMaxUnits) return HFB_ERR_UNSUPPORTED_GRID;
-          job.u[job.nunit++] = TcUnit{(unsigned char)b, (unsigned char)g, (short)row0, (short)col0,
-                                      (short)std::min(cols, (end - col0 + 15) / 16 * 16)};
+          TcUnit u{(unsigned char)b, (unsigned char)g, (short)row0, (short)col0,
+                   (short)std::min(cols, (end - col0 + 15) / 16 * 16), 0, 0, 0, 0, 0};
+          // the vectors j of the block's rows
+          const int ja = row0 / nm, jb = (std::min(row0 + 128, n * nm) - 1) / nm;
+          const int j0 = g == TC_UPPER ? n - 1 - jb : ja, jn = jb - ja + 1;
+          for (int m = 0; m < nm; ++m) {
+            const int a = job.mat[b][g][m];
+            if (a == 1 || a == 2) {
+              u.x0 = (short)j0;
+              u.x_n = (short)jn;
+              u.xmap = (short)a;
+            } else if (j0 < col0 || j0 + jn > std::min(col0 + u.cols, n)) {
+              u.extra0 = (short)j0;
+              u.extra_n = (short)jn;
+            }
+          }
+          if (u.boxes() > kTcMaxBoxes) return HFB_ERR_UNSUPPORTED_GRID;
+          boxes = std::max(boxes, u.boxes());
+          widest = std::max(widest, (int)u.cols);
+          job.u[job.nunit++] = u;
         }
       }
     }
@@ -502,8 +566,10 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
   if (!part) return HFB_ERR_ALLOC;
   int* ticket = c->counters + 1;
   allow_max_dynamic_smem(gram_tc_kernel);
-  gram_tc_kernel<<<std::min(items, sms), kTcThreads, kTcSmem, st>>>(job, (const float*)psi, (const float*)hampsi,
-                                                                   (const float*)hmfpsi, part, ticket, c->dev_status);
+  job.stage_bytes = 2 * kTcABytes + 2 * widest * 128;
+  job.raw_bytes = (uint32_t)(boxes * kTcBoxBytes);
+  job.raw_stages = std::min<int>(kTcMaxRaw, (kTcSmem - 1024 - kTcVps - kTcStages * job.stage_bytes) / job.raw_bytes);
+  gram_tc_kernel<<<std::min(items, sms), kTcThreads, kTcSmem, st>>>(job, maps, part, ticket, c->dev_status);
   HFB_CHECK_LAUNCH();
   TcOut ot;
   for (int q = 0; q < 8; ++q) ot.p[q] = outs_host[q];
