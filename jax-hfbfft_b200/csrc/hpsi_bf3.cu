@@ -36,6 +36,13 @@
 // F[tile][point][line] so that every pass reads them coalesced, with the
 // line means of B precomputed for the Nyquist term.
 //
+// The tile's psi is copied to shared memory once per pass and read there in
+// all three steps; the z pass, whose lines are rows, hands its result back
+// through it.  (Read row by row from global memory, three times and written
+// once, a z tile took 12000 of the SM's load/store cycles: Pb208, 236 states at
+// 48^3, 1.31 ms a call against 1.03 here; Zr90, 108 states at 40^3, 366 us
+// against 313.  Bringing the next z tile into L2 ahead changed nothing.)
+//
 // Scheduling as in the tf32 kernel (hpsi_tc.cu): persistent CTAs take tasks
 // from an atomic ticket in the order [z tiles][y tiles][x tiles] per group
 // of states; a y (x) tile waits before its epilogue until every z (y) tile
@@ -77,6 +84,7 @@ struct HbGeo {
   static constexpr int T = N * N / kHbLines;        // tiles per state and axis
   static constexpr uint32_t BTILE = N2 * 128;       // one bf16 B tile: N2 rows of 64 bf16
   static constexpr uint32_t BAXIS = 3 * BTILE;      // h, m, l
+  static constexpr size_t PSBYTES = sizeof(float2) * 2 * kHbLines * (N + 2);   // the staged tile
   static_assert(DCOL + 2 * N2 <= kHbTmemCols, "TMEM budget of one tile");
   static_assert(N % 8 == 0 && (N * N) % kHbLines == 0 && N <= 48, "grid size");
   static_assert(BTILE % 1024 == 0, "B tiles stay 1024-byte aligned");
@@ -300,44 +308,57 @@ __device__ __forceinline__ bool hb_decode(const HbArgs& a, int task, int& pass, 
   return true;
 }
 
-// The thread's PT points of its row, complex, from a state-sized array
+// Place of point j of line ln and component c in the staged tile: the z pass
+// keeps lines as rows of N + 2 (an odd number of 16-byte units), the others
+// points as rows of 64 lines, the second component shifted by half a row of
+// banks.
 template <int N, int AX>
-__device__ __forceinline__ void hb_load_row(const float2* __restrict__ src, size_t cb, float2 (&v)[HbGeo<N>::PT]) {
-  using G = HbGeo<N>;
-  constexpr size_t STRIDE = AX == 2 ? 1 : (AX == 1 ? (size_t)N : (size_t)N * N);
-  if (AX == 2) {
-    const float4* s4 = reinterpret_cast<const float4*>(src + cb);   // cb even: 16-byte aligned
-#pragma unroll
-    for (int i = 0; i < G::PT / 2; ++i) {
-      const float4 q = __ldg(s4 + i);
-      v[2 * i] = make_float2(q.x, q.y);
-      v[2 * i + 1] = make_float2(q.z, q.w);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < G::PT; ++i) v[i] = __ldg(src + cb + i * STRIDE);
-  }
+__device__ __forceinline__ int hb_at(int c, int ln, int j) {
+  return AX == 2 ? (2 * ln + c) * (N + 2) + j : c * (N * kHbLines + 8) + j * kHbLines + ln;
 }
-
+// Start copying the tile's psi; 16 bytes a copy: two points of a line (z) or two
+// lines' points (N is even, so both lines share their other coordinate).
+template <int N, int AX>
+__device__ __forceinline__ void hb_stage(float2* ps, const float2* __restrict__ psi, int s, int tile) {
+  constexpr size_t N3 = (size_t)N * N * N;
+  constexpr size_t STRIDE = AX == 1 ? (size_t)N : (size_t)N * N;
+#pragma unroll 4
+  for (int e = threadIdx.x; e < N * kHbLines; e += kHbThreads) {
+    const int c = e / (N * kHbLines / 2), r = e % (N * kHbLines / 2);
+    const float2* src = psi + ((size_t)s * 2 + c) * N3;
+    int ln, j;
+    if (AX == 2) {
+      ln = 2 * r / N;
+      j = 2 * r % N;
+      src += (size_t)tile * kHbLines * N + 2 * r;
+    } else {
+      ln = 2 * r % kHbLines;
+      j = 2 * r / kHbLines;
+      src += hb_line_base<N, AX>(tile * kHbLines + ln) + j * STRIDE;
+    }
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(tc::smem_u32(ps + hb_at<N, AX>(c, ln, j))), "l"(src)
+                 : "memory");
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
 // Points 4k .. 4k+3 of the thread's run
 template <int N, int AX>
-__device__ __forceinline__ void hb_load_chunk(const float2* __restrict__ src, size_t cb, int k, float2 (&v)[4]) {
-  constexpr size_t STRIDE = AX == 2 ? 1 : (AX == 1 ? (size_t)N : (size_t)N * N);
+__device__ __forceinline__ void hb_chunk(const float2* own, int k, float2 (&v)[4]) {
   if (AX == 2) {
-    const float4* s4 = reinterpret_cast<const float4*>(src + cb) + 2 * k;
-    const float4 q0 = __ldg(s4), q1 = __ldg(s4 + 1);
+    const float4* s4 = reinterpret_cast<const float4*>(own) + 2 * k;
+    const float4 q0 = s4[0], q1 = s4[1];
     v[0] = make_float2(q0.x, q0.y);
     v[1] = make_float2(q0.z, q0.w);
     v[2] = make_float2(q1.x, q1.y);
     v[3] = make_float2(q1.z, q1.w);
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __ldg(src + cb + (4 * k + i) * STRIDE);
+    for (int i = 0; i < 4; ++i) v[i] = own[(4 * k + i) * kHbLines];
   }
 }
 
 template <int N, int AX, int P>
-__device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbShared& sh, uint32_t bsm, int s,
+__device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbShared& sh, uint32_t bsm, float2* ps, int s,
                                         int tile, uint32_t& phase, bool& b_ready) {
   using G = HbGeo<N>;
   constexpr size_t N3 = (size_t)N * N * N;
@@ -348,31 +369,34 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
   const uint32_t bax = bsm + AX * a.bstride;
 
   // ---- staging: psi -> the A operand; partial alternating sums
+  hb_stage<N, AX>(ps, a.psi, s, tile);
+  float2* own = ps + hb_at<N, AX>(t.c, t.ln, t.j0);
+  // The pointwise step's fields do not depend on GEMM 1: the first are loaded
+  // ahead of it.
+  const float4* fp = a.F + ((size_t)iq * 3 + AX) * N3 + hb_fidx<N>(L, t.j0);
+  float4 fn[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) fn[i] = __ldg(fp + i * kHbLines);
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
   {
-    float2 v[G::PT];
-    hb_load_row<N, AX>(a.psi, cb, v);
     float2 alt = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < G::PT; ++i) {
-      alt.x += (i & 1) ? -v[i].x : v[i].x;   // (-1)^j psi_j, j0 even
-      alt.y += (i & 1) ? -v[i].y : v[i].y;
+    for (int k = 0; k < G::NCK; ++k) {
+      float2 v[4];
+      hb_chunk<N, AX>(own, k, v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        alt.x += (i & 1) ? -v[i].x : v[i].x;   // (-1)^j psi_j, j0 even
+        alt.y += (i & 1) ? -v[i].y : v[i].y;
+      }
+      hb_store_a<N>(t.tl, t.c0 + 2 * k, v[0], v[1], v[2], v[3]);
     }
     sh.alt[t.row][t.g] = alt;
-#pragma unroll
-    for (int k = 0; k < G::NCK; ++k)
-      hb_store_a<N>(t.tl, t.c0 + 2 * k, v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
   }
   tc::tmem_st_wait();
   tc::fence_before();
   __syncthreads();
-  // The pointwise step's first global inputs do not depend on GEMM 1:
-  // they are loaded while it runs.
-  const float4* fp = a.F + ((size_t)iq * 3 + AX) * N3 + hb_fidx<N>(L, t.j0);
-  float4 fn[4];
-  float2 pn[4];
-  hb_load_chunk<N, AX>(a.psi, cb, 0, pn);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) fn[i] = __ldg(fp + i * kHbLines);
   // ---- GEMM 1: e = D psi
   if (threadIdx.x == 0) {
     tc::fence_after();
@@ -394,7 +418,7 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
   const float2 alt = make_float2(sh.alt[t.row][0].x + sh.alt[t.row][1].x, sh.alt[t.row][0].y + sh.alt[t.row][1].y);
 
   // ---- pointwise: o = L_d e over e in the accumulator, w = L_d psi - B e into A.
-  // The global loads of chunk k + 1 are issued before the TMEM accesses of
+  // The fields of chunk k + 1 are loaded before the TMEM accesses of
   // chunk k (which the compiler cannot reorder memory operations across),
   // so they are in flight while chunk k is computed.
 #pragma unroll
@@ -402,15 +426,12 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
     float4 f[4];
     float2 pc[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[i] = fn[i];
-      pc[i] = pn[i];
-    }
+    for (int i = 0; i < 4; ++i) f[i] = fn[i];
     if (k + 1 < G::NCK) {
-      hb_load_chunk<N, AX>(a.psi, cb, k + 1, pn);
 #pragma unroll
       for (int i = 0; i < 4; ++i) fn[i] = __ldg(fp + (4 * (k + 1) + i) * kHbLines);
     }
+    hb_chunk<N, AX>(own, k, pc);
     uint32_t er[4], em[4];
     tc::tmem_ld_x4(t.tl + G::DCOL + t.j0 + 4 * k, er);
     tc::tmem_ld_x4(t.tl + G::DCOL + G::N2 + t.j0 + 4 * k, em);
@@ -452,19 +473,18 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
   // ---- epilogue: o + D w + Nyquist term, 4 points at a time.  The global
   // inputs of chunk k + 1 are loaded before the TMEM reads of chunk k (as in
   // the pointwise step), chunk 0's while GEMM 2 runs: the previous pass's
-  // sum (y, x passes), psi and the local fields for the z pass's upot / spin
-  // terms, psi and v_pair for the x pass's outputs.
+  // sum (y, x passes), the local fields for the z pass's upot / spin terms,
+  // v_pair for the x pass's outputs.
   const float nyq = a.nq[AX] * a.bbar[((size_t)iq * 3 + AX) * N * N + L];
   const float wt = (P == 2 && a.weight) ? (float)a.weight[s] : 1.f;
   const float wu = (P == 2 && a.weightuv) ? (float)a.weightuv[s] : 0.f;
   const float* vpq = a.pot + ((size_t)iq * 12 + 2) * N3 + hb_line_base<N, AX>(L) + (size_t)t.j0 * STRIDE;
   const float4* flp = a.FL + (size_t)iq * N3 + hb_fidx<N>(L, t.j0);
   double ov_mf = 0.0, ov_po = 0.0;
-  float2 qn[4], on[4];
+  float2 on[4];
   float4 gn[4];
   float vn[4];
-  auto fetch = [&](int k, float2 (&pc)[4], float2 (&od)[4], float4 (&gl)[4], float (&vp)[4]) {
-    if (P != 1) hb_load_chunk<N, AX>(a.psi, cb, k, pc);
+  auto fetch = [&](int k, float2 (&od)[4], float4 (&gl)[4], float (&vp)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (P > 0) od[i] = __ldcg(a.acc + cb + (4 * k + i) * STRIDE);
@@ -472,7 +492,7 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
       if (P == 2) vp[i] = __ldg(vpq + (4 * k + i) * STRIDE);
     }
   };
-  if (!sh.bad) fetch(0, qn, on, gn, vn);
+  if (!sh.bad) fetch(0, on, gn, vn);
   if (threadIdx.x == 0 && !tc::mbar_wait(&sh.bar_mma, phase & 1, a.wait_limit)) sh.bad = 1;
   ++phase;
   __syncthreads();
@@ -485,12 +505,12 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
     float vp[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      pc[i] = qn[i];
       old[i] = on[i];
       gl[i] = gn[i];
       vp[i] = vn[i];
     }
-    if (k + 1 < G::NCK) fetch(k + 1, qn, on, gn, vn);
+    if (k + 1 < G::NCK) fetch(k + 1, on, gn, vn);
+    if (P != 1) hb_chunk<N, AX>(own, k, pc);
     uint32_t dr[4], di[4];
     tc::tmem_ld_x4(t.tl + G::DCOL + t.j0 + 4 * k, dr);
     tc::tmem_ld_x4(t.tl + G::DCOL + G::N2 + t.j0 + 4 * k, di);
@@ -511,7 +531,7 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
       }
     }
     if (P == 0) {
-      float4* d4 = reinterpret_cast<float4*>(a.acc + cb) + 2 * k;
+      float4* d4 = reinterpret_cast<float4*>(own) + 2 * k;
       d4[0] = make_float4(z[0].x, z[0].y, z[1].x, z[1].y);
       d4[1] = make_float4(z[2].x, z[2].y, z[3].x, z[3].y);
     } else if (P == 1) {
@@ -539,6 +559,15 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
     }
   }
   tc::fence_before();   // accumulator reads done before the next tile's GEMM 1
+  if (P == 0) {
+    __syncthreads();
+#pragma unroll 4
+    for (int e = threadIdx.x; e < N * kHbLines; e += kHbThreads) {
+      const int c = e / (N * kHbLines / 2), r = e % (N * kHbLines / 2);
+      *reinterpret_cast<float4*>(a.acc + ((size_t)s * 2 + c) * N3 + (size_t)tile * kHbLines * N + 2 * r) =
+          *reinterpret_cast<const float4*>(ps + hb_at<N, 2>(c, 2 * r / N, 2 * r % N));
+    }
+  }
   if (P == 2 && a.ovl) {
     // deterministic per-tile partial sums: warp shuffles, then thread 0
 #pragma unroll
@@ -615,6 +644,7 @@ __global__ void __launch_bounds__(kHbThreads, 2) hpsi_bf3_kernel(HbArgs a) {
   t.tb = sh.tmem_base;
   t.tl = t.tb + ((uint32_t)(32 * q) << 16);
   const uint32_t bsm = tc::smem_u32(bs);
+  float2* ps = reinterpret_cast<float2*>(bs + a.bbytes);
   // K padding of the A operand (n = 24, 40): zero once, never written again
   if (G::KP > N && t.g == 1) {
 #pragma unroll
@@ -632,11 +662,11 @@ __global__ void __launch_bounds__(kHbThreads, 2) hpsi_bf3_kernel(HbArgs a) {
     if (sh.bad || !hb_decode<N>(a, task, pass, s, tile)) break;
     if (tid == 0) sh.next = hb_ticket(a);
     if (pass == 0)
-      hb_tile<N, 2, 0>(a, t, sh, bsm, s, tile, phase, b_ready);
+      hb_tile<N, 2, 0>(a, t, sh, bsm, ps, s, tile, phase, b_ready);
     else if (pass == 1)
-      hb_tile<N, 1, 1>(a, t, sh, bsm, s, tile, phase, b_ready);
+      hb_tile<N, 1, 1>(a, t, sh, bsm, ps, s, tile, phase, b_ready);
     else
-      hb_tile<N, 0, 2>(a, t, sh, bsm, s, tile, phase, b_ready);
+      hb_tile<N, 0, 2>(a, t, sh, bsm, ps, s, tile, phase, b_ready);
     // every thread reads sh.next (written before the tile's first barrier)
     // before this barrier, and thread 0 rewrites it only after it
     task = sh.next;
@@ -778,7 +808,7 @@ int hpsi_bf3_launch_t(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, 
   a.wait_limit = c->wait_limit;
   a.probe = c->timeout_probe;
   c->timeout_probe = 0;   // one launch only
-  size_t smem = (size_t)a.bbytes + 1024;
+  size_t smem = (size_t)a.bbytes + 1024 + G::PSBYTES;
   if (smem < kHbMinSmem) smem = kHbMinSmem;
   allow_max_dynamic_smem(hpsi_bf3_kernel<N>);
   hpsi_bf3_kernel<N><<<ntask < slots ? ntask : slots, kHbThreads, smem, st>>>(a);
