@@ -4,6 +4,9 @@
 #include <stdlib.h>
 #include <string.h>
 #include <atomic>
+#include <mutex>
+#include <set>
+#include <utility>
 #include <vector>
 #include <cudaTypedefs.h>
 #include "hfb_ctx.cuh"
@@ -12,6 +15,24 @@ namespace hfb {
 
 static std::atomic<unsigned long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+// (device, kernel) pairs whose shared-memory limit has been raised
+static std::mutex g_smem_mutex;
+static std::set<std::pair<int, const void*>>& smem_raised() {
+  static std::set<std::pair<int, const void*>> s;
+  return s;
+}
+bool smem_limit_raised(const void* fn) {
+  int d = 0;
+  if (cudaGetDevice(&d) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(g_smem_mutex);
+  return smem_raised().count({d, fn}) != 0;
+}
+void note_smem_limit_raised(const void* fn) {
+  int d = 0;
+  if (cudaGetDevice(&d) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lock(g_smem_mutex);
+  smem_raised().insert({d, fn});
+}
 static thread_local int t_last_cuda_error = 0;
 void note_cuda_error(int e) { t_last_cuda_error = e; }
 

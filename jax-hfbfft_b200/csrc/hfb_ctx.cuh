@@ -59,12 +59,15 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 // Counts every kernel launch of the library (reported by hfb_launch_count).
 // Allow a kernel all the dynamic shared memory the device opts in to (the
-// opt-in maximum less the kernel's static shared memory).  Every call sets
-// the same value for a kernel, so host threads launching it concurrently
-// with different shared-memory sizes never lower the limit under one
-// another's launches.
+// opt-in maximum less the kernel's static shared memory).  Done at a kernel's
+// first launch on a device: the two runtime calls cost about 1 us of host time
+// each launch, of 26 us for hpsi01 on one 16^3 spinor.  Every host thread sets
+// the same value, so it does not matter which one is first.
+bool smem_limit_raised(const void* fn);      // on the current device
+void note_smem_limit_raised(const void* fn);
 template <class F>
 inline void allow_max_dynamic_smem(F* fn) {
+  if (smem_limit_raised((const void*)fn)) return;
   static const int optin = [] {
     int d = 0, v = 0;
     cudaGetDevice(&d);
@@ -72,13 +75,13 @@ inline void allow_max_dynamic_smem(F* fn) {
     return v;
   }();
   cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) {
+  if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) !=
+          cudaSuccess) {
     cudaGetLastError();
     return;
   }
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) !=
-      cudaSuccess)
-    cudaGetLastError();
+  note_smem_limit_raised((const void*)fn);
 }
 void note_cuda_error(int e);   // the CUDA error behind the last HFB_ERR_CUDA of this host thread
 // Tensor map of a rows x row_floats fp32 matrix (row pitch row_floats) read in
