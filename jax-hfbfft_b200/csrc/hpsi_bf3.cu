@@ -40,8 +40,8 @@
 // all three steps; the z pass, whose lines are rows, hands its result back
 // through it.  (Read row by row from global memory, three times and written
 // once, a z tile took 12000 of the SM's load/store cycles: Pb208, 236 states at
-// 48^3, 1.31 ms a call against 1.03 here; Zr90, 108 states at 40^3, 366 us
-// against 313.  Bringing the next z tile into L2 ahead changed nothing.)
+// 48^3, 1.31 ms a call before, 1.03 with it; Zr90, 108 states at 40^3, 366 us
+// and 313.  Bringing the next z tile into L2 ahead changed nothing.)
 //
 // Scheduling as in the tf32 kernel (hpsi_tc.cu): persistent CTAs take tasks
 // from an atomic ticket in the order [z tiles][y tiles][x tiles] per group
@@ -228,19 +228,24 @@ __device__ __forceinline__ void hb_store_a(uint32_t tl, int col, float2 v0, floa
 }
 
 // (D Re, D Im) (+)= A B^T over the six bf16 products, smallest first, each
-// over the K steps
+// over the K steps.  Called by a whole warp, one lane of it issues: the
+// descriptors are then the warp's (computed in one thread they were most of
+// the time between the barriers: Pb208 1.03 ms a call against 0.96)
 template <int N>
-__device__ __forceinline__ void hb_gemm(uint32_t tb, uint32_t bsm, bool accumulate) {
+__device__ __forceinline__ void hb_gemm(uint32_t tb, uint32_t bsm, bool accumulate, bool one) {
   using G = HbGeo<N>;
   constexpr uint32_t idesc = tc::idesc_bf16(128, G::N2);
   constexpr int ap[6] = {4, 2, 0, 2, 0, 0};   // A part (Re; Im is the next part)
   constexpr int bp[6] = {0, 1, 2, 0, 1, 0};   // B tile: 0 h, 1 m, 2 l
   bool first = !accumulate;
+  const uint64_t b0 = tc::sw128_desc(__shfl_sync(0xffffffffu, bsm, 0));
+  tb = __shfl_sync(0xffffffffu, tb, 0);
+  if (!one) return;
 #pragma unroll
   for (int t = 0; t < 6; ++t)
 #pragma unroll
     for (int ks = 0; ks < G::KS; ++ks) {
-      const uint64_t bd = tc::sw128_desc(bsm + bp[t] * G::BTILE + ks * 32);
+      const uint64_t bd = b0 + (bp[t] * G::BTILE + ks * 32) / 16;
       const uint32_t acc = first ? 0u : 1u;
       tc::mma_f16_ta(tb + G::DCOL, tb + ap[t] * G::ACOL + ks * 8, bd, idesc, acc);
       tc::mma_f16_ta(tb + G::DCOL + G::N2, tb + (ap[t] + 1) * G::ACOL + ks * 8, bd, idesc, acc);
@@ -265,6 +270,7 @@ struct HbThread {
   int row, ln, c, g, warp, j0, c0;
   uint32_t tb, tl;
   float kp;
+  bool one;      // the lane that issues for its warp
 };
 
 struct HbShared {
@@ -398,16 +404,16 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
   tc::fence_before();
   __syncthreads();
   // ---- GEMM 1: e = D psi
-  if (threadIdx.x == 0) {
+  if (t.warp == 0) {
     tc::fence_after();
-    if (!b_ready) {
-      // on a timeout b_ready stays false: the exit path waits for the copy
-      if (tc::mbar_wait(&sh.bar_b, 0, a.wait_limit)) b_ready = true;
-      else sh.bad = 1;
-    }
-    if (!sh.bad) {
-      hb_gemm<N>(t.tb, bax, false);
-      tc::mma_commit(&sh.bar_mma);
+    // on a timeout b_ready stays false: the exit path waits for the copy
+    if (!b_ready) b_ready = __all_sync(0xffffffffu, tc::mbar_wait(&sh.bar_b, 0, a.wait_limit));
+    if (!b_ready) sh.bad = 1;
+    __syncwarp();
+    if (b_ready) {
+      hb_gemm<N>(t.tb, bax, false, t.one);
+      if (t.one) tc::mma_commit(&sh.bar_mma);
+      __syncwarp();
       if (!tc::mbar_wait(&sh.bar_mma, phase & 1, a.wait_limit)) sh.bad = 1;
     }
   }
@@ -458,10 +464,13 @@ __device__ __forceinline__ void hb_tile(const HbArgs& a, const HbThread& t, HbSh
   tc::fence_before();
   __syncthreads();
   // ---- GEMM 2: o + D w; a y (x) tile then waits for the z (y) pass of its state
-  if (threadIdx.x == 0) {
+  if (t.warp == 0) {
     tc::fence_after();
-    hb_gemm<N>(t.tb, bax, true);
-    tc::mma_commit(&sh.bar_mma);
+    hb_gemm<N>(t.tb, bax, true, t.one);
+    if (t.one) tc::mma_commit(&sh.bar_mma);
+    __syncwarp();
+  }
+  if (threadIdx.x == 0) {
     if (P > 0 && !hb_wait_count(a.cnt + 3 + 2 * (s - a.s0) + (P - 1), a.cnt + 1, G::T, a.wait_limit)) {
       sh.bad = 1;
       latch_error(a.status, HFB_ERR_TIMEOUT);
@@ -642,6 +651,7 @@ __global__ void __launch_bounds__(kHbThreads, 2) hpsi_bf3_kernel(HbArgs a) {
   t.j0 = t.g * G::PT;
   t.c0 = t.g * (G::PT / 2);
   t.tb = sh.tmem_base;
+  t.one = tc::elect_one();
   t.tl = t.tb + ((uint32_t)(32 * q) << 16);
   const uint32_t bsm = tc::smem_u32(bs);
   float2* ps = reinterpret_cast<float2*>(bs + a.bbytes);
