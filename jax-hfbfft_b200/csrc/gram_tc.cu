@@ -91,6 +91,7 @@ struct TcUnit {
   short row0, col0, cols;      // first stacked row; first column and padded count
   short extra0, extra_n;       // psi rows of S or G that are not columns
   short x0, x_n, xmap;         // rows of lambda or H, and their array
+  int off;                     // of its sums among a slice's: [re, im][128][cols]
   __host__ __device__ int boxes() const {
     return cols / kTcBoxRows + (extra_n + kTcBoxRows - 1) / kTcBoxRows + (x_n + kTcBoxRows - 1) / kTcBoxRows;
   }
@@ -99,7 +100,7 @@ struct TcMaps {
   CUtensorMap m[2][3];         // [isospin][psi, hampsi, hmfpsi]
 };
 struct TcJob {
-  int nunit, slices, kb_total, n3;
+  int nunit, slices, kb_total, n3, slice_sums;
   uint32_t stage_bytes, raw_bytes;
   int raw_stages;
   TcUnit u[kTcMaxUnits];
@@ -418,7 +419,8 @@ gram_tc_kernel(const __grid_constant__ TcJob job, const __grid_constant__ TcMaps
         if (lane == 0) tc::mbar_arrive(&dempty[e % 3]);
       }
       if (ok && !abort_flag) {
-        float* o = part + (((size_t)item * 2 + im) * 128 + qd * 32 + lane) * kTcMaxCols;
+        const TcUnit& U = job.u[item % job.nunit];
+        float* o = part + (size_t)(item / job.nunit) * job.slice_sums + U.off + (im * 128 + qd * 32 + lane) * U.cols;
 #pragma unroll
         for (int g = 0; g < kTcMaxCols / 16; ++g)
           if (g < ng) {
@@ -464,12 +466,12 @@ gram_tc_reduce_kernel(const __grid_constant__ TcJob job, const float* __restrict
 #pragma unroll
   for (int i = 0; i < 8; ++i) s[i] = 0.0;
   if (on) {
-    const float* p = part + ((size_t)blockIdx.y * 2 * 128 + row) * kTcMaxCols + 4 * c4;
+    const float* p = part + U.off + row * U.cols + 4 * c4;
 #pragma unroll 4
     for (int c = sl; c < job.slices; c += kTcRedLanes) {
-      const float* o = p + (size_t)c * job.nunit * 2 * 128 * kTcMaxCols;
+      const float* o = p + (size_t)c * job.slice_sums;
       const float4 re = *reinterpret_cast<const float4*>(o);
-      const float4 im = *reinterpret_cast<const float4*>(o + 128 * kTcMaxCols);
+      const float4 im = *reinterpret_cast<const float4*>(o + 128 * U.cols);
       s[0] += re.x; s[1] += re.y; s[2] += re.z; s[3] += re.w;
       s[4] += im.x; s[5] += im.y; s[6] += im.z; s[7] += im.w;
     }
@@ -534,7 +536,7 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
         for (int col0 = first; col0 < end; col0 += cols) {
           if (job.nunit >= kTcMaxUnits) return HFB_ERR_UNSUPPORTED_GRID;
           TcUnit u{(unsigned char)b, (unsigned char)g, (short)row0, (short)col0,
-                   (short)std::min(cols, (end - col0 + 15) / 16 * 16), 0, 0, 0, 0, 0};
+                   (short)std::min(cols, (end - col0 + 15) / 16 * 16), 0, 0, 0, 0, 0, 0};
           // the vectors j of the block's rows
           const int ja = row0 / nm, jb = (std::min(row0 + 128, n * nm) - 1) / nm;
           const int j0 = g == TC_UPPER ? n - 1 - jb : ja, jn = jb - ja + 1;
@@ -560,9 +562,13 @@ int gram_tc_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const i
   if (job.nunit == 0) return HFB_OK;
   // the widest units first, so that the last items of a launch are short
   std::stable_sort(job.u, job.u + job.nunit, [](const TcUnit& x, const TcUnit& y) { return x.cols > y.cols; });
+  for (int u = 0; u < job.nunit; ++u) {
+    job.u[u].off = job.slice_sums;
+    job.slice_sums += 2 * 128 * job.u[u].cols;
+  }
   job.slices = std::max(1, std::min(kTcMaxSlices, job.kb_total / kTcMinSlice));
   const int items = job.nunit * job.slices, sms = c->sms - leave;
-  float* part = (float*)scratch(c, hfb_ctx_s::S_GRAM, sizeof(float) * (size_t)items * 2 * 128 * kTcMaxCols);
+  float* part = (float*)scratch(c, hfb_ctx_s::S_GRAM, sizeof(float) * (size_t)job.slices * job.slice_sums);
   if (!part) return HFB_ERR_ALLOC;
   int* ticket = c->counters + 1;
   allow_max_dynamic_smem(gram_tc_kernel);
