@@ -16,6 +16,11 @@ __device__ __forceinline__ void cp16(void* smem, const void* gmem, bool ok) {
                "l"(gmem), "r"(ok ? 16 : 0)
                : "memory");
 }
+__device__ __forceinline__ void cp8(void* smem, const void* gmem, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
+               "l"(gmem), "r"(ok ? 8 : 0)
+               : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -43,7 +48,10 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // would fall below 1024 points and its start-up show); they do not depend on
 // which matrices a launch computes, so neither does any sum's order.
 // Measured, S + lambda of Pb208 (140 + 96 states, 48^3): 3.8 ms with 594
-// equal CTAs on 592 places and all of lambda, 2.1 ms here (30 TFLOP/s).
+// equal CTAs on 592 places and all of lambda, 2.1 ms here (30 TFLOP/s).  G's
+// factor v_pair is applied at the fragment loads (multiplied on the way into
+// shared memory, its tiles could not be copied ahead: H + G on 144 SMs 3.3 ms,
+// 2.4 ms here).
 enum { GF_FULL = 0, GF_UPPER = 1, GF_LOWER = 2 };
 
 struct GfGroup {
@@ -89,8 +97,9 @@ template <int GT> struct GfGeo {
   static constexpr int WK = 4 / (WG * WG);          // warps sharing a tile along K
   static constexpr int KB = WG == 2 ? 16 : 32;      // complex k per stage
   static constexpr int LD = KB + 1;                 // rows fall on distinct bank groups
-  static constexpr size_t SMEM = sizeof(double2) * 2 * 2 * GT * LD;
-  static_assert(WK == 1 || sizeof(double2) * WK * GT * GT <= SMEM, "warp sums reuse the stages");
+  static constexpr size_t STAGES = sizeof(double2) * 2 * 2 * GT * LD;
+  static constexpr size_t SMEM = STAGES + sizeof(double) * 2 * KB;   // and v_pair of each stage
+  static_assert(WK == 1 || sizeof(double2) * WK * GT * GT <= STAGES, "warp sums reuse the stages");
 };
 
 template <int GT>
@@ -103,6 +112,7 @@ __device__ __forceinline__ void gf_item(const GfJob& job, size_t K, size_t n3, c
   auto sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(GF_THREADS) : "memory"); };
   double2* As = gf_smem;                 // [2][GT][LD]
   double2* Bs = gf_smem + 2 * GT * LD;
+  double* vs = reinterpret_cast<double*>(Bs + 2 * GT * LD);   // [2][KB]
   const int tile = item % job.ntile, chunk = item / job.ntile;
   int ti, tj;
   const GfGroup gr = gf_tile(job, tile, ti, tj);
@@ -112,7 +122,8 @@ __device__ __forceinline__ void gf_item(const GfJob& job, size_t K, size_t n3, c
   const double2* P = psi + base;
   const double2* X = am == 1 ? hampsi + base : am == 2 ? hmfpsi + base : P;
   const double* vp = job.vp[b];
-  const bool same = am == 0 && ti == tj;   // both operands are the same rows
+  const bool scaled = am == 3;             // by v_pair, at the fragment loads
+  const bool same = (am == 0 || scaled) && ti == tj;   // both operands are the same rows
   const size_t k0 = (size_t)chunk * kchunk;
   const size_t k1 = min(K, k0 + (size_t)kchunk);
   const int lane = tid & 31;
@@ -148,24 +159,16 @@ __device__ __forceinline__ void gf_item(const GfJob& job, size_t K, size_t n3, c
       for (int h = 0; h < NL; ++h) {
         const int gj = j0 + lr + h * RS;
         const bool ok = okk && gj < ns;
-        if (am == 3) {
-          double2 v = make_double2(0.0, 0.0);
-          if (ok) {
-            v = X[(size_t)gj * K + k];
-            const double w = vp[k % n3];
-            v = make_double2(w * v.x, w * v.y);
-          }
-          db[h * RS * LD] = v;
-        } else {
-          cp16(db + h * RS * LD, ok ? X + (size_t)gj * K + k : X, ok);
-        }
+        cp16(db + h * RS * LD, ok ? X + (size_t)gj * K + k : X, ok);
       }
     }
+    if (scaled && lr == 0) cp8(vs + buf * KB + lk, okk ? vp + (k < n3 ? k : k - n3) : vp, okk);
     cp_commit();
   };
   auto stage = [&](int buf, auto tc) {
     constexpr int T = decltype(tc)::value;
     const double* A = reinterpret_cast<const double*>(As + (size_t)buf * GT * LD);
+    const double* V = vs + buf * KB;
     const double* B = same ? A : reinterpret_cast<const double*>(Bs + (size_t)buf * GT * LD);
     constexpr int NS = KB / 2 / G::WK;
     const int ks0 = G::WK == 1 ? 0 : (tid >> 5) * NS;
@@ -178,6 +181,7 @@ __device__ __forceinline__ void gf_item(const GfJob& job, size_t K, size_t n3, c
 #pragma unroll
       for (int v = 0; v < MB; ++v) {
         bv[v] = B[(8 * (MB * cw + v) + fr) * (2 * LD) + kd];
+        if (scaled) bv[v] *= V[kd >> 1];
         const double o = __shfl_xor_sync(0xffffffffu, bv[v], 1);
         bt[v] = (fk & 1) ? -o : o;
       }
