@@ -341,8 +341,8 @@ int hfb_rms_field(hfb_ctx_t ctx, const double* cm, double r0, double scale, doub
 /* Vector-Jacobian products of hpsi and of the densities (the reference
  * differentiates meanfield.py:41-159 and densities.py:237-330 with JAX's
  * reverse mode).  The bilinear form <a|h[P]|b> of hpsi is the integral of
- * each potential field times the pair density of (a, b) that hfb_add_density
- * computes (by polarisation), except for the Nyquist term of cderv02
+ * each potential field times the pair density of (a, b) that
+ * hfb_pair_density computes, except for the Nyquist term of cderv02
  * (levels.py:314-330), -(pi/d)^2 mean_line(B) x_N / n on the Nyquist bin of
  * each line, x_N = sum_j (-1)^j x_j.  These two calls are that term:
  *   hfb_nyquist_pair:  field[iq][r] += sum_ax (pi/d_ax)^2 / n^2 *

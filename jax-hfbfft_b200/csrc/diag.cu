@@ -1041,8 +1041,10 @@ extern "C" int hfb_diagstep(hfb_ctx_t ctx, int prec, const hfb_diag_args* a, voi
   // Pb208 FP64; stream priority did not help, no CTA of the launch ends
   // early), so the H, G launch comes last and leaves four SMs alone: two for
   // the Jacobi solver, one for each isospin's S^-1/2.  The refinement, which
-  // is short, takes its SMs before the launch; the launch's CTAs that do not
-  // fit at once follow it.  Pb208 FP64 iteration: 34.7 ms with the H, G
+  // is short, takes its SMs before the launch: its launch completion event
+  // starts the other stream (from a common event the Gram's CTAs sometimes came
+  // first, and the refinement waited 2.6 ms for them); the launch's CTAs that
+  // do not fit at once follow it.  Pb208 FP64 iteration: 34.7 ms with the H, G
   // launch first, 32.2 ms with it last, 26.5 ms with contract_f64.cu and the
   // free SMs (27.8 ms without them).
   int mask = 1;

@@ -9,8 +9,8 @@ they follow from two exact properties of those discretisations:
   potential field times the matching pair density of (a, b) -- upot: rho,
   bmass: tau, v_pair: 2 chi, aq: current, spot: sdens, wlspot: sodens --
   plus, for bmass, the Nyquist term of cderv02 (levels.py:314-330).  The
-  pair densities come from the density kernel by polarisation,
-  F(a, b) = (F(a + b) - F(a - b)) / 4, each pair first balanced in norm.
+  pair densities come from the density kernel with two operands
+  (hfb_pair_density).
 * The densities are quadratic forms in psi, so their VJP is 2 w h[F_bar] psi
   (+ wu chi_bar psi) with the Nyquist term of the tau cotangent removed.
 
