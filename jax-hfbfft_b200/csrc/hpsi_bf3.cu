@@ -120,15 +120,42 @@ __host__ __device__ __forceinline__ size_t hb_fidx(int L, int j) {
   return ((size_t)(L >> 6) * N + j) * kHbLines + (L & 63);
 }
 
+// First grid point of line L of axis AX (points follow at stride 1, n, n^2
+// for AX = 2, 1, 0).
+template <int N, int AX>
+__host__ __device__ __forceinline__ size_t hb_line_base(int L) {
+  return AX == 2 ? (size_t)L * N : (AX == 1 ? (size_t)(L / N) * N * N + (L % N) : (size_t)L);
+}
+
+// Line means of B for the Nyquist term: bbar[iq][AX][L]
+template <int N>
+__device__ __forceinline__ void hb_mean(const float* __restrict__ pot, float* __restrict__ bbar, int i) {
+  constexpr size_t n3 = (size_t)N * N * N;
+  if (i >= 2 * 3 * N * N) return;
+  const int iq = i / (3 * N * N), ax = (i / (N * N)) % 3, L = i % (N * N);
+  const float* b = pot + ((size_t)iq * 12 + 1) * n3;
+  const size_t base = ax == 2 ? hb_line_base<N, 2>(L) : (ax == 1 ? hb_line_base<N, 1>(L) : hb_line_base<N, 0>(L));
+  const size_t stride = ax == 2 ? 1 : (ax == 1 ? (size_t)N : (size_t)N * N);
+  float s = 0.f;
+  for (int j = 0; j < N; ++j) s += b[base + j * stride];
+  bbar[i] = s * (1.f / N);
+}
+
 // Fields per grid point and pass (current and spin-orbit fields halved, as
 // they enter L_d): x (B, aq_x/2, wl_y/2, wl_z/2), y (B, aq_y/2, wl_x/2,
 // wl_z/2), z (B, aq_z/2, wl_x/2, wl_y/2); local (upot, spot_x, spot_y,
-// spot_z) in the z-pass order.  Also zeroes the scheduling counters.
+// spot_z) in the z-pass order.  Also zeroes the scheduling counters; the first
+// blocks form the line means (a launch of their own before: 5 us with its gap).
 template <int N>
 __global__ void hb_fields_kernel(const float* __restrict__ pot, float4* __restrict__ F, float4* __restrict__ FL,
-                                 int* cnt, int ncnt) {
+                                 float* __restrict__ bbar, int* cnt, int ncnt) {
   constexpr size_t n3 = (size_t)N * N * N;
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  constexpr int MEANS = (6 * N * N + 255) / 256;   // blocks
+  if (blockIdx.x < MEANS) {
+    hb_mean<N>(pot, bbar, blockIdx.x * 256 + threadIdx.x);
+    return;
+  }
+  const size_t i = (blockIdx.x - MEANS) * (size_t)256 + threadIdx.x;
   if (i < (size_t)ncnt) cnt[i] = 0;
   if (i >= 2 * n3) return;
   const int iq = (int)(i / n3);
@@ -142,28 +169,6 @@ __global__ void hb_fields_kernel(const float* __restrict__ pot, float4* __restri
   f[n3 + hb_fidx<N>(x * N + z, y)] = make_float4(bm, 0.5f * p[4 * n3 + g], w0, w2);
   f[2 * n3 + hb_fidx<N>(x * N + y, z)] = make_float4(bm, 0.5f * p[5 * n3 + g], w0, w1);
   FL[(size_t)iq * n3 + hb_fidx<N>(x * N + y, z)] = make_float4(p[g], p[6 * n3 + g], p[7 * n3 + g], p[8 * n3 + g]);
-}
-
-// First grid point of line L of axis AX (points follow at stride 1, n, n^2
-// for AX = 2, 1, 0).
-template <int N, int AX>
-__host__ __device__ __forceinline__ size_t hb_line_base(int L) {
-  return AX == 2 ? (size_t)L * N : (AX == 1 ? (size_t)(L / N) * N * N + (L % N) : (size_t)L);
-}
-
-// Line means of B for the Nyquist term: bbar[iq][AX][L]
-template <int N>
-__global__ void hb_bbar_kernel(const float* __restrict__ pot, float* __restrict__ bbar) {
-  constexpr size_t n3 = (size_t)N * N * N;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * 3 * N * N) return;
-  const int iq = i / (3 * N * N), ax = (i / (N * N)) % 3, L = i % (N * N);
-  const float* b = pot + ((size_t)iq * 12 + 1) * n3;
-  const size_t base = ax == 2 ? hb_line_base<N, 2>(L) : (ax == 1 ? hb_line_base<N, 1>(L) : hb_line_base<N, 0>(L));
-  const size_t stride = ax == 2 ? 1 : (ax == 1 ? (size_t)N : (size_t)N * N);
-  float s = 0.f;
-  for (int j = 0; j < N; ++j) s += b[base + j * stride];
-  bbar[i] = s * (1.f / N);
 }
 
 // L_d of the own component: L_d x_c = i alpha_c x_c + (beta_c + i gamma_c)
@@ -782,9 +787,8 @@ int hpsi_bf3_launch_t(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, 
   float* bbar = reinterpret_cast<float*>(scr + fbytes);
   int* cnt = reinterpret_cast<int*>(scr + fbytes + bbytes_bar);
   const size_t tot = 2 * N3 > (size_t)ncnt ? 2 * N3 : (size_t)ncnt;
-  hb_fields_kernel<N><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>((const float*)pot, F, FL, cnt, ncnt);
-  HFB_CHECK_LAUNCH();
-  hb_bbar_kernel<N><<<(6 * N * N + 255) / 256, 256, 0, st>>>((const float*)pot, bbar);
+  hb_fields_kernel<N><<<(unsigned)((6 * N * N + 255) / 256 + (tot + 255) / 256), 256, 0, st>>>((const float*)pot, F, FL,
+                                                                                            bbar, cnt, ncnt);
   HFB_CHECK_LAUNCH();
   const int slots = 2 * hb_sm_count();
   int group = (slots + G::T / 2) / G::T;
