@@ -15,7 +15,10 @@
 //
 // Units are numbered axis, isospin, tile, state; a CTA (128 threads) takes
 // an equal run of consecutive units whatever the state counts, and writes
-// one partial tile per (axis, isospin, tile) it meets.  A combine kernel adds
+// one partial tile per (axis, isospin, tile) it meets.  Partial tile (CTA k,
+// tile t) lies at k + t: along the units k or t or both step on, so no two
+// share a place, and the buffer holds one tile per CTA and one per tile,
+// whatever the state counts.  A combine kernel adds
 // the partials in order and applies the density mixing of
 // static.py:1820-1823.  (With both components and up to nine accumulators per
 // point in a thread, one CTA per SM, equal chunks of unequal isospins in three
@@ -53,6 +56,7 @@ struct DensGeo {
 // s_z; axis y: tau, current, J parts (two), s_x, s_y; axis z: tau, current,
 // J parts (two).
 constexpr int kDensFields = 7;
+constexpr int kDensPerSm = 4;   // CTAs of an SM that write partial tiles, at most
 
 // How the units are cut up, and where a partial tile lies.
 struct DensCut {
@@ -60,9 +64,12 @@ struct DensCut {
   int iq[2], s0[2], cnt[2]; // isospin, first state, states of each
   int ntile, nst;
   long units, run;          // all units; units per CTA
-  int segs;                 // partial tiles a CTA can write at most
 };
-// first unit of (axis, block, tile), and its number among all tiles
+// number of (axis, block, tile) among all tiles
+__host__ __device__ __forceinline__ long dens_tile(const DensCut& c, int axis, int q, int tile) {
+  return ((long)axis * c.nq + q) * c.ntile + tile;
+}
+// and its first unit
 __host__ __device__ __forceinline__ long dens_first(const DensCut& c, int axis, int q, int tile) {
   return (long)axis * c.ntile * c.nst + (q ? (long)c.ntile * c.cnt[0] : 0) + (long)tile * c.cnt[q];
 }
@@ -285,12 +292,12 @@ density_kernel(const __grid_constant__ DensArgs a) {
   const DensCut& cut = a.cut;
   long u = (long)blockIdx.x * cut.run;
   const long end = min(cut.units, u + cut.run);
-  for (int seg = 0; u < end; ++seg) {
+  while (u < end) {
     int axis, q, tile, s;
     dens_decode(cut, u, axis, q, tile, s);
     const int n = (int)min((long)(cut.cnt[q] - s), end - u);
     const int sa = cut.s0[q] + s;
-    double* out = a.part + ((size_t)blockIdx.x * cut.segs + seg) * kDensFields * G::L * N;
+    double* out = a.part + (blockIdx.x + (size_t)dens_tile(cut, axis, q, tile)) * kDensFields * G::L * N;
     if (axis == 0) dens_segment<R, N, 0, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
     else if (axis == 1) dens_segment<R, N, 1, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
     else dens_segment<R, N, 2, KIND>(a, tile, sa, sa + n, out, xb, tw, sk);
@@ -324,12 +331,9 @@ density_combine_kernel(DensCut cut, const double* __restrict__ part, double mix,
       const int tile = line / L, l = line % L;
       const int off = ax == 2 ? l * N + j : j * L + l;
       const long u0 = dens_first(cut, ax, q, tile), u1 = u0 + cut.cnt[q];
-      const long id = ((long)ax * cut.nq + q) * cut.ntile + tile;   // number of the tile
+      const long id = dens_tile(cut, ax, q, tile);
       for (long k = u0 / cut.run; k <= (u1 - 1) / cut.run; ++k) {
-        int a0, q0, t0, s0;
-        dens_decode(cut, k * cut.run, a0, q0, t0, s0);               // where CTA k starts
-        const long seg = id - (((long)a0 * cut.nq + q0) * cut.ntile + t0);
-        const double* p = part + ((size_t)k * cut.segs + seg) * kDensFields * FS + off;
+        const double* p = part + (size_t)(k + id) * kDensFields * FS + off;
         constexpr int NF[3] = {7, 6, 4};
 #pragma unroll
         for (int g = 0; g < NF[ax]; ++g) f[ax][g] += p[g * FS];
@@ -384,12 +388,13 @@ struct DensOut {
 template <class R, int N, int KIND>
 int density_launch_t(hfb_ctx_s* c, DensArgs a, int nst, int nneut, const DensOut& o, cudaStream_t st) {
   using G = DensGeo<R, N>;
-  // CTAs that are resident together
+  // CTAs that are resident together (those that write partial tiles never
+  // exceed kDensPerSm: their registers)
   static const int per_sm = [] {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, density_kernel<R, N, KIND>, G::THREADS, 0) != cudaSuccess)
       cudaGetLastError();
-    return n > 0 ? n : 1;
+    return n < 1 ? 1 : KIND != DENS_KINETIC && n > kDensPerSm ? kDensPerSm : n;
   }();
   DensCut cut{};
   nneut = nneut < 0 ? 0 : nneut > nst ? nst : nneut;
@@ -408,13 +413,14 @@ int density_launch_t(hfb_ctx_s* c, DensArgs a, int nst, int nneut, const DensOut
   const long places = (long)per_sm * c->sms;
   cut.run = (cut.units + places - 1) / places;
   if (cut.run < 2) cut.run = 2;
-  const int least = cut.nq > 1 && cut.cnt[1] < cut.cnt[0] ? cut.cnt[1] : cut.cnt[0];
-  cut.segs = (int)((cut.run + least - 2) / least + 1);
   const long ctas = (cut.units + cut.run - 1) / cut.run;
   a.cut = cut;
   a.part = nullptr;
   if (KIND != DENS_KINETIC) {
-    a.part = (double*)scratch(c, hfb_ctx_s::S_DENS, sizeof(double) * (size_t)ctas * cut.segs * kDensFields * G::L * N);
+    // one size for all state counts, precisions and kinds: the buffer is not
+    // moved under a captured graph
+    const size_t tiles = (size_t)kDensPerSm * c->sms + 3 * 2 * G::NTILE;
+    a.part = (double*)scratch(c, hfb_ctx_s::S_DENS, sizeof(double) * tiles * kDensFields * G::L * N);
     if (!a.part) return HFB_ERR_ALLOC;
   }
   a.kin = nullptr;

@@ -1,0 +1,93 @@
+"""The library's host code on the CPU, against a stand-in for the CUDA runtime
+(fake_cudart.c, preloaded into a child process): how much scratch a call
+takes, which calls allocate at all, and what a launch needs to have been set
+on its device.  No kernel runs, and none needs a GPU."""
+import ctypes as C
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+F64, F32 = 0, 1   # HFB_F64, HFB_F32
+
+
+# ------------------------------------------------------------- scenarios ----
+# each runs in a child process with the stand-in preloaded; its return value
+# is printed
+class _Lib:
+    def __init__(self):
+        sys.path.insert(0, os.path.join(os.path.dirname(HERE), "jax-hfbfft_b200", "hfb"))
+        import types
+        sys.modules.setdefault("torch", types.ModuleType("torch"))   # only the prototypes are needed
+        import _lib
+        self.hfb, self.fake = _lib.load(), C.CDLL(None)
+        self.fake.fake_bytes.restype = C.c_ulonglong
+        self.fake.fake_widest_cluster.restype = self.fake.fake_allocs.restype = C.c_long
+        self.fake.fake_launches.restype = C.c_long
+        assert self.fake.fake_launches() == 0
+        self.mem = C.create_string_buffer(1 << 16)
+        self.p = (C.addressof(self.mem) + 255) & ~255   # any device address: nothing is read
+
+    def ctx(self, n):
+        h = C.c_void_p()
+        assert self.hfb.hfb_ctx_create(n, n, n, 1.0, 1.0, 1.0, 0, 0, C.byref(h)) == 0
+        return h
+
+    def add_density(self, ctx, prec, nst, nneut):
+        p = self.p
+        return self.hfb.hfb_add_density(ctx, prec, nst, nneut, p, p, p, p, p, 1.0, p, p, p, p, p, p, None, None, None)
+
+    def pair_density(self, ctx, prec, nst, nneut):
+        return self.hfb.hfb_pair_density(ctx, prec, nst, nneut, *[self.p] * 10, None)
+
+
+def density_scratch():
+    lib = _Lib()
+    ctx = lib.ctx(16)
+    b0 = lib.fake.fake_bytes()
+    rc = [lib.add_density(ctx, F64, 601, 1)]
+    taken, a0 = lib.fake.fake_bytes() - b0, lib.fake.fake_allocs()
+    for prec in (F64, F32):
+        for nst, nneut in ((20, 10), (300, 299), (900, 450)):
+            rc += [lib.add_density(ctx, prec, nst, nneut), lib.pair_density(ctx, prec, nst, nneut)]
+    return rc, taken, lib.fake.fake_allocs() - a0
+
+
+# ----------------------------------------------------------------- tests ----
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I", "/usr/local/cuda/include",
+                    os.path.join(HERE, "fake_cudart.c"), "-o", so], check=True)
+    sys.path.insert(0, os.path.join(os.path.dirname(HERE), "jax-hfbfft_b200"))
+    import build
+    if not os.path.exists(build.OUT):
+        build.build()
+
+    def run(name):
+        env = {k: v for k, v in os.environ.items() if not k.startswith("HFB_")}
+        env["LD_PRELOAD"] = so
+        r = subprocess.run([sys.executable, os.path.abspath(__file__), name], env=env, capture_output=True, text=True,
+                           timeout=120)
+        assert r.returncode == 0, r.stderr
+        import ast
+        return ast.literal_eval(r.stdout.strip().splitlines()[-1])
+    return run
+
+
+def test_density_scratch_does_not_grow_with_the_states(child):
+    """At most one partial tile per CTA (four an SM) and one per (axis,
+    isospin, tile), whatever the state counts: at 16^3, with tiles of 16 lines
+    and 7 fields, (4 * 148 + 6 * 16) * 7 * 16 * 16 * 8 bytes and the arena's
+    eighth on top, 11.1 MB.  A later call with other counts, in the other
+    precision or for pairs finds the buffer large enough."""
+    rc, taken, later = child("density_scratch")
+    assert set(rc) == {0}
+    assert taken <= 12e6
+    assert later == 0
+
+
+if __name__ == "__main__":
+    print(repr(globals()[sys.argv[1]]()))
