@@ -55,6 +55,18 @@ def density_scratch():
     return rc, taken, lib.fake.fake_allocs() - a0
 
 
+def nyquist_scratch():
+    lib = _Lib()
+    ctx, p = lib.ctx(16), lib.p
+    a0 = lib.fake.fake_allocs()
+    rc = [lib.hfb.hfb_nyquist_apply(ctx, prec, 40, 20, p, p, p, p + 256, None) for prec in (F64, F32)]
+    applied = lib.fake.fake_allocs() - a0
+    rc += [lib.hfb.hfb_nyquist_pair(ctx, F64, 5, 3, p, p, p, p, None)]
+    a0 = lib.fake.fake_allocs()
+    rc += [lib.hfb.hfb_nyquist_pair(ctx, prec, 400, 3, p, p, p, p, None) for prec in (F64, F32)]
+    return rc, applied, lib.fake.fake_allocs() - a0
+
+
 # ----------------------------------------------------------------- tests ----
 @pytest.fixture(scope="module")
 def child(tmp_path_factory):
@@ -86,6 +98,15 @@ def test_density_scratch_does_not_grow_with_the_states(child):
     rc, taken, later = child("density_scratch")
     assert set(rc) == {0}
     assert taken <= 12e6
+    assert later == 0
+
+
+def test_nyquist_calls_do_not_allocate_with_the_states(child):
+    """hfb_nyquist_apply takes no scratch, so it may be a context's first call
+    inside a capture; hfb_nyquist_pair's has one size."""
+    rc, applied, later = child("nyquist_scratch")
+    assert set(rc) == {0}
+    assert applied == 0
     assert later == 0
 
 
