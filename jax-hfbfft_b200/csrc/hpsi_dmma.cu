@@ -472,11 +472,12 @@ int hpsi_dmma_launch_t(hfb_ctx_s* c, HdArgs a, cudaStream_t st) {
   const long items = (long)a.ns * N, places = (long)G::CTAS * c->sms;
   const unsigned grid = (unsigned)(items < places ? items : places);
   // a table of the line means (one launch, about 8 us with its gap) pays from
-  // a few planes a CTA on (about 1 us each without it)
+  // a few planes a CTA on (about 1 us each without it).  It lies behind the
+  // derivative matrices: in the arena's slot, which the single-precision
+  // kernels grow, it could move under a captured graph.
   a.bbar = nullptr;
   if (items > 8 * places) {
-    double* bbar = (double*)scratch(c, hfb_ctx_s::S_HPT, sizeof(double) * 6 * N * N);
-    if (!bbar) return HFB_ERR_ALLOC;
+    double* bbar = c->hpsi_d64 + 3 * G::DSZ;
     hd_bbar_kernel<<<dim3((N * N + 127) / 128, 3, 2), 128, 0, st>>>(N, a.pot, bbar);
     HFB_CHECK_LAUNCH();
     a.bbar = bbar;
@@ -516,7 +517,8 @@ int hpsi_dmma_prepare(hfb_ctx_s* c) {
           d[(size_t)ax * G::DSZ + (G::HP + j) * G::LDH + l] = 0.5 * (p + q);
         }
     }
-    if (cudaMalloc(&c->hpsi_d64, d.size() * sizeof(double)) != cudaSuccess) {
+    // and room for the line means of a launch, [2][3][n^2]
+    if (cudaMalloc(&c->hpsi_d64, (d.size() + 6 * N * N) * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       c->hpsi_d64 = nullptr;
       return HFB_ERR_ALLOC;

@@ -38,8 +38,8 @@ __device__ __forceinline__ LineGeo line_geo(int n, int ax, int line) {
 // The sums over a line, sum_j (-1)^j x_j, are formed for every line and for
 // runs of an isospin's states at once (one thread each): with all the states of
 // an isospin in one loop, 24 blocks did it all (532 us for 70 states at 32^3;
-// 64 us here, lines and their sum).  At most kVjGroups runs an isospin, so that their sums have
-// one size whatever the state count.
+// 64 us here, lines and their sum).  At most kVjGroups runs an isospin, so that
+// their sums have one size whatever the state count.
 constexpr int kVjGroups = 64;
 struct VjRuns {
   int first[2], end[2], run[2], groups[2];   // states of each isospin, states a run, runs

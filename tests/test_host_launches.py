@@ -67,6 +67,14 @@ def nyquist_scratch():
     return rc, applied, lib.fake.fake_allocs() - a0
 
 
+def hpsi_f64_scratch():
+    lib = _Lib()
+    ctx, p = lib.ctx(48), lib.p
+    a0 = lib.fake.fake_allocs()
+    rc = [lib.hfb.hfb_hpsi(ctx, F64, p, nst, 1, p, p, p, p, p, p, None) for nst in (1, 60, 236)]
+    return rc, lib.fake.fake_allocs() - a0
+
+
 # ----------------------------------------------------------------- tests ----
 @pytest.fixture(scope="module")
 def child(tmp_path_factory):
@@ -108,6 +116,14 @@ def test_nyquist_calls_do_not_allocate_with_the_states(child):
     assert set(rc) == {0}
     assert applied == 0
     assert later == 0
+
+
+def test_hpsi_f64_takes_no_scratch(child):
+    """With few planes a CTA and with many (the table of line means): what a
+    capture holds is not moved by a later single-precision call."""
+    rc, allocs = child("hpsi_f64_scratch")
+    assert set(rc) == {0}
+    assert allocs == 0
 
 
 if __name__ == "__main__":
