@@ -739,7 +739,7 @@ static int eigh_refine(hfb_ctx_s* c, int nb, Pair2 nper, int ld, const double2* 
   if (!buf) return HFB_ERR_ALLOC;
   int* fallback = (int*)(buf + wb);
   const RefineArgs a{nper, ld, A, sA, W, sW, V, sV, tol_rel > 0.0 ? tol_rel : 1e-13, fallback};
-  const int r = refine_launch(nb, a, buf, begun, st);
+  const int r = refine_launch(c, nb, a, buf, begun, st);
   if (r) return r;
   EighBatch eb{};
   eb.tol_rel = tol_rel;

@@ -40,7 +40,8 @@ struct RefineArgs {
   int* fallback;      // [nb]: set when the refinement does not apply to matrix b
 };
 size_t refine_bytes(int nb, int ld);
-int refine_launch(int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st);   // begun: every CTA runs (or null)
+// begun: recorded once every CTA runs (or null)
+int refine_launch(hfb_ctx_s* c, int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st);
 
 struct LoewdinArgs {
   Pair2 nper, off;

@@ -793,7 +793,31 @@ size_t refine_bytes(int nb, int ld) {
          sizeof(double) * ((size_t)nb * ld + 12 * kClMax) + sizeof(int) * (size_t)nb * ld * 4;
 }
 
-int refine_launch(int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st) {
+// Largest cluster of the refinement on the context's device: 16 CTAs, which the
+// kernel has to be allowed on each device, or 8 where those are refused or no
+// 16 SMs of a cluster are free to the process.  Asked once per context.
+static int refine_widest(hfb_ctx_s* c) {
+  if (c->refine_ctas) return c->refine_ctas;
+  c->refine_ctas = 8;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClMax;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kClMax);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int places = 0;
+  if (cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&places, refine_kernel, &cfg) != cudaSuccess)
+    cudaGetLastError();
+  else if (places > 0)
+    c->refine_ctas = kClMax;
+  return c->refine_ctas;
+}
+
+int refine_launch(hfb_ctx_s* c, int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cudaStream_t st) {
   if (a.ld > kRefMaxN) return HFB_ERR_UNSUPPORTED_GRID;
   const size_t sm = (size_t)nb * a.ld * a.ld;
   double2* m = (double2*)work;
@@ -803,10 +827,10 @@ int refine_launch(int nb, const RefineArgs& a, void* work, cudaEvent_t begun, cu
   double* d = (double*)(w.Q + (size_t)nb * a.ld * kClusterMax);
   w.ev = d; w.slots = d + (size_t)nb * a.ld;
   w.cinfo = (int*)(w.slots + 12 * kClMax);
-  static const bool wide =
-      cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
   const int n = nb > 1 ? max2(a.nper) : a.nper.v[0];
-  return cluster_launch(refine_kernel, 1, cluster_size(n, wide ? 16 : 8), begun, st, a, w, nb);
+  int size = cluster_size(n, kClMax);
+  if (size > 8) size = refine_widest(c);
+  return cluster_launch(refine_kernel, 1, size, begun, st, a, w, nb);
 }
 
 size_t construct_bytes(int ld) { return sizeof(double2) * 2 * 2 * (size_t)ld * ld + sizeof(double) * 2 * 4 * kClMax; }

@@ -25,6 +25,7 @@ struct hfb_ctx_s {
                          // HFB_NO_TCGEN05=1 in the environment at creation selects CUDA cores)
   int lambda_refine;     // FP64 diagstep diagonalises lambda by eigen refinement (default 1;
                          // HFB_LAMBDA_JACOBI=1 at creation selects the Jacobi solver)
+  int refine_ctas;       // its largest cluster on this device (0: not asked yet)
   cudaEvent_t ev_fork, ev_join;
   cudaStream_t side2;    // a second one (Newton-Schulz beside the eigensolve and the H, G Gram)
   cudaEvent_t ev_fork2, ev_join2;

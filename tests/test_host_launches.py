@@ -75,6 +75,21 @@ def hpsi_f64_scratch():
     return rc, lib.fake.fake_allocs() - a0
 
 
+def clusters():
+    lib = _Lib()
+    p, out = lib.p, []
+    eigh = lambda ctx, n: lib.hfb.hfb_eigh_near_diagonal(ctx, 2, n, n, p, p, p, None)  # noqa: E731
+    for device in (0, 1):
+        lib.fake.fake_set_device(device)
+        ctx = lib.ctx(8)
+        out += [(eigh(ctx, 80), lib.fake.fake_widest_cluster()), (eigh(ctx, 100), lib.fake.fake_widest_cluster())]
+    lib.fake.fake_cluster_places(0)          # no place for a cluster of 16
+    out.append((eigh(lib.ctx(8), 100), lib.fake.fake_widest_cluster()))
+    lib.fake.fake_attribute_fails(1)         # the opt-in is refused
+    out.append((eigh(lib.ctx(8), 100), lib.fake.fake_widest_cluster()))
+    return out
+
+
 # ----------------------------------------------------------------- tests ----
 @pytest.fixture(scope="module")
 def child(tmp_path_factory):
@@ -124,6 +139,12 @@ def test_hpsi_f64_takes_no_scratch(child):
     rc, allocs = child("hpsi_f64_scratch")
     assert set(rc) == {0}
     assert allocs == 0
+
+
+def test_refinement_cluster_on_every_device(child):
+    """The opt-in to 16 CTAs (from 81 states on) holds for one device; where it
+    is refused or such a cluster has no place, 8 do."""
+    assert child("clusters") == [(0, 8), (0, 16)] * 2 + [(0, 8), (0, 8)]
 
 
 if __name__ == "__main__":
