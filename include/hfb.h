@@ -112,7 +112,10 @@ int hfb_laplace(hfb_ctx_t ctx, int prec, int nsp, const void* psin, const double
 /* ---- meanfield.py ------------------------------------------------------ */
 /* hpsi01 (meanfield.py:41-159) batched over nst states; state s uses the
  * potentials of isospin (s >= nneut).  Any of pout / pout_mf / pout_del may
- * be NULL except that one of pout / pout_mf is required. */
+ * be NULL except that one of pout / pout_mf is required.  psi and the array
+ * that takes h psi (pout_mf, or pout without it) lie on 16-byte boundaries
+ * (single precision on CUDA cores: 8), else HFB_ERR_ARG; so do psi, hampsi
+ * and hmfpsi of hfb_grstep. */
 int hfb_hpsi(hfb_ctx_t ctx, int prec, const void* pot, int nst, int nneut, const void* psi,
              const double* weight, const double* weightuv, void* pout, void* pout_mf,
              void* pout_del, void* stream);

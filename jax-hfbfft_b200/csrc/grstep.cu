@@ -442,6 +442,7 @@ extern "C" int hfb_laplace(hfb_ctx_t ctx, int prec, int nsp, const void* psin, c
 
 extern "C" int hfb_grstep(hfb_ctx_t ctx, int prec, const hfb_grstep_args* a, void* stream) {
   if (!ctx || !a || !a->psi || !a->hampsi || !a->hmfpsi || !a->pot || !a->sp_energy) return HFB_ERR_ARG;
+  if (!hpsi_aligned(ctx, prec, a->psi, a->hampsi) || !hpsi_aligned(ctx, prec, a->psi, a->hmfpsi)) return HFB_ERR_ARG;
   cudaStream_t st = as_stream(stream);
   const int ns = a->nst, n = ctx->n;
   if (ns <= 0) return HFB_OK;

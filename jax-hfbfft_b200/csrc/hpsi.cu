@@ -326,6 +326,11 @@ int hpsi_launch_t(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, cons
   return HFB_OK;
 }
 
+bool hpsi_aligned(hfb_ctx_s* c, int prec, const void* psi, const void* acc) {
+  const bool fft = prec != HFB_F64 && !hpsi_bf3_available(c, prec) && !hpsi_tc_available(c, prec);
+  return (((uintptr_t)psi | (uintptr_t)acc) & (fft ? 7 : 15)) == 0;
+}
+
 int hpsi_ovl_parts(hfb_ctx_s* c, int prec) {
   if (hpsi_bf3_available(c, prec)) return hpsi_bf3_parts(c);
   return hpsi_tc_available(c, prec) ? hpsi_tc_parts(c) : c->n;
@@ -358,6 +363,7 @@ extern "C" int hfb_hpsi(hfb_ctx_t ctx, int prec, const void* pot, int nst, int n
   if (prec != HFB_F64 && prec != HFB_F32) return HFB_ERR_ARG;
   // pout_mf doubles as the accumulator; without it the pout buffer is used.
   void* acc = pout_mf ? pout_mf : pout;
+  if (!hfb::hpsi_aligned(ctx, prec, psi, acc)) return HFB_ERR_ARG;
   return hfb::hpsi_launch(ctx, prec, pot, 0, nst, nneut, psi, weight, weightuv, acc, pout, pout_mf, pout_del, nullptr,
                           hfb::as_stream(stream));
 }

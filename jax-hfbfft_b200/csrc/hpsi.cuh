@@ -38,6 +38,12 @@ int hpsi_dmma_launch(hfb_ctx_s* c, const void* pot, int s0, int ns, int nneut, c
                      const double* weightuv, void* acc, void* pout, void* pout_mf, void* pout_del, double* ovl,
                      cudaStream_t st);
 
+// Whether the kernel that hpsi_launch runs may take these addresses: the
+// tensor-core kernels copy two single-precision points, or one double-precision
+// one, at a time (16 bytes).  Asked at the library's entries, before any launch:
+// choosing another kernel inside hpsi_launch would change hpsi_ovl_parts.
+bool hpsi_aligned(hfb_ctx_s* c, int prec, const void* psi, const void* acc);
+
 // Partial sums per state that hpsi_launch writes into ``ovl``.
 int hpsi_ovl_parts(hfb_ctx_s* c, int prec);
 

@@ -7,7 +7,7 @@ from dataclasses import dataclass
 
 import torch
 
-from ._lib import call, ptr, stream_ptr, prec_of, HFB_F64, HFB_F32
+from ._lib import aligned, call, ptr, stream_ptr, prec_of, HFB_F64, HFB_F32
 
 
 @dataclass
@@ -57,7 +57,7 @@ def init_meanfield(grids, dtype=torch.complex128):
 def hpsi01(grids, meanfield, iq, weight, weightuv, pinn):
     """h_q on a 2-spinor or a batch of spinors of one isospin
     (meanfield.py:41-159).  Returns ``(pout, pout_mf, pout_del)``."""
-    x = pinn.contiguous()
+    x = aligned(pinn.contiguous())
     nst = x.numel() // (2 * grids.n3)
     rd = torch.float64 if x.dtype == torch.complex128 else torch.float32
     if meanfield.pot.dtype != rd:

@@ -31,7 +31,7 @@ from types import SimpleNamespace
 
 import torch
 
-from ._lib import call, ptr, stream_ptr, prec_of, HFB_F64, HFB_F32
+from ._lib import aligned, call, ptr, stream_ptr, prec_of, HFB_F64, HFB_F32
 
 _FIELDS = ("upot", "bmass", "v_pair", "aq", "spot", "wlspot")
 _DENS = ("rho", "chi", "tau", "current", "sdens", "sodens")
@@ -88,6 +88,7 @@ def _pack(grids, fields, dtype):
 
 
 def _hpsi(grids, pot, x, nneut, w, wu):
+    x = aligned(x)
     out = torch.empty_like(x)
     call("hfb_hpsi", grids.ctx.handle, prec_of(x), ptr(pot), x.shape[0], nneut, ptr(x), ptr(w), ptr(wu), ptr(out),
          None, None, stream_ptr())

@@ -90,6 +90,34 @@ def clusters():
     return out
 
 
+def hpsi_alignment():
+    lib = _Lib()
+    p, out = lib.p, []
+    from _lib import GrstepArgs
+    ctx = lib.ctx(24)
+
+    def hpsi(kind, prec, psi, pout, mf):
+        lib.hfb.hfb_set_hpsi_kernel(ctx, kind)
+        n0 = lib.fake.fake_launches()
+        r = lib.hfb.hfb_hpsi(ctx, prec, p, 2, 1, psi, None, None, pout, mf, None, None)
+        return r, lib.fake.fake_launches() - n0 > 0
+
+    for kind in (0, 1, 2):
+        out.append([hpsi(kind, F32, p, p + 8, p), hpsi(kind, F32, p + 8, p, p), hpsi(kind, F32, p, p + 8, None),
+                    hpsi(kind, F32, p, p, p + 8)])
+    out.append([hpsi(0, F64, p, p, p), hpsi(0, F64, p + 8, p, p)])
+    steps = []
+    for off in ("psi", "hampsi", "hmfpsi", None):
+        a = GrstepArgs()
+        for f, t in a._fields_:
+            if t is C.c_void_p:
+                setattr(a, f, p + 8 * (f == off))
+        a.nst, a.nneut, a.e0dmp = 2, 1, 100.0
+        n0 = lib.fake.fake_launches()
+        steps.append((lib.hfb.hfb_grstep(ctx, F32, C.byref(a), None), lib.fake.fake_launches() - n0 > 0))
+    return out, steps
+
+
 # ----------------------------------------------------------------- tests ----
 @pytest.fixture(scope="module")
 def child(tmp_path_factory):
@@ -145,6 +173,17 @@ def test_refinement_cluster_on_every_device(child):
     """The opt-in to 16 CTAs (from 81 states on) holds for one device; where it
     is refused or such a cluster has no place, 8 do."""
     assert child("clusters") == [(0, 8), (0, 16)] * 2 + [(0, 8), (0, 8)]
+
+
+def test_misaligned_states_are_refused_before_any_launch(child):
+    """16 bytes for psi and for the array that takes h psi; any address of a
+    float2 for the other outputs and for the kernel on CUDA cores."""
+    ok, bad = (0, True), (1, False)
+    out, steps = child("hpsi_alignment")
+    assert out[0] == out[1] == [ok, bad, bad, bad]
+    assert out[2] == [ok, ok, ok, ok]
+    assert out[3] == [ok, bad]
+    assert steps == [bad, bad, bad, ok]
 
 
 if __name__ == "__main__":
