@@ -181,13 +181,13 @@ def ptr(t):
     return t.data_ptr()
 
 
-def launch_count():
 def aligned(t):
     """``t``, or a copy of it when its data is off a 16-byte boundary (a view
     of single-precision states may be)."""
     return t.clone() if t.data_ptr() % 16 else t
 
 
+def launch_count():
     """Kernels launched by libhfb in this process so far."""
     return int(load().hfb_launch_count())
 
