@@ -265,6 +265,11 @@ int hfb_eigh(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w, 
  * eigh of static.py:300-310 / 397-407. */
 int hfb_eigh_near_diagonal(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w,
                            double* v, void* stream);
+/* The same; jacobi (optional device int[nb]) tells which solver gave each
+ * matrix: 0 the refinement, 1 the Jacobi solver.  Matrices are taken two at a
+ * time and share the choice. */
+int hfb_eigh_near_diagonal_info(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w,
+                                double* v, int* jacobi, void* stream);
 
 /* lastdiag (static.py:1072-1168): quasiparticle spectrum of one isospin
  * block after convergence.  hmatrix and gapmatrix are complex [nst][ldh]

@@ -730,14 +730,15 @@ int zgemm_small_one(int n, int ld, int ta, int tb, const double2* A, const doubl
 // Eigenpairs of up to two nearly diagonal Hermitian matrices (lower
 // triangles at A + b sA, leading dimension ld): w ascending at W + b sW,
 // eigenvectors in the columns of V + b sV, by refinement (diag_cluster.cu);
-// Jacobi for the matrices it does not apply to.
+// Jacobi for the matrices it does not apply to.  ``jacobi`` (optional, device
+// [nb]) receives 1 where that was so, else 0.
 static int eigh_refine(hfb_ctx_s* c, int nb, Pair2 nper, int ld, const double2* A, size_t sA, double* W, size_t sW,
                        double2* V, size_t sV, double tol_rel, cudaStream_t st,
-                       cudaEvent_t begun = nullptr) {
+                       cudaEvent_t begun = nullptr, int* jacobi = nullptr) {
   const size_t wb = (refine_bytes(nb, ld) + 15) / 16 * 16;
   char* buf = (char*)scratch(c, hfb_ctx_s::S_EIG, wb + sizeof(int) * nb);
   if (!buf) return HFB_ERR_ALLOC;
-  int* fallback = (int*)(buf + wb);
+  int* fallback = jacobi ? jacobi : (int*)(buf + wb);
   const RefineArgs a{nper, ld, A, sA, W, sW, V, sV, tol_rel > 0.0 ? tol_rel : 1e-13, fallback};
   const int r = refine_launch(c, nb, a, buf, begun, st);
   if (r) return r;
@@ -988,6 +989,11 @@ extern "C" int hfb_eigh(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, 
 
 extern "C" int hfb_eigh_near_diagonal(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w,
                                       double* v, void* stream) {
+  return hfb_eigh_near_diagonal_info(ctx, nb, n, lda, a, w, v, nullptr, stream);
+}
+
+extern "C" int hfb_eigh_near_diagonal_info(hfb_ctx_t ctx, int nb, int n, int lda, const double* a, double* w,
+                                           double* v, int* jacobi, void* stream) {
   if (!ctx || !a || !w || !v || n <= 0 || lda < n || nb <= 0) return HFB_ERR_ARG;
   if (lda > 256) return HFB_ERR_UNSUPPORTED_GRID;
   cudaStream_t st = as_stream(stream);
@@ -998,7 +1004,7 @@ extern "C" int hfb_eigh_near_diagonal(hfb_ctx_t ctx, int nb, int n, int lda, con
     nper.v[0] = n;
     nper.v[1] = cnt > 1 ? n : 0;
     int r = eigh_refine(ctx, cnt, nper, lda, (const double2*)a + b0 * mstride, mstride, w + (size_t)b0 * n, n,
-                        (double2*)v + b0 * mstride, mstride, 0.0, st);
+                        (double2*)v + b0 * mstride, mstride, 0.0, st, nullptr, jacobi ? jacobi + b0 : nullptr);
     if (r) return r;
   }
   return HFB_OK;

@@ -98,6 +98,7 @@ _PROTOS = {
     "hfb_gram": [vp, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, C.c_double, vp, vp],
     "hfb_eigh": [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp],
     "hfb_eigh_near_diagonal": [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp],
+    "hfb_eigh_near_diagonal_info": [vp, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp],
     "hfb_pair": [vp, C.POINTER(PairArgs), vp],
     "hfb_lastdiag": [vp, C.c_int, C.c_int, vp, vp, vp, vp, C.c_int, vp, vp, vp],
     "hfb_natural_begin": [vp, C.POINTER(NaturalArgs), vp],
