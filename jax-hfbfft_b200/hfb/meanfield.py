@@ -57,9 +57,11 @@ def init_meanfield(grids, dtype=torch.complex128):
 def hpsi01(grids, meanfield, iq, weight, weightuv, pinn):
     """h_q on a 2-spinor or a batch of spinors of one isospin
     (meanfield.py:41-159).  Returns ``(pout, pout_mf, pout_del)``."""
-    x = aligned(pinn.contiguous())
+    x = pinn.contiguous()
     nst = x.numel() // (2 * grids.n3)
     rd = torch.float64 if x.dtype == torch.complex128 else torch.float32
+    if rd == torch.float32:
+        x = aligned(x)
     if meanfield.pot.dtype != rd:
         meanfield.pack(x.dtype)
     dev = x.device

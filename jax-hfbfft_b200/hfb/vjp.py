@@ -88,9 +88,11 @@ def _pack(grids, fields, dtype):
 
 
 def _hpsi(grids, pot, x, nneut, w, wu):
-    x = aligned(x)
+    prec = prec_of(x)
+    if prec == HFB_F32:
+        x = aligned(x)
     out = torch.empty_like(x)
-    call("hfb_hpsi", grids.ctx.handle, prec_of(x), ptr(pot), x.shape[0], nneut, ptr(x), ptr(w), ptr(wu), ptr(out),
+    call("hfb_hpsi", grids.ctx.handle, prec, ptr(pot), x.shape[0], nneut, ptr(x), ptr(w), ptr(wu), ptr(out),
          None, None, stream_ptr())
     return out
 
