@@ -142,10 +142,11 @@ int hfb_poisson(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream)
  * library allocate: applications whose device memory is entirely owned by
  * their own pool allocator, and latency-critical loops where an allocation
  * and the synchronisation it implies would stall.  The work buffer is a
- * fixed 4 MiB array inside the library (64^3 complex doubles), so the
- * Coulomb grid n2 must be at most 64^3: n <= 32 for a non-periodic grid
- * (n2 = 2n); every periodic grid a context accepts (n2 = n <= 48) fits.
- * Larger Coulomb grids return HFB_ERR_UNSUPPORTED_GRID.  Call it with the context's device current
+ * fixed 1 MiB array inside the library, the half spectrum of a 32^3 density
+ * on the doubled grid, so the Coulomb grid n2 must be at most 64^3: n <= 32
+ * for a non-periodic grid (n2 = 2n); every periodic grid a context accepts
+ * (n2 = n <= 48) fits.  Larger Coulomb grids return
+ * HFB_ERR_UNSUPPORTED_GRID.  Call it with the context's device current
  * (HFB_ERR_ARG otherwise).  The first call on each device looks up the
  * array's device address, so make that first call before any stream
  * capture.  All calls share the one buffer (it keeps the last call's

@@ -682,12 +682,15 @@ extern "C" int hfb_skyrme(hfb_ctx_t ctx, const hfb_force* f, int tcoul, const do
 // the context's growable scratch arena.
 namespace hfb {
 
-// Doubled-grid work buffer: 64^3 complex doubles (4 MiB).  The Coulomb grid
-// n2 (2n non-periodic, n periodic) must be at most 64: n <= 32 for a
-// non-periodic grid; every periodic grid a context accepts (n <= 48) fits.
-// Every GPU that loads the library holds it until the process exits.
+// Its size is that of the work array (poisson_work) of the largest Coulomb grid
+// served, n2 = 64 (2n non-periodic: n <= 32; every periodic grid a context
+// accepts, n2 = n <= 48, fits): 32 x 64 x 33 complex doubles, 1 MiB.  The larger
+// non-periodic grids (3.4 MiB at n = 48) are left to hfb_poisson: every GPU that
+// loads the library holds the array until the process exits.
 constexpr int kNoAllocN2 = 64;
-static __device__ __align__(256) double2 g_poisson_noalloc[(size_t)kNoAllocN2 * kNoAllocN2 * kNoAllocN2];
+constexpr size_t kNoAllocWork = (size_t)(kNoAllocN2 / 2) * kNoAllocN2 * (kNoAllocN2 / 2 + 1);
+static_assert(kNoAllocWork >= (size_t)48 * 48 * (48 / 2 + 1), "the periodic grids");
+static __device__ __align__(256) double2 g_poisson_noalloc[kNoAllocWork];
 
 // Device address of g_poisson_noalloc per device ordinal, looked up on the
 // first call made on that device (the array's host-side name is only a
@@ -715,7 +718,7 @@ static int noalloc_buffer(int dev, double2** out) {
 extern "C" int hfb_poisson_noalloc(hfb_ctx_t ctx, const double* rho_p, double* wcoul, void* stream) {
   using namespace hfb;
   if (!ctx || !rho_p || !wcoul) return HFB_ERR_ARG;
-  if (ctx->n2 > kNoAllocN2) return HFB_ERR_UNSUPPORTED_GRID;   // work buffer too small for this grid
+  if (ctx->n2 > kNoAllocN2) return HFB_ERR_UNSUPPORTED_GRID;   // the work array is not sized for this grid
   // the buffer is looked up on the current device; the context's Green's
   // function lives on the device it was created on: they must be the same
   int dev = -1;
