@@ -46,7 +46,10 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // than SMs leaves whole SMs to what runs beside it.  The slices are short
 // enough for about four tickets a group (fewer on small grids, where a slice
 // would fall below 1024 points and its start-up show); they do not depend on
-// which matrices a launch computes, so neither does any sum's order.
+// which matrices a launch computes, so neither does any sum's order.  S + lambda
+// of 140 states at 48^3 alone with 1, 2, 4 and 8 tickets: 2.76, 2.10, 2.08, 1.95
+// ms; of 61 states 654, 495, 468, 448 us; at 32^3 2 to 8 are equal.  (The S +
+// lambda, H + G launches of a Pb208 iteration are equal with 4 and 6.)
 // Measured, S + lambda of Pb208 (140 + 96 states, 48^3): 3.8 ms with 594
 // equal CTAs on 592 places and all of lambda, 2.1 ms here (30 TFLOP/s).  G's
 // factor v_pair is applied at the fragment loads (multiplied on the way into
@@ -446,7 +449,11 @@ int gram_f64_launch(hfb_ctx_s* c, int nblk, const int* s0, const int* ns, const 
                     double2* const* outs, int ldo, int leave, cudaStream_t st) {
   const size_t K = (size_t)2 * c->n * c->n * c->n;
   // tile edge by the MMA work of Hermitian matrices; the smaller edges have
-  // fewer MMAs per fragment load (10 and 25 % slower at the same work)
+  // fewer MMAs per fragment load.  Time at the same work against edge 48 at
+  // 48^3, S + H: 140 states, edge 32 1.09, 24 1.02, 16 1.11; 48 states, 24 1.05,
+  // 16 1.17.  With these factors the choice is the fastest edge or within 5 % of
+  // it for 10 to 140 states from 24^3 to 48^3 (with all of lambda, whose work is
+  // not halved, up to 20 % off at 48 states)
   const int edge[4] = {48, 32, 24, 16};
   const double slow[4] = {1.0, 1.05, 1.1, 1.25};
   int gt = 48, tiles = 0;

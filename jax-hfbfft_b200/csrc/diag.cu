@@ -2,8 +2,10 @@
 // (463-482) and construct_hfb_matrices (484-577).
 //
 //  * Gram contractions C_a = wxyz Psi^H X_a (X = psi, hampsi, hmfpsi,
-//    v_pair psi) over K = 2 n^3: one kernel reads each psi tile once for all
-//    requested matrices; split-K partials are summed in a fixed order.
+//    v_pair psi) over K = 2 n^3: one launch over the output tiles of all
+//    requested matrices; split-K partials are summed in a fixed order.  On the
+//    tensor cores in gram_tc.cu (FP32) and contract_f64.cu (FP64); the kernel on
+//    CUDA cores here serves what those do not.
 //  * Hermitian eigensolver: cyclic two-sided Jacobi in one CTA on the folded
 //    lower triangle held in shared memory (round-robin ordering, n/2 disjoint
 //    rotations per round); the rotations are recorded and replayed onto the

@@ -66,9 +66,11 @@ constexpr int kTcMaxBoxes = 18;         // columns, rows among them or not, othe
 constexpr int kTcItems = 6;             // 32-byte row quarters per splitting thread and block
 static_assert(kTcItems * kTcSplitWarps * 32 >= 4 * kTcBoxRows * kTcMaxBoxes, "splitters' share");
 constexpr int kTcTmemCols = 512, kTcAccCols = 160;   // three accumulators
-// up to this many states hi*(hi|lo) is one MMA of twice the columns (Zr90, 61 +
-// 47 states, 40^3: 337 us against 360); by the states of the isospin, not the
-// columns of the unit, so that it depends on nothing else
+// up to this many states hi*(hi|lo) is one MMA of twice the columns, which is
+// what an accumulator holds; by the states of the isospin, not the columns of
+// the unit, so that it depends on nothing else.  16 states at 48^3 (S + lambda)
+// 171 us against 179 apart, 48 states 220 and 222, 80 states 269 and 265; all
+// four matrices at 40^3: 16 states 171 and 173, 61 states 251 and 247
 constexpr int kTcPairCols = kTcAccCols / 2;
 constexpr uint32_t kTcABytes = 128 * 128;   // 128 rows x 128 bytes
 constexpr long long kTcWaitLimit = 2000000000LL;

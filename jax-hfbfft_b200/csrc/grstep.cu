@@ -385,7 +385,7 @@ __global__ void simple_step_kernel(int ns, size_t n3, const double* spe_new, con
 // One block: a warp per state for the plane partials, then one warp's
 // fixed-order sums over the states (a thread per state and one thread's
 // sums took 61 us for 236 states of 48 planes, a serial chain of L2
-// latencies; 6 us here).
+// latencies; 20 us here for 236 states of 96 planes).
 __global__ void __launch_bounds__(1024)
 grstep_finish_kernel(int ns, int do_fluct, int nplanes, const double2* __restrict__ fl, double wxyz,
                      const double* spe_new, const double* wocc, const double* wstates, double* sp_energy, double* ef1,

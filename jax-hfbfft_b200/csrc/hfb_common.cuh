@@ -187,8 +187,8 @@ template <int M, int SIGN, class Z> struct DFT {
 // After forward(), lane q owns X[k2 + M k1] for k2 = q + P t (t < T, k2 < M)
 // and k1 = 0..P-1 in f[t][k1] (the "frequency" distribution); inverse() takes
 // that distribution back to the space distribution.  Unnormalised in both
-// directions.  ``xb`` is this line's shared exchange buffer (N elements) and
-// ``tw`` a shared table tw[j] = exp(-2 pi i j / N).
+// directions.  ``xb`` is this line's shared exchange buffer (XB elements, more
+// than N) and ``tw`` a shared table tw[j] = exp(-2 pi i j / N).
 template <class R, int N_, int P_> struct Pencil {
   static constexpr int N = N_;
   static constexpr int P = P_;

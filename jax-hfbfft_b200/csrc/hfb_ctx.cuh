@@ -19,7 +19,7 @@ struct hfb_ctx_s {
   double2* coul_q;       // Green's function in k space, n2^3 (coulomb.py:23-52)
   int* dev_status;       // latched device-side error code
   int* counters;         // behind dev_status, zero between launches: [0] finished blocks of the gradient step's
-                         // maximum, [1] tickets of the FP64 Gram
+                         // maximum, [1] tickets of the Gram launches
   cudaStream_t side;     // secondary stream for independent work inside a call
   int use_tcgen05;       // single-precision contractions on the tensor cores (default 1;
                          // HFB_NO_TCGEN05=1 in the environment at creation selects CUDA cores)

@@ -11,8 +11,8 @@ device, so each result is the one the instance gives alone.
 
 ``run_sweep_graph`` instead advances a group of instances together: after
 their start-up iterations, blocks of iterations of every instance in the
-group are captured into one CUDA graph (hfb.graph) and each graph launch
-runs them all, with the host reading the energies once per block.
+group are captured into CUDA graphs (hfb.graph) that run side by side, with
+the host reading the energies once per block.
 
 ``sweep_cases`` draws the instances of the sweep workload: species uniform
 over SPECIES and each coupling (t0-t3, x0-x3, W0; W0 moves b4p with it)
@@ -105,8 +105,8 @@ def run_sweep(cases, workers=8, maxiter=1500):
 
 
 def run_sweep_graph(cases, group=32, maxiter=1500, block=10):
-    """Solve every case with the graph driver, ``group`` instances per
-    graph (the groups one after the other).  Results in case order."""
+    """Solve every case with the graph driver, ``group`` instances at a
+    time (the groups one after the other).  Results in case order."""
     from . import graph
     out = []
     for g0 in range(0, len(cases), group):
@@ -128,7 +128,7 @@ def main(argv=None):
     ap.add_argument("--workers", type=int, default=16)
     ap.add_argument("--seed", type=int, default=20261203)
     ap.add_argument("--maxiter", type=int, default=1500)
-    ap.add_argument("--graph", action="store_true", help="graph driver: groups of instances per CUDA graph")
+    ap.add_argument("--graph", action="store_true", help="graph driver: groups of instances as CUDA graphs")
     ap.add_argument("--group", type=int, default=32)
     args = ap.parse_args(argv)
     cases = sweep_cases(args.instances, args.seed)
